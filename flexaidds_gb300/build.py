@@ -17,11 +17,9 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 UNITS = [("fxe_build.cu", ["--fmad=false"]), ("fxe_contacts.cu", []), ("fxe_thermo.cu", []), ("fxe_ga.cu", []),
          ("fxe_cluster.cu", ["--fmad=false"]), ("fxe_ensemble.cu", []), ("fxe_prepare.cu", ["--fmad=false"]),
          ("fxe_capi.cu", []),
-         # the polyhedron kernel twice: single precision, and double precision with the
-         # reference's expressions and every operation rounded separately
-         ("fxe_voronoi.cu", ["-DFXE_REAL=float", "-DFXE_VARIANT=f32"], "fxe_voronoi_f32.o"),
-         ("fxe_voronoi.cu", ["-DFXE_REAL=double", "-DFXE_VARIANT=f64", "-DFXE_REFERENCE_FORMULAS=1",
-                             "--fmad=false"], "fxe_voronoi_f64.o")]
+         # the polyhedron kernels: single precision, and double precision with the reference's
+         # expressions and every operation rounded separately
+         ("fxe_voronoi.cu", []), ("fxe_poly64.cu", ["--fmad=false"])]
 
 
 def nvcc() -> str:

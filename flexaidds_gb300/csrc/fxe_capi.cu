@@ -27,16 +27,12 @@ void launch_poses(const DevSystem&, const DevWork&, int, int*, uint8_t*, size_t,
 cudaError_t configure_voronoi();
 size_t pose_hist_bytes();
 int pose_max_blocks_per_sm();
-int pose_warps_per_block();
-int pose_tile_for(int, size_t, int);
-int pose_launch_blocks(int, size_t, int);
 }
 namespace f64 {
 void launch_poses(const DevSystem&, const DevWork&, int, int*, uint8_t*, size_t, int, cudaStream_t);
 cudaError_t configure_voronoi();
 size_t pose_hist_bytes();
 int pose_max_blocks_per_sm();
-int pose_warps_per_block();
 int pose_tile_for(int, size_t, int);
 int pose_launch_blocks(int, size_t, int);
 }
@@ -44,18 +40,14 @@ int pose_launch_blocks(int, size_t, int);
 // How the pose order of a polyhedron launch over n poses may be dealt: {full tiles that start
 // together (0: none, the order stays sorted), poses per tile}; the order kernel deals when those
 // tiles are all the launch has or its scored poses do not fill them (launch_order_poses). Only
-// lockstep launches have tiles.
+// reference-precision launches have tiles.
 struct Deal {
     int deal, tile;
 };
 inline Deal order_deal(int precision, int n, size_t hist_bytes, int blocks_per_sm) {
-    const bool fast = precision == FXE_PRECISION_FAST;
-    const int tile = fast ? f32::pose_tile_for(n, hist_bytes, blocks_per_sm)
-                          : f64::pose_tile_for(n, hist_bytes, blocks_per_sm);
-    if (tile < 1) return {0, 0};
-    const int blocks = fast ? f32::pose_launch_blocks(n, hist_bytes, blocks_per_sm)
-                            : f64::pose_launch_blocks(n, hist_bytes, blocks_per_sm);
-    return {std::min(n / tile, blocks), tile};
+    if (precision == FXE_PRECISION_FAST) return {0, 0};
+    const int tile = f64::pose_tile_for(n, hist_bytes, blocks_per_sm);
+    return {std::min(n / tile, f64::pose_launch_blocks(n, hist_bytes, blocks_per_sm)), tile};
 }
 // Face history of a polyhedron launch, large enough for either precision's launch: the warps the
 // device holds at once, kHistStride bytes each (configure_voronoi first).

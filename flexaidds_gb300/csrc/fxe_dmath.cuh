@@ -1,0 +1,131 @@
+// fxe_dmath.cuh — double-precision quotients and square roots, correctly rounded, with five FP64
+// instructions each, and conversions on the integer units.
+//
+// GB300's FP64 unit takes one warp instruction per 64 cycles and SM quarter, whatever its active
+// lanes (measured: 66 cycles per DFMA of one warp, dependent or not; 16.4 per SM with four or more
+// warps; conversions from and to double and comparisons cost the same), and the compiler's quotient
+// and root are nine such instructions each (146 cycles per SM). Here the reciprocal (or reciprocal
+// root) of the operand's significand comes from the single-precision unit — its approximation, then
+// one Newton-Raphson step on the operand split in two floats, about 45 bits — and is put together as
+// a double with integer arithmetic.
+//
+// Quotient: one more Newton step in double (two fused multiply-adds) leaves the reciprocal y within
+// 2^-84 of 1/b before its rounding, so z0 = a y is within two units in the last place of a / b, and
+// z1 = z0 + (a - b z0) y, whose residual is exact, is correctly rounded (P. W. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34,
+// 1990). Root: two such corrections, z + (x - z z) y / 2: the first leaves z within 2^-80 of the root
+// before its rounding, the second rounds it correctly. Both equal the plain operators bit for bit
+// (checked on 1.6e9 operands of every kind); an exponent out of the range the steps need, and a
+// divisor whose significand is all ones (the theorem's exception), fall back to them. The plain
+// operators sit in functions of their own that are called: left in line, the compiler evaluates them
+// beside the short form and selects.
+#pragma once
+
+#include <cstdint>
+
+namespace fxe {
+
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rsqrt_approx(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Biased exponents of operands the short forms take: 2^-350 .. 2^350.
+constexpr unsigned kExpLo = 673, kExpSpan = 701;
+
+__device__ __forceinline__ int biased_exp(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+
+// The significand of x as a float in [1, 2), truncated.
+__device__ __forceinline__ float top_float(double x) {
+    return __uint_as_float(0x3f800000u | ((unsigned)(__double2hiint(x) & 0xfffff) << 3) |
+                           ((unsigned)__double2loint(x) >> 29));
+}
+
+// (double)x on the integer units (a denormal or special x: the plain conversion).
+__device__ __forceinline__ double f2d(float x) {
+    const unsigned u = __float_as_uint(x), m = u & 0x7fffffffu;
+    double d = __hiloint2double((int)((u & 0x80000000u) | ((m >> 3) + (m ? 0x38000000u : 0u))), (int)(u << 29));
+    if (m - 1u < 0x7fffffu || m >= 0x7f800000u) d = (double)x;
+    return d;
+}
+
+// x as a float, truncated; 0 below the normal range, infinity above it.
+__device__ __forceinline__ float d2f_trunc(double x) {
+    const int hi = __double2hiint(x);
+    const int h = (hi & 0x7fffffff) - 0x38000000;
+    unsigned u = __funnelshift_l((unsigned)__double2loint(x), (unsigned)h, 3);
+    if (h < 0x100000) u = 0u;
+    if (h >= 0x0ff00000) u = 0x7f800000u;
+    return __uint_as_float(u | ((unsigned)hi & 0x80000000u));
+}
+
+// (r + yl) * 2^k, r in [0.5, 1] and |yl| < 2^-18: the sum as an integer of 2^-62, whose top 53 bits
+// complete the exponent field (1021 + k).
+__device__ __forceinline__ double join_recip(float r, float yl, int k) {
+    // (the approximation may land a step outside [0.5, 1])
+    const float rc = fminf(fmaxf(r, 0.5f), 1.0f);
+    yl += r - rc;
+    const unsigned rb = __float_as_uint(rc);
+    const unsigned mant = ((rb & 0x7fffffu) | 0x800000u) << ((rb >> 23) - 126u);   // rc * 2^24
+    const long long y62 = ((long long)mant << 38) + ((long long)__float2int_rn(yl * 0x1.0p48f) << 14);
+    return __longlong_as_double((y62 >> 9) + ((long long)(1021 + k) << 52));
+}
+
+// 1 / |b| to about 45 bits.
+__device__ __forceinline__ double recip45(double b) {
+    const float bh = top_float(b);
+    const float bl = (float)(__double2loint(b) & 0x1fffffff) * 0x1.0p-52f;
+    const float r = rcp_approx(bh);
+    float e = fmaf(-bh, r, 1.0f);
+    e = fmaf(-bl, r, e);
+    return join_recip(r, r * fmaf(e, e, e), 1023 - biased_exp(b));
+}
+
+// 1 / (2 sqrt(x)) for x > 0 to about 45 bits.
+__device__ __forceinline__ double half_rsqrt45(double x) {
+    const int ex = (__double2hiint(x) >> 20) - 1023;
+    const float sc = (ex & 1) ? 2.0f : 1.0f;
+    const float xh = top_float(x) * sc;
+    const float xl = (float)(__double2loint(x) & 0x1fffffff) * (sc * 0x1.0p-52f);
+    const float r = rsqrt_approx(xh);
+    const float r2 = r * r, r2l = fmaf(r, r, -r2);
+    float t = fmaf(-xh, r2, 1.0f);
+    t = fmaf(-xh, r2l, t);
+    t = fmaf(-xl, r2, t);
+    return join_recip(r, r * t * fmaf(t, 0.375f, 0.5f), -(ex >> 1) - 1);
+}
+
+// a / b; *slow: the plain operator is needed.
+__device__ __forceinline__ double div_short(double a, double b, bool* slow) {
+    const double ab = fabs(b);
+    double y = recip45(b);
+    y = __fma_rn(__fma_rn(-ab, y, 1.0), y, y);
+    double q = __dmul_rn(a, y);
+    q = __fma_rn(__fma_rn(-ab, q, a), y, q);
+    if (__double2hiint(b) < 0) q = -q;
+    const bool a_ok = (unsigned)(biased_exp(a) - (int)kExpLo) < kExpSpan || (__double2hiint(a) | __double2loint(a)) == 0;   // (-0: the plain operator)
+    const bool ones = (((unsigned)__double2hiint(b) | 0xfff00000u) & (unsigned)__double2loint(b)) == 0xffffffffu;
+    *slow = !a_ok || (unsigned)(biased_exp(b) - (int)kExpLo) >= kExpSpan || ones;
+    return q;
+}
+
+// sqrt(x); *slow: the plain function is needed.
+__device__ __forceinline__ double sqrt_short(double x, bool* slow) {
+    const double h = half_rsqrt45(x);
+    double g = __dmul_rn(x, __hiloint2double(__double2hiint(h) + (1 << 20), __double2loint(h)));
+    g = __fma_rn(__fma_rn(-g, g, x), h, g);
+    g = __fma_rn(__fma_rn(-g, g, x), h, g);
+    *slow = (unsigned)((__double2hiint(x) >> 20) - (int)kExpLo) >= kExpSpan;
+    return g;
+}
+
+__device__ __noinline__ double plain_div(double a, double b) { return a / b; }
+__device__ __noinline__ double plain_sqrt(double x) { return sqrt(x); }
+
+}  // namespace fxe

@@ -1,13 +1,14 @@
-// fxe_voronoi.cu — Voronoi contact surfaces and complementarity scoring (the candidate lists
-// come from contacts_kernel, fxe_contacts.cu).
+// fxe_voronoi.cu — Voronoi contact surfaces and complementarity scoring in single precision (fast
+// precision; fxe_poly64.cu holds the double-precision form). The candidate lists come from
+// contacts_kernel (fxe_contacts.cu).
 //
 // pose_kernel      one warp per pose: calc_region's loop over the scorable atoms in Calclist
 //                  order (LIB/Vcontacts.cpp:74-139) — each atom's list without the saved atoms
 //                  that kept no contact with it, its extended-radical-plane polyhedron started
 //                  from the seed an earlier atom left (voronoi_poly2, :147-490), faces
-//                  (order_faces, :699-831) and spherical areas (calc_areas, :838-1044) in FP64
-//                  (reference precision) or FP32 (fast precision), the contacts it keeps
-//                  (save_areas) and the seeds it leaves (save_seeds) —
+//                  (order_faces, :699-831) and spherical areas (calc_areas, :838-1044) with
+//                  well-conditioned equivalents of the reference's area expressions, the contacts
+//                  it keeps (save_areas) and the seeds it leaves (save_seeds) —
 //                  then vcfunction's walk over the kept contacts (LIB/vcfunction.cpp:14-574).
 //
 // The atoms of one pose stay in order because the reference's results depend on it: which
@@ -21,52 +22,17 @@
 #include "fxe_common.cuh"
 
 namespace fxe {
-namespace FXE_VARIANT {
+namespace f32 {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kFaceWords = (kMaxCand + 31) / 32;
 constexpr uint8_t kNone = 255;
 
-// Floating-point type of the polyhedron arithmetic: single precision by default; building
-// with -DFXE_REAL=double gives the same algorithm in double precision (for comparisons).
-#ifndef FXE_REAL
-#define FXE_REAL float
-#endif
-#ifndef FXE_VARIANT
-#define FXE_VARIANT f32
-#endif
-using real = FXE_REAL;
-// Double builds evaluate the areas with the reference's own expressions (they are not well
-// conditioned for small or nearly degenerate triangles, and the double build reproduces the
-// reference's values there too); single builds use well-conditioned equivalents.
-#ifndef FXE_REFERENCE_FORMULAS
-#define FXE_REFERENCE_FORMULAS 0
-#endif
-// Double builds decide the hull walk's plane tests in single precision first and redo a test
-// in double only when its single-precision result is within its error bound of deciding the
-// other way (see walk_step_group).
-#ifndef FXE_FILTER
-#define FXE_FILTER (FXE_REFERENCE_FORMULAS)
-#endif
-// Poses (warps) per block of pose_kernel, and whether the block's warps meet after every atom.
-// The double kernel's code (about 220 KB) outgrows the SM's instruction caches, and its top stall
-// was instruction fetch with eight warps of an SM at unrelated points of it: eight warps per block
-// (one block per SM, 20 KB of workspace each) that take eight neighbouring poses of the queue and
-// meet at a block barrier after each atom fetch the same code at about the same time (measured on
-// GB300, plain-scale workload: 22.9 -> 19.2 ms per launch; four warps per block 20.5 ms, ten
-// 21.7 ms). The single-precision kernel is not fetch-bound: two warps per block, twenty per SM,
-// each taking the next pose on its own.
-constexpr bool kLockstep = FXE_REFERENCE_FORMULAS;
-constexpr int kVorWarps = kLockstep ? 8 : 2;
-// The kernel outgrows the instruction cache: its rarely taken or bulky helpers are called, not
-// inlined (double build; measured one by one), and no loop is unrolled — every loop carries
-// `#pragma unroll 1` unless it says otherwise (measured on GB300, plain-scale workload: 36.0 ->
-// 30.4 ms per launch in double precision, 6.8 -> 4.9 ms in single).
-#if FXE_REFERENCE_FORMULAS
-#define FXE_COLD __noinline__
-#else
-#define FXE_COLD
-#endif
+using real = float;
+// Poses (warps) per block of pose_kernel, twenty per SM, each taking the next pose on its own. No
+// loop is unrolled — the kernel outgrows the instruction cache: every loop carries `#pragma unroll 1`
+// unless it says otherwise (measured on GB300, plain-scale workload: 6.8 -> 4.9 ms per launch).
+constexpr int kVorWarps = 2;
 struct __align__(4 * sizeof(real)) real4 {
     real x, y, z, w;
 };
@@ -142,9 +108,6 @@ struct VorShared {
         real tmp[32];                  // one value per lane, for in-order sums
         uint8_t elist[kMaxEdges + 8];  // the hull edges with an end outside the sphere
     };
-#if FXE_FILTER
-    float4 plf[kMaxPlanes];        // the planes rounded to single precision, for pre-tests
-#endif
     uint8_t flag[kMaxPlanes];
     uint8_t sprev[kMaxCand];       // per face: point 1 before a replayed stale read (kNone: none)
     uint8_t flist[kMaxCand];       // faces whose test point is checked against the other planes
@@ -161,7 +124,7 @@ __device__ __forceinline__ real dot3(const real4& a, real x, real y, real z) {
 }
 
 // solve_3x3 (LIB/Vcontacts.cpp:1384-1414) in FP32.
-__device__ FXE_COLD bool solve3(const real4& e0, const real4& e1, const real4& e2, real* pt) {
+__device__ bool solve3(const real4& e0, const real4& e1, const real4& e2, real* pt) {
     const real c00 = e1.y * e2.z - e2.y * e1.z;
     const real c01 = -e1.x * e2.z + e2.x * e1.z;
     const real c02 = e1.x * e2.y - e2.x * e1.y;
@@ -201,7 +164,7 @@ __device__ __forceinline__ real solve3_coord(const real4& e0, const real4& e1, c
 
 // solve_2xS (LIB/Vcontacts.cpp:1427-1476) in FP32.
 // rr is the square of the radius as the reference forms it: a single-precision product.
-__device__ FXE_COLD bool solve2s(const real4& a, const real4& b, real rr, real* p0, real* p1) {
+__device__ bool solve2s(const real4& a, const real4& b, real rr, real* p0, real* p1) {
     const real e2x = a.y * b.z - a.z * b.y;
     const real e2y = a.z * b.x - a.x * b.z;
     const real e2z = a.x * b.y - a.y * b.x;
@@ -259,33 +222,7 @@ __device__ __forceinline__ real angle_between(real ux, real uy, real uz, real vx
     return atan2(sqrt(wx * wx + wy * wy + wz * wz), ux * vx + uy * vy + uz * vz);
 }
 
-#if FXE_REFERENCE_FORMULAS
-// The reference's own expression (double builds): reproduces its values, including those of
-// nearly degenerate triangles, to rounding.
-__device__ FXE_COLD real sph_arc(const real4& ao, const real4& b, const real4& c, real rado) {
-    const real cosAOB = (ao.x * b.x + ao.y * b.y + ao.z * b.z) / (ao.w * b.w);
-    const real cosBOC = (b.x * c.x + b.y * c.y + b.z * c.z) / (b.w * c.w);
-    // (x / 8 and x * 0.125 are the same correctly rounded value: the multiply is the cheaper)
-    const real h = sqrt((1 + cosBOC) * real(0.125));
-    const real U = (1 + cosAOB) * h;
-    const real V = (1 - cosAOB) * h;
-    const real W = sqrt((1 - cosAOB) * (1 + cosAOB) * (1 - cosBOC) * real(0.125));
-    const real tS = (1 - U + V + W + W) / (1 + U - V - W - W);
-    const real tSB = (1 - U - V) / (1 + U + V);
-    const real tSA = (1 - U + V - W - W) / (1 + U - V + W + W);
-    real tanprod = real(0.0);
-    if ((tS * tSA) > real(0.0)) tanprod = sqrt(tSB * tSB * tS * tSA);
-    const real px = b.x - ao.x, py = b.y - ao.y, pz = b.z - ao.z;
-    const real qx = c.x - ao.x, qy = c.y - ao.y, qz = c.z - ao.z;
-    const real cosBAC = (px * qx + py * qy + pz * qz) / sqrt((px * px + py * py + pz * pz) * (qx * qx + qy * qy + qz * qz));
-    real angBAC;
-    if (cosBAC > real(1.0)) angBAC = real(0.0);
-    else if (cosBAC < real(-1.0)) angBAC = (real)kPi;
-    else angBAC = acos(cosBAC);
-    return rado * (angBAC * (rado - ao.w) - real(4.0) * rado * atan(sqrt(tanprod)));
-}
-#else
-__device__ FXE_COLD real sph_arc(const real4& ao, const real4& b, const real4& c, real rado) {
+__device__ real sph_arc(const real4& ao, const real4& b, const real4& c, real rado) {
     const real sector = angle_between(b.x - ao.x, b.y - ao.y, b.z - ao.z, c.x - ao.x, c.y - ao.y, c.z - ao.z);
     const real th = angle_between(ao.x, ao.y, ao.z, b.x, b.y, b.z);
     const real ph = angle_between(b.x, b.y, b.z, c.x, c.y, c.z);
@@ -293,7 +230,6 @@ __device__ FXE_COLD real sph_arc(const real4& ao, const real4& b, const real4& c
     const real tri = real(4.0) * atan(fabs(tan(ph * real(0.25))) * sqrt(t));
     return rado * (sector * (rado - ao.w) - rado * tri);
 }
-#endif
 
 __device__ __forceinline__ real4 centre_of(const real4& pl) {
     return make_real4(-pl.x * pl.w, -pl.y * pl.w, -pl.z * pl.w, fabs(pl.w));
@@ -338,41 +274,11 @@ struct WalkStep {
     int pc;      // closing plane, -1 if none
 };
 
-#if FXE_FILTER
-// Single-precision value of vt = -(P.s + w) / (P.V) and a bound on its distance from the same
-// expression evaluated in double: every input is rounded once to float and every operation
-// rounds, 16 units of roundoff (2^-20) per sum of absolute terms covers both; the quotients use
-// the fast reciprocal (at most 2 units in the last place off, covered by 4 units of |vt| and the
-// 1/16 margin on the bound). den_ok is false when the sign of P.V is not certain (the double test
-// skips P.V == 0 exactly), when |P.V| is too small for the fast quotient, or when the bound is
-// not finite.
-__device__ __forceinline__ float vt_pretest(const float4& P, float sx, float sy, float sz, float Vx,
-                                            float Vy, float Vz, float* err, bool* den_ok) {
-    const float g = 9.5367431640625e-07f;   // 2^-20
-    const float den = P.x * Vx + P.y * Vy + P.z * Vz;
-    const float eden = g * (fabsf(P.x * Vx) + fabsf(P.y * Vy) + fabsf(P.z * Vz));
-    const float num = P.x * sx + P.y * sy + P.z * sz + P.w;
-    const float enm = g * (fabsf(P.x * sx) + fabsf(P.y * sy) + fabsf(P.z * sz) + fabsf(P.w));
-    // an all-zero normal (an excluded candidate's inert plane) has P.V == 0 exactly in double
-    // too, and the double test skips it; report it as a decided non-positive value
-    if (P.x == 0.0f && P.y == 0.0f && P.z == 0.0f) {
-        *den_ok = true;
-        *err = 0.0f;
-        return -1.0f;
-    }
-    const bool ok = fabsf(den) > 2.0f * eden && fabsf(den) > 1e-30f;
-    const float vt = __fdividef(-num, den);
-    const float er = __fdividef(enm + fabsf(vt) * eden, fabsf(den) - eden) * 1.0625f + fabsf(vt) * 4.8e-7f;
-    *den_ok = ok && er < 3.0e38f;
-    *err = er;
-    return vt;
-}
-#endif
 
 // The vertex that ends edge e (LIB/Vcontacts.cpp:283-330), in full precision: the plane with
 // the smallest positive vt along the edge (planes spread over the lanes) and, when that point
 // lies outside the sphere, the bounding planes too. The result is uniform across the warp.
-__device__ FXE_COLD WalkStep walk_step_exact(const VorShared& sh, int NC, int e, real rr, int lane) {
+__device__ WalkStep walk_step_exact(const VorShared& sh, int NC, int e, real rr, int lane) {
     const uchar4 ep = sh.u.e.ep[e];
     const real3 V = sh.u.e.ev[e];
     const real4 s = sh.vx[sh.u.e.es[e].x];
@@ -464,76 +370,6 @@ __device__ GroupStep walk_step_group(const VorShared& sh, int NC, int e, real rr
     }
     const int pA = ep.x, pB = ep.y, oldC = ep.z;
     GroupStep r;
-#if FXE_FILTER
-    // planes pre-tested in single precision; when the winner is surely positive and every other
-    // plane surely not positive or surely farther, only the winner's vt is evaluated in double
-    const float sx = (float)s.x, sy = (float)s.y, sz = (float)s.z;
-    const float Vx = (float)V.x, Vy = (float)V.y, Vz = (float)V.z;
-    float best = 9.9e9f, beste = 0.0f;
-    int bi = INT_MAX;
-    // and the two smallest lower bounds (vt - err) over the planes whose vt may be positive: every
-    // plane but the winner must be surely not positive or surely farther
-    float lo1 = 3.0e38f, lo2 = 3.0e38f;
-    int lo1i = INT_MAX;
-    bool unsure = false;
-    if (has) {
-        #pragma unroll 1
-        for (int c = sub; c < NC; c += kWalkLanes) {
-            if (c == pA || c == pB || c == oldC) continue;
-            float er;
-            bool ok;
-            const float vt = vt_pretest(sh.plf[c], sx, sy, sz, Vx, Vy, Vz, &er, &ok);
-            if (!ok) {
-                unsure = true;
-                continue;
-            }
-            if (vt > 0.0f && vt < best) { best = vt; beste = er; bi = c; }
-            if (vt + er > 0.0f) {
-                const float lo = vt - er;
-                if (lo < lo1) { lo2 = lo1; lo1 = lo; lo1i = c; }
-                else if (lo < lo2) lo2 = lo;
-            }
-        }
-    }
-#pragma unroll
-    for (int o = kWalkLanes / 2; o > 0; o >>= 1) {
-        const float b2 = __shfl_xor_sync(kFull, best, o);
-        const float e2 = __shfl_xor_sync(kFull, beste, o);
-        const int i2 = __shfl_xor_sync(kFull, bi, o);
-        if (b2 < best || (b2 == best && i2 < bi)) { best = b2; beste = e2; bi = i2; }
-    }
-    if (bi != INT_MAX && !(best - beste > 0.0f)) unsure = true;
-    const float mylo = lo1i == bi ? lo2 : lo1;
-    if (mylo < 3.0e38f && !(bi != INT_MAX && mylo > best + beste)) unsure = true;
-    unsure = (__ballot_sync(kFull, unsure) & gmask) != 0u;
-    real vtmin = real(9.9e9);
-    if (!unsure && bi != INT_MAX) {
-        const real4 P = sh.pl[bi];
-        const real den = P.x * V.x + P.y * V.y + P.z * V.z;
-        vtmin = -(P.x * s.x + P.y * s.y + P.z * s.z + P.w) / den;
-    }
-    r.x = s.x + vtmin * V.x;
-    r.y = s.y + vtmin * V.y;
-    r.z = s.z + vtmin * V.z;
-    // outside the sphere: the bounding planes (10 A out) are most of the time surely farther
-    bool need = false;
-    if (has && !unsure && r.x * r.x + r.y * r.y + r.z * r.z > rr) {
-        need = bi == INT_MAX;
-        if (!need && sub < 4) {
-            const int c = NC + sub;
-            if (c != pA && c != pB && c != oldC) {
-                float er;
-                bool ok;
-                const float vt = vt_pretest(sh.plf[c], sx, sy, sz, Vx, Vy, Vz, &er, &ok);
-                need = !(ok && (vt + er <= 0.0f || vt - er > (float)vtmin * 1.0000005f));
-            }
-        }
-    }
-    // (every lane takes part in the ballot: it must not sit behind a short-circuit)
-    const unsigned need_lanes = __ballot_sync(kFull, need);
-    r.unsure = unsure || (need_lanes & gmask) != 0u;
-    r.pc = bi == INT_MAX ? -1 : bi;
-#else
     real vtmin = real(9.9e9);
     int pC = INT_MAX;
     if (has) {
@@ -572,7 +408,6 @@ __device__ GroupStep walk_step_group(const VorShared& sh, int NC, int e, real rr
     }
     r.pc = pC == INT_MAX ? -1 : pC;
     r.unsure = false;
-#endif
     return r;
 }
 
@@ -599,26 +434,8 @@ __device__ __forceinline__ int arc_segment(const VorShared& sh, const uint8_t* p
 
 // Area of the fan triangle v0 va vb on the sphere of radius rado.
 __device__ __forceinline__ real fan_triangle(const real4& v0, const real4& va, const real4& vb, real rado) {
-#if FXE_REFERENCE_FORMULAS
-    // L'Huilier-type tangent products as the reference writes them (LIB/Vcontacts.cpp:927-940)
-    const real cNN1 = (va.x * vb.x + va.y * vb.y + va.z * vb.z) / (va.w * vb.w);
-    const real cN0a = (v0.x * va.x + v0.y * va.y + v0.z * va.z) / (v0.w * va.w);
-    const real cN0b = (v0.x * vb.x + v0.y * vb.y + v0.z * vb.z) / (v0.w * vb.w);
-    // (x / 8 and x * 0.125 are the same correctly rounded value: the multiply is the cheaper)
-    const real U = sqrt((1 + cN0a) * (1 + cNN1) * (1 + cN0b) * real(0.125));
-    const real V = sqrt((1 - cN0a) * (1 - cNN1) * (1 + cN0b) * real(0.125));
-    const real W = sqrt((1 - cN0a) * (1 + cNN1) * (1 - cN0b) * real(0.125));
-    const real Xv = sqrt((1 + cN0a) * (1 - cNN1) * (1 - cN0b) * real(0.125));
-    const real tS = (1 - U + V + W + Xv) / (1 + U - V - W - Xv);
-    const real tSA = (1 - U - V - W + Xv) / (1 + U + V + W - Xv);
-    const real tSB = (1 - U - V + W - Xv) / (1 + U + V - W + Xv);
-    const real tSC = (1 - U + V - W - Xv) / (1 + U - V + W + Xv);
-    const real tanprod = sqrt(tS * tSA * tSB * tSC);
-    return tanprod > real(0.0) ? real(4.0) * rado * rado * atan(sqrt(tanprod)) : real(0.0);
-#else
     // the same triangle's solid angle, well conditioned in FP32
     return rado * rado * solid_angle(v0, va, vb);
-#endif
 }
 
 // Adds each lane's value v to the area of face X (X < 0: nothing), lanes of one face in lane
@@ -656,7 +473,7 @@ __device__ __forceinline__ int engulf_comm(const VorShared& sh, int NC, int X, i
 // engulfed faces' points one after another; here each (face, point) item of the flat face lists
 // goes to a lane, the arcs are evaluated together, and each neighbour's sum is formed in the
 // reference's order. tot_pts: the length of the flat face lists.
-__device__ FXE_COLD void engulf_corrections(VorShared& sh, int NC, int tot_pts, real rado, real rr, real two_pi_r,
+__device__ void engulf_corrections(VorShared& sh, int NC, int tot_pts, real rado, real rr, real two_pi_r,
                                             int epi, int lane) {
     if (epi > 0) {
         // the items that credit an arc, in order, packed (face, current point, next point,
@@ -781,9 +598,6 @@ __device__ int voronoi_warp(VorShared& sh, int NC, real rado, int lane, int* no_
         const real by[4] = {real(1.0), -real(1.0), real(0.0), real(0.0)};
         const real bz[4] = {real(0.0), real(0.0), real(1.0), -real(1.0)};
         sh.pl[NC + lane] = make_real4(bx[lane], by[lane], bz[lane], -real(10.0));
-#if FXE_FILTER
-        sh.plf[NC + lane] = make_float4((float)bx[lane], (float)by[lane], (float)bz[lane], -10.0f);
-#endif
         sh.flag[NC + lane] = 0;
     }
     #pragma unroll 1
@@ -1304,13 +1118,9 @@ __device__ int voronoi_warp(VorShared& sh, int NC, real rado, int lane, int* no_
             const real a = Vx * Vx + Vy * Vy + Vz * Vz;
             const real b = 2 * (P.x * Vx + P.y * Vy + P.z * Vz);
             const real c = P.x * P.x + P.y * P.y + P.z * P.z - rr;
-#if FXE_REFERENCE_FORMULAS
-            const real k = (sqrt(b * b - real(4.0) * a * c) - b) / (2 * a);
-#else
             // positive root of a k^2 + b k + c = 0 without cancellation when b > 0
             const real sq = sqrt(b * b - real(4.0) * a * c);
             const real k = b > real(0.0) ? (-real(2.0) * c) / (sq + b) : (sq - b) / (2 * a);
-#endif
             P.x += k * Vx; P.y += k * Vy; P.z += k * Vz;
             P.w = rado;
             sh.vx[vi] = P;
@@ -1457,9 +1267,6 @@ __device__ int load_planes(VorShared& sh, const DevSystem& S, const DevWork& W, 
             const real4 P = make_real4((real)(pj.x - me.x) / d, (real)(pj.y - me.y) / d, (real)(pj.z - me.z) / d,
                                        -(num / (real(2.0) * d)));
             sh.pl[r] = P;
-#if FXE_FILTER
-            sh.plf[r] = make_float4((float)P.x, (float)P.y, (float)P.z, (float)P.w);
-#endif
             sh.flag[r] = eng ? kEngulf : 0;
         }
         NC += __popc(m);
@@ -1482,8 +1289,7 @@ __device__ double pose_clash_sum(const DevSystem& S, const DevWork& W, int p, in
 // pose_kernel: calc_region + vcfunction for one pose per warp
 // ------------------------------------------------------------------------------------------
 // Shared memory per warp sets how many poses an SM holds at once, so the per-pose seeds and
-// record masks live in the workspace (W.pose_seed, W.pose_rec); 20.0 KB of shared memory per pose
-// in double precision, 11.1 KB in single.
+// record masks live in the workspace (W.pose_seed, W.pose_rec); 11.1 KB of shared memory per pose.
 struct PoseShared {
     VorShared v;
     uint8_t order[kMaxLig];          // mobile atoms in Calclist order
@@ -1516,43 +1322,35 @@ __device__ void finish_failed(const DevWork& W, int p, int lane, int status, dou
     if (lane == 0) W.out[p] = cf;
 }
 
-// p < 0: no pose (the warp only keeps its block's barriers). n_iter: the atom steps the block
-// takes together in lockstep (at least this pose's scored atoms; unused otherwise).
 __device__ __forceinline__ void score_pose(const DevSystem& S, const DevWork& W, int p, int lane,
-                                           PoseShared& ps, uint8_t* hist, int n_iter) {
+                                           PoseShared& ps, uint8_t* hist) {
     VorShared& sh = ps.v;
-    // a pose that fails stops here; in lockstep its warp still meets the block after every step
-    bool alive = p >= 0;
-    if (p < 0) p = 0;
     const int nl = n_mobile(S);      // the scored atoms: side-chain atoms, then the ligand
     // polyhedron seeds (Calc indices, -1 = none) and the mobile partners each processed atom kept
     int (*const seed)[3] = reinterpret_cast<int (*)[3]>(W.pose_seed + (size_t)p * kMaxLig * 3);
     uint32_t (*const rec)[kMaskWords] = reinterpret_cast<uint32_t (*)[kMaskWords]>(W.pose_rec + (size_t)p * kMaxLig * kMaskWords);
     const size_t lb = (size_t)p * nl;
-    if (alive && W.pose_grid[p].z) {
+    if (W.pose_grid[p].z) {
         finish_failed(W, p, lane, FXE_POSE_CAPACITY, 0.0);
-        alive = false;
+        return;
     }
     // clash pre-filter (LIB/Vcontacts.cpp:36-51)
-    if (alive) {
-        const double clash = pose_clash_sum(S, W, p, lane);
-        if (clash >= kClashThreshold) {
-            finish_failed(W, p, lane, FXE_POSE_CLASHED, clash);
-            alive = false;
-        }
+    const double clash = pose_clash_sum(S, W, p, lane);
+    if (clash >= kClashThreshold) {
+        finish_failed(W, p, lane, FXE_POSE_CLASHED, clash);
+        return;
     }
-    if (!kLockstep && !alive) return;
     #pragma unroll 1
-    for (int l = lane; alive && l < nl; l += 32) {
+    for (int l = lane; l < nl; l += 32) {
         ps.order[W.mob_rank[lb + l]] = (uint8_t)l;
         seed[l][0] = seed[l][1] = seed[l][2] = -1;
 #pragma unroll
         for (int w = 0; w < kMaskWords; ++w) rec[l][w] = 0;
     }
-    if (alive && lane < kMaskWords) ps.done[lane] = 0;
+    if (lane < kMaskWords) ps.done[lane] = 0;
     // the face history starts the pose at zero, as the reference's ptorder does on a workspace
     // cleared before the pose
-    if (alive && hist) {
+    if (hist) {
         uint4* h4 = reinterpret_cast<uint4*>(hist);
         #pragma unroll 1
         for (int k = lane; k < kHistBytes / 16; k += 32) h4[k] = make_uint4(0u, 0u, 0u, 0u);
@@ -1560,16 +1358,13 @@ __device__ __forceinline__ void score_pose(const DevSystem& S, const DevWork& W,
     __syncwarp();
     // calc_region: atoms in Calclist order (LIB/Vcontacts.cpp:74-139)
     #pragma unroll 1
-    for (int r = 0; r < (kLockstep ? n_iter : nl); ++r) {
-        if (!alive || r >= nl) goto atom_end;
-        {
+    for (int r = 0; r < nl; ++r) {
         const int a = ps.order[r];
         const int n_cand = W.cand_n[lb + a];
         if (n_cand < 0) {
             if (lane == 0) atomicAdd(&W.counters[2], 1);
             finish_failed(W, p, lane, FXE_POSE_CAPACITY, 0.0);
-            alive = false;
-            goto atom_end;
+            return;
         }
         const size_t cb = (lb + a) * kMaxCand;
         // get_contlist4's list: saved atoms drop out unless they kept a contact with this one, and
@@ -1594,7 +1389,7 @@ __device__ __forceinline__ void score_pose(const DevSystem& S, const DevWork& W,
                 W.cand_area[cb + c] = 0.0;
                 W.cand_flag[cb + c] = 0;
             }
-            goto atom_end;
+            continue;
         }
         const float4 me = W.mob_pos[lb + a];
         const float rado = me.w + kRw;
@@ -1622,14 +1417,12 @@ __device__ __forceinline__ void score_pose(const DevSystem& S, const DevWork& W,
         if (st == kAtomCapacity) {
             if (lane == 0) atomicAdd(&W.counters[2], 1);
             finish_failed(W, p, lane, FXE_POSE_CAPACITY, 0.0);
-            alive = false;
-            goto atom_end;
+            return;
         }
         if (st == kAtomHullFail) {
             if (lane == 0) atomicAdd(&W.counters[1], 1);
             finish_failed(W, p, lane, FXE_POSE_POLYHEDRON_FAILED, (double)kPolyPenalty);
-            alive = false;
-            goto atom_end;
+            return;
         }
         // save_areas (LIB/Vcontacts.cpp:1149-1220): contacts with area > 0 on a contact plane;
         // candidates outside the contact list record nothing
@@ -1682,11 +1475,6 @@ __device__ __forceinline__ void score_pose(const DevSystem& S, const DevWork& W,
         }
         __syncwarp();
     }
-    atom_end:
-        if (kLockstep) __syncthreads();
-        if (!kLockstep && !alive) return;
-    }
-    if (!alive) return;
     // vcfunction (LIB/vcfunction.cpp:84-513): scored atoms in Calc order (side-chain atoms,
     // then the ligand), their kept contacts; each residue's terms are summed on their own and the
     // records added up ligand first, then the side chains in order (LIB/ic2cf.cpp:133-245)
@@ -1801,35 +1589,16 @@ __device__ __forceinline__ uint8_t* warp_hist(uint8_t* hist_all) {
     return hist_all ? hist_all + (size_t)(blockIdx.x * kVorWarps + (threadIdx.x >> 5)) * kHistStride : nullptr;
 }
 
-// tile: poses a lockstep block takes at a time (its first `tile` warps score them; the others
-// keep meeting the barriers); unused without lockstep.
 __global__ void __launch_bounds__(kVorWarps * 32)
-pose_kernel(DevSystem S, DevWork W, int n, int* next, uint8_t* hist_all, int tile) {
+pose_kernel(DevSystem S, DevWork W, int n, int* next, uint8_t* hist_all) {
     extern __shared__ __align__(16) unsigned char smem[];
     PoseShared& ps = reinterpret_cast<PoseShared*>(smem)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     uint8_t* hist = warp_hist(hist_all);
-    if (kLockstep) {
-        // the block takes `tile` neighbouring poses of the queue at once
-        __shared__ int base_s;
-        #pragma unroll 1
-        for (;;) {
-            if (threadIdx.x == 0) base_s = atomicAdd(next, tile);
-            __syncthreads();
-            const int base = base_s;
-            __syncthreads();
-            if (base >= n) break;
-            const int w = (int)(threadIdx.x >> 5);
-            const int q = w < tile ? base + w : n;
-            score_pose(S, W, q < n ? W.pose_order[q] : -1, lane, ps, hist, n_mobile(S));
-            __syncwarp();
-        }
-    } else {
-        #pragma unroll 1
-        for (int q = next_pose(next, lane); q < n; q = next_pose(next, lane)) {
-            score_pose(S, W, W.pose_order[q], lane, ps, hist, 0);
-            __syncwarp();
-        }
+    #pragma unroll 1
+    for (int q = next_pose(next, lane); q < n; q = next_pose(next, lane)) {
+        score_pose(S, W, W.pose_order[q], lane, ps, hist);
+        __syncwarp();
     }
 }
 
@@ -1837,102 +1606,41 @@ pose_kernel(DevSystem S, DevWork W, int n, int* next, uint8_t* hist_all, int til
 // from the job table (they stay in L1), keeping shared memory for the polyhedron workspace.
 __global__ void __launch_bounds__(kVorWarps * 32)
 pose_kernel_jobs(const Job* __restrict__ jobs, int n_jobs, int total, int* next, const int* __restrict__ order,
-                 uint8_t* hist_all, int tile) {
+                 uint8_t* hist_all) {
     extern __shared__ __align__(16) unsigned char smem[];
     PoseShared& ps = reinterpret_cast<PoseShared*>(smem)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     uint8_t* hist = warp_hist(hist_all);
-    if (kLockstep) {
-        // the block takes `tile` neighbouring poses of the queue at once and steps through as
-        // many atoms as the largest of them has
-        __shared__ int base_s, steps_s;
-        #pragma unroll 1
-        for (;;) {
-            if (threadIdx.x == 0) {
-                base_s = atomicAdd(next, tile);
-                steps_s = 0;
-            }
-            __syncthreads();
-            const int base = base_s;
-            const int w = (int)(threadIdx.x >> 5);
-            const int q = w < tile ? base + w : total;
-            int gp = -1, j = 0;
-            if (q < total) {
-                gp = order[q];
-                j = find_job(jobs, n_jobs, gp, false);
-                if (lane == 0) atomicMax(&steps_s, n_mobile(jobs[j].S));
-            }
-            __syncthreads();
-            const int steps = steps_s;
-            __syncthreads();
-            if (base >= total) break;
-            const Job& job = jobs[j];
-            score_pose(job.S, job.W, gp < 0 ? -1 : gp - job.pose0, lane, ps, hist, steps);
-            __syncwarp();
-        }
-    } else {
-        #pragma unroll 1
-        for (int q = next_pose(next, lane); q < total; q = next_pose(next, lane)) {
-            const int gp = order[q];
-            const Job& job = jobs[find_job(jobs, n_jobs, gp, false)];
-            score_pose(job.S, job.W, gp - job.pose0, lane, ps, hist, 0);
-            __syncwarp();
-        }
+    #pragma unroll 1
+    for (int q = next_pose(next, lane); q < total; q = next_pose(next, lane)) {
+        const int gp = order[q];
+        const Job& job = jobs[find_job(jobs, n_jobs, gp, false)];
+        score_pose(job.S, job.W, gp - job.pose0, lane, ps, hist);
+        __syncwarp();
     }
 }
 
-size_t pose_smem_bytes() { return sizeof(PoseShared) * kVorWarps; }
-size_t pose_jobs_smem_bytes() { return sizeof(PoseShared) * kVorWarps; }
+constexpr size_t kPoseSmem = sizeof(PoseShared) * kVorWarps;
 
-static int g_resident_blocks = 0;   // blocks of pose_kernel the device holds at once
 static int g_sms = 0, g_per_sm = 0;  // SMs, and blocks of pose_kernel one SM holds
 
-// Blocks of a launch over n poses: no more than the device holds at once (the warps take poses
-// from a queue), no more than blocks_per_sm per SM when that is set (> 0; the autotuner's
-// occupancy cap), and no more than the face history holds (hist_bytes; 0: no history).
-// Blocks a launch may run at once: as many as the device holds, no more than blocks_per_sm per
-// SM when that is set (> 0), no more than the face history holds (hist_bytes; 0: no history).
-static int pose_max_blocks(size_t hist_bytes, int blocks_per_sm) {
-    int b = g_resident_blocks > 0 ? g_resident_blocks : 1;
-    if (blocks_per_sm > 0 && g_sms > 0 && blocks_per_sm < g_per_sm && g_sms * blocks_per_sm < b)
-        b = g_sms * blocks_per_sm;
+size_t pose_hist_bytes() { return (size_t)g_sms * g_per_sm * kVorWarps * kHistStride; }
+
+// Blocks of a launch over n poses: one per kVorWarps poses, no more than the device holds at once
+// (the warps take poses from a queue), no more than blocks_per_sm per SM when that is set (> 0; the
+// autotuner's occupancy cap), and no more than the face history holds (hist_bytes; 0: no history).
+static unsigned pose_blocks(int n, size_t hist_bytes, int blocks_per_sm) {
+    int r = g_sms * (blocks_per_sm > 0 && blocks_per_sm < g_per_sm ? blocks_per_sm : g_per_sm);
     if (hist_bytes) {
         const size_t cap = hist_bytes / (kVorWarps * kHistStride);
-        if ((size_t)b > cap) b = (int)cap;
+        if ((size_t)r > cap) r = (int)cap;
     }
-    return b > 0 ? b : 1;
+    const int b = (n + kVorWarps - 1) / kVorWarps;
+    if (b < r) r = b;
+    return (unsigned)(r > 0 ? r : 1);
 }
 
-// Poses a lockstep block takes at a time (0 without lockstep): all its warps' worth, or fewer
-// when the launch's poses would not reach every block the device runs at once, so that they
-// spread over more SMs (a pose's time is its chain of atoms, shorter with fewer warps sharing the
-// SM's double-precision pipe).
-int pose_tile_for(int n, size_t hist_bytes, int blocks_per_sm) {
-    if (!kLockstep) return 0;
-    if (hist_bytes < kVorWarps * kHistStride) hist_bytes = 0;
-    const int r = pose_max_blocks(hist_bytes, blocks_per_sm);
-    const int t = (int)(((long long)n + r - 1) / r);
-    return t < 1 ? 1 : (t > kVorWarps ? kVorWarps : t);
-}
-
-// Blocks of a launch over n poses: one per tile of poses (per kVorWarps poses without lockstep),
-// no more than pose_max_blocks.
-static unsigned pose_blocks(int n, size_t hist_bytes, int blocks_per_sm) {
-    const int per = kLockstep ? pose_tile_for(n, hist_bytes, blocks_per_sm) : kVorWarps;
-    int b = (n + per - 1) / per;
-    const int r = pose_max_blocks(hist_bytes, blocks_per_sm);
-    if (b > r) b = r;
-    return (unsigned)(b > 0 ? b : 1);
-}
-
-size_t pose_hist_bytes() { return (size_t)g_resident_blocks * kVorWarps * kHistStride; }
-// The blocks of a launch.
-int pose_launch_blocks(int n, size_t hist_bytes, int blocks_per_sm) {
-    if (hist_bytes < kVorWarps * kHistStride) hist_bytes = 0;
-    return (int)pose_blocks(n, hist_bytes, blocks_per_sm);
-}
 int pose_max_blocks_per_sm() { return g_per_sm; }
-int pose_warps_per_block() { return kVorWarps; }
 
 // hist / hist_bytes: the launch's face history (reference face order), or null / 0;
 // blocks_per_sm: occupancy cap (0: as many as fit).
@@ -1941,8 +1649,7 @@ void launch_poses(const DevSystem& S, const DevWork& W, int n, int* next, uint8_
     if (hist_bytes < kVorWarps * kHistStride) hist = nullptr;
     if (!hist) hist_bytes = 0;
     cudaMemsetAsync(next, 0, sizeof(int), st);
-    pose_kernel<<<pose_blocks(n, hist_bytes, blocks_per_sm), kVorWarps * 32, pose_smem_bytes(), st>>>(
-        S, W, n, next, hist, pose_tile_for(n, hist_bytes, blocks_per_sm));
+    pose_kernel<<<pose_blocks(n, hist_bytes, blocks_per_sm), kVorWarps * 32, kPoseSmem, st>>>(S, W, n, next, hist);
 }
 
 void launch_poses_jobs(const Job* jobs, int n_jobs, int total, int* next, const int* order, uint8_t* hist,
@@ -1950,25 +1657,24 @@ void launch_poses_jobs(const Job* jobs, int n_jobs, int total, int* next, const 
     if (hist_bytes < kVorWarps * kHistStride) hist = nullptr;
     if (!hist) hist_bytes = 0;
     cudaMemsetAsync(next, 0, sizeof(int), st);
-    pose_kernel_jobs<<<pose_blocks(total, hist_bytes, blocks_per_sm), kVorWarps * 32, pose_jobs_smem_bytes(), st>>>(
-        jobs, n_jobs, total, next, order, hist, pose_tile_for(total, hist_bytes, blocks_per_sm));
+    pose_kernel_jobs<<<pose_blocks(total, hist_bytes, blocks_per_sm), kVorWarps * 32, kPoseSmem, st>>>(
+        jobs, n_jobs, total, next, order, hist);
 }
 
 cudaError_t configure_voronoi() {
-    cudaError_t e = cudaFuncSetAttribute(pose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pose_smem_bytes());
+    cudaError_t e = cudaFuncSetAttribute(pose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPoseSmem);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(pose_kernel_jobs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pose_jobs_smem_bytes());
+    e = cudaFuncSetAttribute(pose_kernel_jobs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPoseSmem);
     if (e != cudaSuccess) return e;
     int dev = 0, sms = 0, per_sm = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pose_kernel, kVorWarps * 32, pose_smem_bytes())) != cudaSuccess)
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pose_kernel, kVorWarps * 32, kPoseSmem)) != cudaSuccess)
         return e;
     g_sms = sms;
     g_per_sm = per_sm > 0 ? per_sm : 1;
-    g_resident_blocks = sms * g_per_sm;
     return cudaSuccess;
 }
 
-}  // namespace FXE_VARIANT
+}  // namespace f32
 }  // namespace fxe
