@@ -125,7 +125,7 @@ __device__ __forceinline__ double sqrt_short(double x, bool* slow) {
     return g;
 }
 
-__device__ __noinline__ double plain_div(double a, double b) { return a / b; }
-__device__ __noinline__ double plain_sqrt(double x) { return sqrt(x); }
+static __device__ __noinline__ double plain_div(double a, double b) { return a / b; }
+static __device__ __noinline__ double plain_sqrt(double x) { return sqrt(x); }
 
 }  // namespace fxe

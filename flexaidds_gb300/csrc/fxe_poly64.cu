@@ -54,23 +54,23 @@ constexpr int kWarps = 16;
 #endif
 constexpr int kWalkBudget = FXE_WALK_BUDGET;
 
-// Capacities of one polyhedron. The compact shape holds what the polyhedra of ordinary poses need
-// (on the benchmark's systems at most 73 vertices, 125 face points and 125 area items over 2,300
-// atoms; means 25, 43 and 33), and a hull walk up to the reference's abort at 200 edges (about 135
-// vertices: those past `verts` lie in storage the faces use later), in 14.1 KB per pose, so that
-// sixteen poses fit an SM. A pose one of whose atoms outgrows it is scored again, from its start, in
-// the large shape when its block is through with its tile.
+// Capacities of one polyhedron. The compact shape holds the polyhedra of ordinary poses (on the
+// benchmark's systems at most 44 vertices inside the sphere, 125 face points and 125 area items over
+// 2,300 atoms; means 17, 43 and 33) and any hull walk and its arc points (176 vertices: those past
+// `verts` lie in storage the faces use later), in 14.1 KB per pose, so that sixteen poses fit an SM. A
+// pose one of whose atoms outgrows it is scored again, from its start, in the large shape when its
+// block is through with its tile.
 template <int kV, int kX, int kP, int kI, int kN>
 struct Shape {
-    static constexpr int verts = kV;         // vertex indices are bytes (255 means "none")
-    static constexpr int walk_verts = kX;    // of the hull walk
+    static constexpr int verts = kV;         // of the faces; vertex indices are bytes (255 means "none")
+    static constexpr int walk_verts = kX;    // of the hull walk and its arc points
     static constexpr int pts = kP;
     static constexpr int items = kI;
     static constexpr int poses = kN;         // of a block at a time
     static constexpr int vwords = (kV + 31) / 32;
     static constexpr int over = kV >= kMaxVerts ? kAtomCapacity : kAtomRetry;
 };
-using Compact = Shape<104, 136, 352, 256, kWarps>;
+using Compact = Shape<104, kMaxVerts, 352, 256, kWarps>;
 using Large = Shape<kMaxVerts, kMaxVerts, kMaxFacePts, 3 * kMaxFacePts + 8, 5>;
 
 struct __align__(32) real4 {
@@ -151,7 +151,7 @@ struct Vor {
     real4 vx[Sh::verts + 2];
     union {
         struct {
-            real4 vx[Sh::walk_verts - Sh::verts + 1];   // the walk's vertices from Sh::verts on
+            real4 vx[Sh::walk_verts - Sh::verts + 1];   // the walk's vertices and arc points from Sh::verts on
             // (two spare slots: the step that reaches the 200-edge limit writes up to two edges)
             uchar4 ep[kMaxEdges + 2];      // plane0, plane1, start plane, end plane
             uchar2 es[kMaxEdges + 2];      // start vertex, end vertex
@@ -169,16 +169,22 @@ struct Vor {
     uchar4 vp[Sh::walk_verts];         // the vertex's planes (kNone = sphere)
     int cidx[kMaxCand];                // Calc index of each contact
     uint16_t foff[kMaxCand + 1];
-    uint16_t toff[kMaxCand + 1];       // per face: first triangle / arc item
-    uint16_t aoff[kMaxCand + 1];
+    union {
+        struct {
+            uint16_t toff[kMaxCand + 1];   // per face: first triangle / arc item
+            uint16_t aoff[kMaxCand + 1];
+        };
+        uint8_t elist[kMaxEdges + 8];      // before the faces: the hull edges with an end outside the sphere
+    };
     uint8_t cslot[kMaxCand];           // the contact's slot in the atom's candidate list
     uint8_t cmob[kMaxCand];            // the contact's mobile index (kNone: a rigid atom)
     uint8_t fnp[kMaxCand];
     uint8_t fseed[kMaxCand];           // the face's first vertex of three contact planes (kNone: none)
     uint8_t flag[kMaxPlanes];
-    uint8_t sprev[kMaxCand];           // per face: point 1 before a replayed stale read (kNone: none)
-    uint8_t flist[kMaxCand];           // faces whose test point is checked against the other planes
-    uint8_t elist[kMaxEdges + 8];      // the hull edges with an end outside the sphere
+    union {
+        uint8_t sprev[kMaxCand];       // per face: point 1 before a replayed stale read (kNone: none)
+        uint8_t flist[kMaxCand];       // before and after: faces whose test point is checked
+    };
     uint32_t excl[kFaceWords];         // candidates left out of the atom's list
     uint32_t cmask[kFaceWords];        // faces with a test point
     uint32_t bad[kFaceWords];          // faces whose test point lies in front of another plane
@@ -328,24 +334,61 @@ __device__ __forceinline__ real4 centre_of(const real4& pl) {
     return make_real4(-pl.x * pl.w, -pl.y * pl.w, -pl.z * pl.w, fabs(pl.w));
 }
 
-// test_point (LIB/Vcontacts.cpp:1357-1372) for several faces at once: face X = sh.flist[i], i < nf, keeps its test
-// point, held in sh.u.f.val[3i .. 3i+2], when the point lies behind every flagged contact plane
-// other than X. The (face, plane) pairs are spread over the lanes; a face with a plane in front of
-// its point gets its bit in sh.bad.
+// Test point i of the faces' inside tests (faces_inside): in double in the first half of sh.u.f.val,
+// truncated to single precision in the second (test_point_f).
 template <class Sh>
-__device__ __forceinline__ void faces_inside(Vor<Sh>& sh, int NC, int nf, int lane) {
-    if (lane < kFaceWords) sh.bad[lane] = 0u;
-    __syncwarp();
-    const int n = nf * NC;
-    const unsigned inv = NC > 1 ? 0xffffffffu / (unsigned)NC + 1u : 0u;   // k / NC for these small k
+__device__ __forceinline__ float* test_point_f(Vor<Sh>& sh, int i) { return reinterpret_cast<float*>(&sh.u.f.val[Sh::items / 2]) + 3 * i; }
+template <class Sh>
+__device__ __forceinline__ void put_test_point(Vor<Sh>& sh, int i, double x, double y, double z) {
+    double* q = &sh.u.f.val[3 * i];
+    q[0] = x;
+    q[1] = y;
+    q[2] = z;
+    float* f = test_point_f(sh, i);
+    f[0] = d2f_trunc(x);
+    f[1] = d2f_trunc(y);
+    f[2] = d2f_trunc(z);
+}
+
+template <class Sh>
+__device__ __noinline__ bool in_front_exact(const Vor<Sh>& sh, int k, const double* q) {
+    return gt0(dot3(sh.pl[k], q[0], q[1], q[2]) + sh.pl[k].w);
+}
+
+// test_point (LIB/Vcontacts.cpp:1357-1372) for several faces at once: face X = sh.flist[i], i < nf, keeps its test
+// point i when the point lies behind every flagged contact plane other than X; a face with a plane
+// in front of its point gets its bit in sh.bad. One plane per lane, decided in single precision
+// unless the value is within its error bound (as in `behind`).
+template <class Sh>
+__device__ __noinline__ void faces_inside(Vor<Sh>& sh, int NC, int nf, int lane) {
+    uint32_t bad[kFaceWords] = {0u, 0u, 0u};
     #pragma unroll 1
-    for (int k = lane; k < n; k += 32) {
-        const int fi = NC > 1 ? (int)__umulhi((unsigned)k, inv) : k, cp = k - fi * NC;
-        const int X = sh.flist[fi];
-        if (cp == X || sh.flag[cp] == 0) continue;
-        const double* q = &sh.u.f.val[3 * fi];
-        const real4 P = sh.pl[cp];
-        if (gt0(dot3(P, q[0], q[1], q[2]) + P.w)) atomicOr(&sh.bad[X >> 5], 1u << (X & 31));
+    for (int c0 = 0; nf > 0 && c0 < NC; c0 += 32) {
+        const int cp = c0 + lane;
+        const bool on = cp < NC && sh.flag[cp] != 0;
+        const real4 P = sh.pl[on ? cp : 0];
+        const float Px = d2f_trunc(P.x), Py = d2f_trunc(P.y), Pz = d2f_trunc(P.z), Pw = d2f_trunc(P.w);
+        #pragma unroll 1
+        for (int i = 0; i < nf; ++i) {
+            const int X = sh.flist[i];
+            const float* f = test_point_f(sh, i);
+            const float x = f[0], y = f[1], z = f[2];
+            const float v = fmaf(Px, x, fmaf(Py, y, fmaf(Pz, z, Pw)));
+            const float e = 0x1.0p-20f * (fabsf(Px * x) + fabsf(Py * y) + fabsf(Pz * z) + fabsf(Pw));
+            bool front = false;
+            if (on && cp != X) front = fabsf(v) > e ? v > 0.0f : in_front_exact(sh, cp, &sh.u.f.val[3 * i]);
+            if (__any_sync(kFull, front)) {
+                const uint32_t b = 1u << (X & 31);
+                if (X < 32) bad[0] |= b;
+                else if (X < 64) bad[1] |= b;
+                else bad[2] |= b;
+            }
+        }
+    }
+    if (lane == 0) {
+        sh.bad[0] = bad[0];
+        sh.bad[1] = bad[1];
+        sh.bad[2] = bad[2];
     }
     __syncwarp();
 }
@@ -398,32 +441,24 @@ __device__ __forceinline__ bool edge_flip(const Vor<Sh>& sh, int p0, int p1, int
 }
 
 // Single-precision value of vt = -(P.s + w) / (P.V) and a bound on its distance from the same
-// expression evaluated in double: every input is truncated once to float (2^-23 of it), V's
-// coordinates are within 2^-20 of the double ones, and every operation rounds (2^-24); 16 units of
-// roundoff (2^-20) per sum of absolute terms covers the rest; the quotients use
-// the fast reciprocal (at most 2 units in the last place off, covered by 4 units of |vt| and the
-// 1/16 margin on the bound). den_ok is false when the sign of P.V is not certain (the double test
-// skips P.V == 0 exactly), when |P.V| is too small for the fast quotient, or when the bound is
-// not finite.
+// expression evaluated in double. With inputs truncated to float (2^-23 of them), V's coordinates
+// within 2^-20, unit normals (the bounding planes' are 1.23 long) and roundings of 2^-24, P.V is
+// within 2.1 * 2^-20 (kDenErr: 2.5 * 2^-20) and P.s + w within 2^-20 (1.25 |s|_1 + |w|), es being
+// its first part; with |P.V| above 16 kDenErr the quotient's denominator is known to a sixteenth, and
+// the reciprocal and the two products round by less than 4 units of |vt|. *ok is false below that
+// (the double test also skips P.V == 0 exactly).
+constexpr float kDenErr = 2.5f * 0x1.0p-20f;
+__device__ __forceinline__ float start_err(float sx, float sy, float sz) {
+    return 1.25f * 0x1.0p-20f * (fabsf(sx) + fabsf(sy) + fabsf(sz));
+}
 __device__ __forceinline__ float vt_pretest(const float4& P, float sx, float sy, float sz, float Vx,
-                                            float Vy, float Vz, float* err, bool* den_ok) {
-    const float g = 9.5367431640625e-07f;   // 2^-20
-    const float den = P.x * Vx + P.y * Vy + P.z * Vz;
-    const float eden = g * (fabsf(P.x) * (fabsf(Vx) + 1.0f) + fabsf(P.y) * (fabsf(Vy) + 1.0f) + fabsf(P.z) * (fabsf(Vz) + 1.0f));
-    const float num = P.x * sx + P.y * sy + P.z * sz + P.w;
-    const float enm = g * (fabsf(P.x * sx) + fabsf(P.y * sy) + fabsf(P.z * sz) + fabsf(P.w));
-    // an all-zero normal has P.V == 0 exactly in double too, and the double test skips it; report
-    // it as a decided non-positive value
-    if (P.x == 0.0f && P.y == 0.0f && P.z == 0.0f) {
-        *den_ok = true;
-        *err = 0.0f;
-        return -1.0f;
-    }
-    const bool ok = fabsf(den) > 2.0f * eden && fabsf(den) > 1e-30f;
-    const float vt = __fdividef(-num, den);
-    const float er = __fdividef(enm + fabsf(vt) * eden, fabsf(den) - eden) * 1.0625f + fabsf(vt) * 4.8e-7f;
-    *den_ok = ok && er < 3.0e38f;
-    *err = er;
+                                            float Vy, float Vz, float es, float* err, bool* ok) {
+    const float den = fmaf(P.x, Vx, fmaf(P.y, Vy, P.z * Vz));
+    const float num = fmaf(P.x, sx, fmaf(P.y, sy, fmaf(P.z, sz, P.w)));
+    const float rd = rcp_approx(den);
+    const float vt = -num * rd, av = fabsf(vt);
+    *ok = fabsf(den) > 16.0f * kDenErr;
+    *err = fmaf(av, 4.8e-7f, fmaf(av, kDenErr, fmaf(fabsf(P.w), 0x1.0p-20f, es)) * (1.08f * fabsf(rd)));
     return vt;
 }
 
@@ -519,6 +554,7 @@ __device__ __forceinline__ WalkStep walk_step_group(const Vor<Sh>& sh, int NC, i
     const float Vx = flip ? -Vf.x : Vf.x, Vy = flip ? -Vf.y : Vf.y, Vz = flip ? -Vf.z : Vf.z;
     const float sf = d2f_trunc(sc);
     const float sx = __shfl_sync(kFull, sf, base), sy = __shfl_sync(kFull, sf, base + 1), sz = __shfl_sync(kFull, sf, base + 2);
+    const float es = start_err(sx, sy, sz);
     float best = 9.9e9f, beste = 0.0f;
     int bi = INT_MAX;
     // and the two smallest lower bounds (vt - err) over the planes whose vt may be positive: every
@@ -532,7 +568,7 @@ __device__ __forceinline__ WalkStep walk_step_group(const Vor<Sh>& sh, int NC, i
             if (k == pA || k == pB || k == oldC) continue;
             float er;
             bool ok;
-            const float vt = vt_pretest(sh.plf[k], sx, sy, sz, Vx, Vy, Vz, &er, &ok);
+            const float vt = vt_pretest(sh.plf[k], sx, sy, sz, Vx, Vy, Vz, es, &er, &ok);
             if (!ok) {
                 unsure = true;
                 continue;
@@ -580,7 +616,7 @@ __device__ __forceinline__ WalkStep walk_step_group(const Vor<Sh>& sh, int NC, i
         if (k != pA && k != pB && k != oldC) {
             float er;
             bool ok;
-            const float bt = vt_pretest(sh.plf[k], sx, sy, sz, Vx, Vy, Vz, &er, &ok);
+            const float bt = vt_pretest(sh.plf[k], sx, sy, sz, Vx, Vy, Vz, es, &er, &ok);
             need = !(ok && (bt + er <= 0.0f || bt - er > vtf * 1.0000005f));   // (vtf: truncated, 2^-23 of it)
         }
     }
@@ -760,7 +796,7 @@ __device__ __forceinline__ int hull_walk(Vor<Sh>& sh, int NC, double rr, int lan
                 pC = w.pc;
             }
             if (pC < 0) return kAtomHullFail;
-            if (vn >= Sh::walk_verts - 1) return Sh::over;
+            if (vn >= kMaxVerts - 1) return kAtomCapacity;
             const uchar4 ep = sh.u.e.ep[e];
             const int pA = ep.x, pB = ep.y;
             // edges (pA, pC) and (pB, pC): the first match after this edge, else a new edge
@@ -823,7 +859,23 @@ __device__ __forceinline__ int hull_walk(Vor<Sh>& sh, int NC, double rr, int lan
         __syncwarp();
     }
     walk = Walk{vn, edgenum, startedge};
-    return vn > Sh::verts - 1 ? Sh::over : kAtomOk;
+    return kAtomOk;
+}
+
+// Whether point x lies behind plane k (a negative value of the plane's equation), decided in single
+// precision unless the value is within its error bound (inputs truncated by 2^-23 of them, sums
+// rounded by 2^-24: 2^-20 of the sum of absolute terms covers both).
+template <class Sh>
+__device__ __noinline__ bool behind_exact(const Vor<Sh>& sh, int k, const double* x) {
+    return lt0(dot3(sh.pl[k], x[0], x[1], x[2]) + sh.pl[k].w);
+}
+template <class Sh>
+__device__ __forceinline__ bool behind(const Vor<Sh>& sh, int k, const double* x) {
+    const float4 P = sh.plf[k];
+    const float fx = d2f_trunc(x[0]), fy = d2f_trunc(x[1]), fz = d2f_trunc(x[2]);
+    const float v = fmaf(P.x, fx, fmaf(P.y, fy, fmaf(P.z, fz, P.w)));
+    const float e = 0x1.0p-20f * (fabsf(P.x * fx) + fabsf(P.y * fy) + fabsf(P.z * fz) + fabsf(P.w));
+    return fabsf(v) > e ? v < 0.0f : behind_exact(sh, k, x);
 }
 
 // Arc points where edges leave the sphere (LIB/Vcontacts.cpp:418-462), then the vertices inside it,
@@ -833,8 +885,8 @@ __device__ __forceinline__ int arc_points(Vor<Sh>& sh, double rado, double rr, i
     // vertex distances to the centre, all at once
     #pragma unroll 1
     for (int vi = lane; vi < vn; vi += 32) {
-        const real4 X = sh.vx[vi];
-        sh.vx[vi].w = dsqrt(X.x * X.x + X.y * X.y + X.z * X.z);
+        real4& X = *walk_vertex(sh, vi);
+        X.w = dsqrt(X.x * X.x + X.y * X.y + X.z * X.z);
     }
     __syncwarp();
     // the edges with an end outside the sphere listed in order, then their sphere intersections a
@@ -846,7 +898,7 @@ __device__ __forceinline__ int arc_points(Vor<Sh>& sh, double rado, double rr, i
         bool out = false;
         if (e < edgenum) {
             const uchar2 se = sh.u.e.es[e];
-            out = lt_nn(rado, sh.vx[se.x].w) || lt_nn(rado, sh.vx[se.y].w);
+            out = lt_nn(rado, walk_vertex(sh, se.x)->w) || lt_nn(rado, walk_vertex(sh, se.y)->w);
         }
         const unsigned m = __ballot_sync(kFull, out);
         if (out) sh.elist[n_out + __popc(m & lanemask_lt())] = (uint8_t)e;
@@ -863,23 +915,22 @@ __device__ __forceinline__ int arc_points(Vor<Sh>& sh, double rado, double rr, i
         if (k < n_out) {
             q = sh.u.e.ep[sh.elist[k]];
             if (solve2s(sh.pl[q.x], sh.pl[q.y], rr, a0, a1)) {
-                const real4 ta = sh.pl[q.z], tb = sh.pl[q.w];
-                k0v = lt0(dot3(ta, a0[0], a0[1], a0[2]) + ta.w) && lt0(dot3(tb, a0[0], a0[1], a0[2]) + tb.w);
-                k1v = lt0(dot3(ta, a1[0], a1[1], a1[2]) + ta.w) && lt0(dot3(tb, a1[0], a1[1], a1[2]) + tb.w);
+                k0v = behind(sh, q.z, a0) && behind(sh, q.w, a0);
+                k1v = behind(sh, q.z, a1) && behind(sh, q.w, a1);
                 cnt = (int)k0v + (int)k1v;
             }
         }
         int tot;
         const int off = warp_excl_scan(cnt, lane, &tot);
-        if (vn + tot > Sh::verts - 1) return Sh::over;
+        if (vn + tot > kMaxVerts - 1) return kAtomCapacity;
         int w = vn + off;
         if (k0v) {
-            sh.vx[w] = make_real4(a0[0], a0[1], a0[2], rado);
+            *walk_vertex(sh, w) = make_real4(a0[0], a0[1], a0[2], rado);
             sh.vp[w] = make_uchar4(q.x, q.y, kNone, 0);
             ++w;
         }
         if (k1v) {
-            sh.vx[w] = make_real4(a1[0], a1[1], a1[2], rado);
+            *walk_vertex(sh, w) = make_real4(a1[0], a1[1], a1[2], rado);
             sh.vp[w] = make_uchar4(q.x, q.y, kNone, 0);
         }
         vn += tot;
@@ -893,7 +944,7 @@ __device__ __forceinline__ int arc_points(Vor<Sh>& sh, double rado, double rr, i
         uchar4 P = make_uchar4(0, 0, 0, 0);
         bool keep = false;
         if (vi < vn) {
-            X = sh.vx[vi];
+            X = *walk_vertex(sh, vi);
             P = sh.vp[vi];
             keep = le_nn(X.w, rado);
         }
@@ -901,14 +952,14 @@ __device__ __forceinline__ int arc_points(Vor<Sh>& sh, double rado, double rr, i
         __syncwarp();
         if (keep) {
             const int w = nv + __popc(m & lanemask_lt());
-            sh.vx[w] = X;
+            if (w < Sh::verts) sh.vx[w] = X;
             sh.vp[w] = P;
         }
         nv += __popc(m);
         __syncwarp();
     }
     *nv_out = nv;
-    return kAtomOk;
+    return nv > Sh::verts - 1 ? Sh::over : kAtomOk;
 }
 
 // The first set bit at or after bit `from` of the vertex mask a & b (b may be null), or -1.
@@ -989,17 +1040,14 @@ __device__ __forceinline__ int order_faces(Vor<Sh>& sh, int NC, int NV, double r
         }
         const bool cand = face && cnt > 2 && first_arc >= 0;
         const unsigned m = __ballot_sync(kFull, cand);
-        if (3 * (nf + __popc(m)) > Sh::items) return Sh::over;
+        if (3 * (nf + __popc(m)) > Sh::items / 2) return Sh::over;
         if (lane == 0) sh.cmask[x0 >> 5] = m;
         if (cand) {
             const int fi = nf + __popc(m & lanemask_lt());
             sh.flist[fi] = (uint8_t)X;
             const real4 cp = centre_of(sh.pl[X]);
             const real4 pv = sh.vx[first_arc];
-            double* ex = &sh.u.f.val[3 * fi];
-            ex[0] = 2.0 * cp.x - pv.x;
-            ex[1] = 2.0 * cp.y - pv.y;
-            ex[2] = 2.0 * cp.z - pv.z;
+            put_test_point(sh, fi, 2.0 * cp.x - pv.x, 2.0 * cp.y - pv.y, 2.0 * cp.z - pv.z);
         }
         nf += __popc(m);
     }
@@ -1246,16 +1294,13 @@ __device__ __forceinline__ int area_items(Vor<Sh>& sh, int NC, int NV, double ra
         int ao = a_run + warp_excl_scan(na, lane, &ta);
         a_run += ta;
         const unsigned m = __ballot_sync(kFull, ring);
-        if (T + a_run > Sh::items || 3 * (nf + __popc(m)) > Sh::items) return Sh::over;
+        if (T + a_run > Sh::items || 3 * (nf + __popc(m)) > Sh::items / 2) return Sh::over;
         if (X < NC) sh.aoff[X] = (uint16_t)ao;
         if (ring) {
             const int fi = nf + __popc(m & lanemask_lt());
             sh.flist[fi] = (uint8_t)X;
             const real4 cp = centre_of(sh.pl[X]);
-            double* q = &sh.u.f.val[3 * fi];
-            q[0] = cp.x;
-            q[1] = cp.y;
-            q[2] = cp.z;
+            put_test_point(sh, fi, cp.x, cp.y, cp.z);
         }
         nf += __popc(m);
         const uint32_t self = (uint32_t)X | ((uint32_t)X << 24);
@@ -1808,7 +1853,7 @@ __device__ __forceinline__ int score_pose(const DevSystem& S, const DevWork& W, 
 }
 
 constexpr size_t kPoseSmem = sizeof(PoseShared<Compact>) * Compact::poses;
-static_assert(kPoseSmem <= 226 * 1024, "sixteen poses per SM");
+static_assert(kPoseSmem + 512 <= 227 * 1024, "sixteen poses per SM");
 static_assert(sizeof(PoseShared<Large>) * Large::poses <= kPoseSmem, "the large shape's poses fit the same block");
 
 // Poses are handed out from a queue (`next`, zeroed before the launch; order: n poses): the launch
