@@ -27,6 +27,8 @@
 #include <cstdint>
 
 #include "fxe_common.cuh"
+#include "fxe_dmath.cuh"
+#include "fxe_sort.cuh"
 
 namespace fxe {
 
@@ -65,10 +67,9 @@ __device__ __forceinline__ DrawThreshold draw_threshold(double p) {
 }
 
 constexpr int kGaThreads = 256;
-// The one-block-per-job sorts (replacement, fitness): a wider block, so that each bitonic stage
-// is a couple of exchanges per thread.
-constexpr int kGaSortThreads = 1024;
-constexpr int kGaMaxSort = 4096;   // 2P entries sorted in shared memory: P <= 2048
+// The one-block-per-job sorts (replacement, fitness).
+constexpr int kGaSortThreads = kSortThreads;
+constexpr int kGaMaxPop = 2048;
 
 // Order-preserving 64-bit image of a double that is not a NaN: the images compare as unsigned
 // integers in the order the values compare (-0 and +0, which compare equal, share one image), so
@@ -77,29 +78,6 @@ __device__ __forceinline__ uint64_t order_key(double x) {
     uint64_t b = (uint64_t)__double_as_longlong(x);
     if ((b << 1) == 0) b = 0;
     return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
-}
-
-// Ascending bitonic sort of (key, index) pairs in shared memory, n a power of two.
-__device__ void bitonic_sort(uint64_t* key, int* idx, int n) {
-    for (int k = 2; k <= n; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < n; i += blockDim.x) {
-                const int l = i ^ j;
-                if (l > i) {
-                    const bool up = (i & k) == 0;
-                    const uint64_t a = key[i], b = key[l];
-                    const int ia = idx[i], ib = idx[l];
-                    // order by key, then by index, so equal energies keep a fixed order
-                    const bool gt = a > b || (a == b && ia > ib);
-                    if (gt == up) {
-                        key[i] = b; key[l] = a;
-                        idx[i] = ib; idx[l] = ia;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
 }
 
 // roulette_wheel (LIB/gaboom.cpp:1158-1186) over the fitness in roulette order: the first
@@ -205,9 +183,65 @@ __global__ void __launch_bounds__(kGaThreads) ga_init_kernel(const GaJob* __rest
     initial_candidates(J, 0, min(J.ncand, J.gen[1]), blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
+// adapt_prob (LIB/gaboom.cpp:848-880) for parents of fitness f1 and f2.
+__device__ __forceinline__ void adapt_prob(const GaJob& J, double f1, double f2, double fit_max, double fit_avg, double* crossp,
+                                           double* mutp) {
+    const double hi = f1 > f2 ? f1 : f2, lo = f1 > f2 ? f2 : f1;
+    double denom = fit_max - fit_avg;
+    if (denom < 1e-15) denom = 1e-15;   // GA_FITNESS_DENOM_FLOOR, LIB/ga_constants.h:38
+    *crossp = hi > fit_avg ? J.k[0] * (fit_max - hi) / denom : J.k[2];
+    *mutp = lo > fit_avg ? J.k[1] * (fit_max - lo) / denom : J.k[3];
+}
+
+// The crossover's draws (LIB/gaboom.cpp:2527-2598): whether it happens, its genes and bit points.
+struct Crossover {
+    bool on;
+    int gen_a, gen_b, pnt_a, pnt_b;
+};
+template <typename Draw>
+__device__ __forceinline__ Crossover draw_crossover(const GaJob& J, Draw&& draw, double crossp) {
+    const int ng = J.ng;
+    Crossover x{false, 0, 0, 0, 0};
+    if (!(draw() < crossp)) return x;
+    x.on = true;
+    x.gen_a = (int)(draw() * (double)ng);
+    x.gen_b = (int)(draw() * (double)ng);
+    if (x.gen_a >= ng) x.gen_a = ng - 1;
+    if (x.gen_b >= ng) x.gen_b = ng - 1;
+    if (J.intragenes) {
+        x.pnt_a = (int)(draw() * 32.0);
+        x.pnt_b = (int)(draw() * 32.0);
+        if (x.gen_a > x.gen_b) {
+            const int tg = x.gen_a, tp = x.pnt_a;
+            x.gen_a = x.gen_b; x.pnt_a = x.pnt_b;
+            x.gen_b = tg; x.pnt_b = tp;
+        }
+        if (x.gen_a == x.gen_b && x.pnt_a < x.pnt_b) {
+            const int tp = x.pnt_b;
+            x.pnt_b = x.pnt_a;
+            x.pnt_a = tp;
+        }
+    } else {
+        if (x.gen_a > x.gen_b) {
+            const int tg = x.gen_a;
+            x.gen_a = x.gen_b;
+            x.gen_b = tg;
+        }
+        if (x.gen_a != x.gen_b) {
+            x.pnt_a = draw() < 0.5 ? 32 : 0;
+            x.pnt_b = draw() < 0.5 ? 32 : 0;
+            if (x.gen_b - x.gen_a == 1 && x.pnt_a == 0 && x.pnt_b == 32) x.pnt_b = x.pnt_a;
+        } else {
+            x.pnt_a = 32;
+            x.pnt_b = 0;
+        }
+    }
+    return x;
+}
+
 // One pair of children: two roulette draws, optional adaptive probabilities, crossover with
 // probability crossp, both children mutated bit by bit. draw() gives the next uniform in [0, 1)
-// of the pair's stream, in the order the reference makes its draws.
+// of the pair's draws, in the order the reference makes them.
 template <typename Draw>
 __device__ __forceinline__ void breed_pair_with(const GaJob& J, Draw&& draw, int32_t* john, int32_t* mary) {
     const int ng = J.ng;
@@ -217,65 +251,25 @@ __device__ __forceinline__ void breed_pair_with(const GaJob& J, Draw&& draw, int
     const int pb = roulette(J, draw());
     const int a = J.ford[pa], b = J.ford[pb];
     double crossp = J.cross_rate, mutp = J.mut_rate;
-    if (J.adaptive) {
-        const double f1 = J.fit[pa], f2 = J.fit[pb];
-        const double hi = f1 > f2 ? f1 : f2, lo = f1 > f2 ? f2 : f1;
-        double denom = fit_max - fit_avg;
-        if (denom < 1e-15) denom = 1e-15;   // GA_FITNESS_DENOM_FLOOR, LIB/ga_constants.h:38
-        crossp = hi > fit_avg ? J.k[0] * (fit_max - hi) / denom : J.k[2];
-        mutp = lo > fit_avg ? J.k[1] * (fit_max - lo) / denom : J.k[3];
-    }
-    const DrawThreshold mut = draw_threshold(mutp);
+    if (J.adaptive) adapt_prob(J, J.fit[pa], J.fit[pb], fit_max, fit_avg, &crossp, &mutp);
     int32_t* m = mary;
     for (int q = 0; q < ng; ++q) {
         john[q] = J.pop[(size_t)a * ng + q];
         m[q] = J.pop[(size_t)b * ng + q];
     }
-    if (draw() < crossp) {
-        // LIB/gaboom.cpp:2527-2598
-        int gen_a = (int)(draw() * (double)ng);
-        int gen_b = (int)(draw() * (double)ng);
-        if (gen_a >= ng) gen_a = ng - 1;
-        if (gen_b >= ng) gen_b = ng - 1;
-        int pnt_a, pnt_b;
-        if (J.intragenes) {
-            pnt_a = (int)(draw() * 32.0);
-            pnt_b = (int)(draw() * 32.0);
-            if (gen_a > gen_b) {
-                const int tg = gen_a, tp = pnt_a;
-                gen_a = gen_b; pnt_a = pnt_b;
-                gen_b = tg; pnt_b = tp;
-            }
-            if (gen_a == gen_b && pnt_a < pnt_b) {
-                const int tp = pnt_b;
-                pnt_b = pnt_a;
-                pnt_a = tp;
-            }
-        } else {
-            if (gen_a > gen_b) {
-                const int tg = gen_a;
-                gen_a = gen_b;
-                gen_b = tg;
-            }
-            if (gen_a != gen_b) {
-                pnt_a = draw() < 0.5 ? 32 : 0;
-                pnt_b = draw() < 0.5 ? 32 : 0;
-                if (gen_b - gen_a == 1 && pnt_a == 0 && pnt_b == 32) pnt_b = pnt_a;
-            } else {
-                pnt_a = 32;
-                pnt_b = 0;
-            }
-        }
+    const Crossover x = draw_crossover(J, draw, crossp);
+    if (x.on) {
+        const int gen_a = x.gen_a, gen_b = x.gen_b;
         for (int j = gen_a; j <= gen_b; ++j) {
-            const int np = j == gen_a ? pnt_a : 32;
+            const int np = j == gen_a ? x.pnt_a : 32;
             // the reference's mask: 1, then np times optr |= optr << 1
             const uint32_t optr = np >= 31 ? 0xFFFFFFFFu : ((2u << np) - 1u);
             const uint32_t uj = (uint32_t)john[j], um = (uint32_t)m[j];
             john[j] = (int32_t)((uj & ~optr) | (um & optr));
             m[j] = (int32_t)((uj & optr) | (um & ~optr));
         }
-        if (pnt_b > 0) {
-            const int np = pnt_b - 1;
+        if (x.pnt_b > 0) {
+            const int np = x.pnt_b - 1;
             const uint32_t optr = np >= 31 ? 0xFFFFFFFFu : ((2u << np) - 1u);
             const uint32_t uj = (uint32_t)john[gen_b], um = (uint32_t)m[gen_b];
             john[gen_b] = (int32_t)((uj & ~optr) | (um & optr));
@@ -291,7 +285,7 @@ __device__ __forceinline__ void breed_pair_with(const GaJob& J, Draw&& draw, int
             if (pr >= 0.0f && !(draw() < (double)pr)) continue;
             uint32_t optr = 0u;
             for (int bit = 0; bit < 32; ++bit)
-                if (draw.below(mut)) optr |= 1u << bit;
+                if (draw() < mutp) optr |= 1u << bit;
             ch[q] ^= (int32_t)optr;
         }
     }
@@ -301,37 +295,99 @@ __device__ __forceinline__ void breed_pair_with(const GaJob& J, Draw&& draw, int
 struct StreamDraws {
     uint64_t seed, st, d;
     __device__ __forceinline__ double operator()() { return uniform(seed, st, d++); }
-    __device__ __forceinline__ bool below(const DrawThreshold& t) { return uniform_bits(seed, st, d++) < t.bits; }
 };
 
-// Pair k of the children of generation g + 1, from the generation's counter-based stream.
-__device__ void breed_pair(const GaJob& J, int g, int k, int32_t* john, int32_t* mary) {
-    const uint64_t st = ((uint64_t)(g + 1) << 32) + (uint64_t)k;   // streams of generation g + 1
-    breed_pair_with(J, StreamDraws{J.seed, st, 0}, john, mary);
+// One gene of a child after the crossover of breed_pair_with: its own value u and its mate's.
+__device__ __forceinline__ uint32_t crossed(uint32_t own, uint32_t mate, int np) {
+    const uint32_t optr = np >= 31 ? 0xFFFFFFFFu : ((2u << np) - 1u);
+    return (own & ~optr) | (mate & optr);
+}
+
+// Pair k of the children of generation g + 1, from the generation's counter-based stream, by one
+// warp: breed_pair_with's draws in its order, the genes spread over the lanes (genes lane and
+// lane + 32; ng <= 64) and a gene's 32 mutation draws one per lane. A thread per pair made 1,216 draws
+// one after another on nine SMs (184 us per generation of 2,000); the warps spread over the device.
+// cand: the pair's two chromosomes; sig: their signatures.
+__device__ void breed_pair_warp(const GaJob& J, int g, int k, int lane, int32_t* cand, uint64_t* sig) {
+    const int ng = J.ng;
+    StreamDraws draw{J.seed, ((uint64_t)(g + 1) << 32) + (uint64_t)k, 0};   // streams of generation g + 1
+    const double fit_max = J.fstat[1], fit_avg = J.fstat[2];
+    const int pa = roulette(J, draw());
+    const int pb = roulette(J, draw());
+    const int a = J.ford[pa], b = J.ford[pb];
+    double crossp = J.cross_rate, mutp = J.mut_rate;
+    if (J.adaptive) adapt_prob(J, J.fit[pa], J.fit[pb], fit_max, fit_avg, &crossp, &mutp);
+    const DrawThreshold mut = draw_threshold(mutp);
+    const Crossover x = draw_crossover(J, draw, crossp);
+    uint32_t c0[2] = {0u, 0u}, c1[2] = {0u, 0u};
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int q = lane + 32 * h;
+        if (q < ng) {
+            uint32_t u = (uint32_t)J.pop[(size_t)a * ng + q], v = (uint32_t)J.pop[(size_t)b * ng + q];
+            if (x.on) {
+                if (q >= x.gen_a && q <= x.gen_b) {
+                    const int np = q == x.gen_a ? x.pnt_a : 32;
+                    const uint32_t t = crossed(u, v, np);
+                    v = crossed(v, u, np);
+                    u = t;
+                }
+                if (q == x.gen_b && x.pnt_b > 0) {
+                    const uint32_t t = crossed(u, v, x.pnt_b - 1);
+                    v = crossed(v, u, x.pnt_b - 1);
+                    u = t;
+                }
+            }
+            c0[h] = u;
+            c1[h] = v;
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        uint32_t* const ch = c == 0 ? c0 : c1;
+        for (int q = 0; q < ng; ++q) {
+            const float pr = J.gene_prob[q];
+            if (pr >= 0.0f && !(draw() < (double)pr)) continue;
+            const uint32_t optr = __ballot_sync(0xffffffffu, uniform_bits(draw.seed, draw.st, draw.d + lane) < mut.bits);
+            draw.d += 32;
+            if (lane == (q & 31)) {
+                if (q < 32) ch[0] ^= optr;
+                else ch[1] ^= optr;
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if (lane + 32 * h < ng) cand[c * ng + lane + 32 * h] = (int32_t)ch[h];
+        // hash_genes of the child (see signature): the lanes decode, the fold is in gene order
+        uint64_t sg = 0;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int q = lane + 32 * h;
+            const int32_t v = q < ng ? (int32_t)(gene_ic(J, q, (int32_t)ch[h]) + 0.5) : 0;
+            for (int i = 32 * h; i < ng && i < 32 * h + 32; ++i)
+                sg ^= (uint64_t)(int64_t)__shfl_sync(0xffffffffu, v, i & 31) + 0x9e3779b9ull + (sg << 6) + (sg >> 2);
+        }
+        if (lane == 0) sig[c] = sg;
+    }
 }
 
 // Pairs k0 .. k0 + npairs - 1 of the running generation's children as candidates, with their
-// signatures.
-// (the pairs first, first + stride, ... of the batch: the threads of a block, or of a grid)
-__device__ void bred_candidates(const GaJob& J, int g, long long k0, int npairs, int first, int stride) {
-    const int ng = J.ng;
-    for (int k = first; k < npairs; k += stride) {
-        int32_t* john = J.cand + (size_t)(2 * k) * ng;
-        int32_t* mary = john + ng;
-        breed_pair(J, g, (int)(k0 + k), john, mary);
-        J.cand_sig[2 * k] = signature(J, john);
-        J.cand_sig[2 * k + 1] = signature(J, mary);
-    }
+// signatures: the pairs first, first + stride, ... of the batch, one warp each (of a block, or of a grid).
+__device__ void bred_candidates(const GaJob& J, int g, long long k0, int npairs, int first, int stride, int lane) {
+    for (int k = first; k < npairs; k += stride)
+        breed_pair_warp(J, g, (int)(k0 + k), lane, J.cand + (size_t)(2 * k) * J.ng, J.cand_sig + 2 * k);
 }
 
 __global__ void __launch_bounds__(kGaThreads) ga_breed_kernel(const GaJob* __restrict__ all, const int* __restrict__ run) {
     const GaJob& J = all[run[blockIdx.y]];
-    bred_candidates(J, J.gen[0], 0, min(J.ncand, J.gen[1]), blockIdx.x * blockDim.x + threadIdx.x,
-                    gridDim.x * blockDim.x);
+    bred_candidates(J, J.gen[0], 0, min(J.ncand, J.gen[1]), (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)),
+                    (int)(gridDim.x * (blockDim.x >> 5)), threadIdx.x & 31);
 }
 
 // Blocks per job of the first candidate batch (pairs up to P + 8 with P <= 2048; one pair per thread).
 constexpr int kGaBatchBlocks = (2048 + 8 + kGaThreads - 1) / kGaThreads;
+// Blocks per job of the breeding kernel: a warp per pair, over the device's SMs when a job runs alone.
+constexpr int kBreedBlocks = (2048 + 8) / (kGaThreads / 32);
 
 constexpr int kGaMaxBatches = 16;   // candidate batches before duplicates are let through
 
@@ -341,23 +397,28 @@ constexpr int kGaMaxBatches = 16;   // candidate batches before duplicates are l
 // at a time, candidate c is taken exactly when its signature is in neither the set the batch
 // started from nor at an earlier candidate of the batch (an earlier copy joined the set or was in
 // it), up to the candidate that completes the generation; candidates after it are not looked at.
-// So the block decides all of a batch's candidates at once: the first occurrences by a sort of
-// (signature, index) pairs in shared memory, the set by read-only probes, the cut by an ordered
-// scan; then it copies the taken ones into place and inserts their signatures. When a batch runs
+// So the block decides all of a batch's candidates at once: the first occurrences by a hash table of
+// (signature, lowest index) in shared memory, the set by read-only probes, the cut by an ordered
+// scan; then it copies the taken ones into place and inserts their signatures. (A bitonic sort of the
+// signatures in the table's place took most of the kernel's 145 us at 2,000 children.) When a batch runs
 // out, the block breeds the next batch of pairs. After kGaMaxBatches batches candidates are taken
 // as they come (counted in gen[2]), where the reference would loop until mutation finds new genes.
 // gen[1] sizes the next generation's first batch from what this one used; gen[3] counts rejected
 // candidates.
 constexpr int kAcceptThreads = 1024;
-constexpr int kAcceptSort = 8192;                  // >= 2 (P + 8) candidates with P <= 2048
-constexpr size_t kAcceptSmem = (size_t)kAcceptSort * (sizeof(uint64_t) + sizeof(uint16_t)) + kAcceptSort;
+constexpr int kAcceptMax = 2 * (kGaMaxPop + 8);    // candidates of a batch
+constexpr int kAcceptTable = 8192;                 // hash slots: at most half of them taken
+static_assert(kAcceptTable >= kAcceptMax * 3 / 2 && kAcceptTable <= 65536, "");
+constexpr size_t kAcceptSmem = (size_t)kAcceptTable * (sizeof(uint64_t) + sizeof(int)) + (size_t)kAcceptMax * (sizeof(uint16_t) + 1);
 
 template <bool kInitial>
 __global__ void __launch_bounds__(kAcceptThreads) ga_accept_kernel(const GaJob* __restrict__ all, const int* __restrict__ run) {
     extern __shared__ __align__(16) unsigned char acc_smem[];
-    uint64_t* skey = reinterpret_cast<uint64_t*>(acc_smem);
-    uint16_t* sidx = reinterpret_cast<uint16_t*>(skey + kAcceptSort);
-    uint8_t* take = reinterpret_cast<uint8_t*>(sidx + kAcceptSort);
+    unsigned long long* hkey = reinterpret_cast<unsigned long long*>(acc_smem);
+    int* hidx = reinterpret_cast<int*>(hkey + kAcceptTable);
+    uint16_t* place = reinterpret_cast<uint16_t*>(hidx + kAcceptTable);   // a candidate's slot, then its rank
+    uint8_t* take = reinterpret_cast<uint8_t*>(place + kAcceptMax);
+    __shared__ int s_zero;
     __shared__ int wsum[kAcceptThreads / 32];
     __shared__ int s_cut, s_taken, s_rej;
     const GaJob& J = all[run[blockIdx.x]];
@@ -374,37 +435,32 @@ __global__ void __launch_bounds__(kAcceptThreads) ga_accept_kernel(const GaJob* 
         if (force) {
             for (int c = tid; c < ncb; c += kAcceptThreads) take[c] = 1;
         } else {
-            int n2 = 1;
-            while (n2 < ncb) n2 <<= 1;
-            for (int k = tid; k < n2; k += kAcceptThreads) {
-                skey[k] = k < ncb ? J.cand_sig[k] : ~0ull;
-                sidx[k] = (uint16_t)k;
+            for (int k = tid; k < kAcceptTable; k += kAcceptThreads) {
+                hkey[k] = 0ull;
+                hidx[k] = 0x7fffffff;
+            }
+            if (tid == 0) s_zero = 0x7fffffff;
+            __syncthreads();
+            // (0 marks an empty slot: that signature has a counter of its own)
+            for (int c = tid; c < ncb; c += kAcceptThreads) {
+                const unsigned long long h = J.cand_sig[c];
+                if (h == 0ull) {
+                    atomicMin(&s_zero, c);
+                    continue;
+                }
+                int i = (int)(mix64(h) & (kAcceptTable - 1));
+                for (int n = 0; n < kAcceptTable; ++n, i = (i + 1) & (kAcceptTable - 1)) {
+                    const unsigned long long prev = atomicCAS(&hkey[i], 0ull, h);
+                    if (prev == 0ull || prev == h) break;
+                }
+                atomicMin(&hidx[i], c);
+                place[c] = (uint16_t)i;
             }
             __syncthreads();
-            for (int len = 2; len <= n2; len <<= 1)
-                for (int j = len >> 1; j > 0; j >>= 1) {
-                    for (int k = tid; k < n2; k += kAcceptThreads) {
-                        const int l = k ^ j;
-                        if (l > k) {
-                            const bool up = (k & len) == 0;
-                            const uint64_t ka = skey[k], kb = skey[l];
-                            const bool gt = ka > kb || (ka == kb && sidx[k] > sidx[l]);
-                            if (gt == up) {
-                                skey[k] = kb;
-                                skey[l] = ka;
-                                const uint16_t t = sidx[k];
-                                sidx[k] = sidx[l];
-                                sidx[l] = t;
-                            }
-                        }
-                    }
-                    __syncthreads();
-                }
-            for (int k = tid; k < n2; k += kAcceptThreads) {
-                const int c = sidx[k];
-                if (c >= ncb) continue;
-                const bool first = k == 0 || skey[k] != skey[k - 1];
-                take[c] = first && !seen_contains(J, skey[k]) ? 1 : 0;
+            for (int c = tid; c < ncb; c += kAcceptThreads) {
+                const unsigned long long h = J.cand_sig[c];
+                const bool first = (h == 0ull ? s_zero : hidx[place[c]]) == c;
+                take[c] = first && !seen_contains(J, h) ? 1 : 0;
             }
         }
         __syncthreads();
@@ -444,8 +500,7 @@ __global__ void __launch_bounds__(kAcceptThreads) ga_accept_kernel(const GaJob* 
         for (int c = c0; c < c1 && c <= cut; ++c) {
             if (c >= ncb) break;
             if (take[c]) {
-                const int slot = i + rank;
-                for (int q = 0; q < ng; ++q) J.child[(size_t)slot * ng + q] = J.cand[(size_t)c * ng + q];
+                place[c] = (uint16_t)rank;
                 if (!force) seen_insert_concurrent(J, J.cand_sig[c]);
                 ++rank;
                 ++my_taken;
@@ -456,6 +511,12 @@ __global__ void __launch_bounds__(kAcceptThreads) ga_accept_kernel(const GaJob* 
         if (my_taken) atomicAdd(&s_taken, my_taken);
         if (my_rej) atomicAdd(&s_rej, my_rej);
         __syncthreads();
+        const int n_copy = min(cut + 1, ncb) * ng;
+        const unsigned inv = ng > 1 ? 0xffffffffu / (unsigned)ng + 1u : 0u;   // t / ng for these small t
+        for (int t = tid; t < n_copy; t += kAcceptThreads) {
+            const int c = ng > 1 ? (int)__umulhi((unsigned)t, inv) : t;
+            if (take[c]) J.child[(size_t)(i + place[c]) * ng + (t - c * ng)] = J.cand[t];
+        }
         const int taken = s_taken;
         if (J.reject && force) forced += taken;
         rejected += s_rej;
@@ -467,7 +528,7 @@ __global__ void __launch_bounds__(kAcceptThreads) ga_accept_kernel(const GaJob* 
         base += 2 * npairs;
         npairs = J.ncand;
         if (kInitial) initial_candidates(J, base, npairs, threadIdx.x, blockDim.x);
-        else bred_candidates(J, g, base >> 1, npairs, threadIdx.x, blockDim.x);
+        else bred_candidates(J, g, base >> 1, npairs, warp, kAcceptThreads / 32, lane);
         __syncthreads();
     }
     if (threadIdx.x == 0) {
@@ -487,12 +548,17 @@ __global__ void __launch_bounds__(kAcceptThreads) ga_accept_kernel(const GaJob* 
 // Selection. kInitial: the evaluated initial population becomes generation 0. Otherwise the
 // replacement: BOOM merges the P parents and nnew children, STEADY keeps the best P - nnew
 // parents with the children in the places of the worst (child i at place P - 1 - i); the merged
-// set is sorted by energy, the best P kept, saved as the generation's snapshot, and the
-// generation counter advanced.
+// set is ordered by energy (equal energies by place, parents first), the best P kept, saved as the
+// generation's snapshot, and the generation counter advanced. The parents are in order already: the
+// children are sorted, and every entry's place in the merged order is its own place plus the entries
+// of the other list before it, found by binary search.
 template <bool kInitial>
 __global__ void __launch_bounds__(kGaSortThreads) ga_select_kernel(GaJob* __restrict__ all, const int* __restrict__ run) {
-    __shared__ uint64_t key[kGaMaxSort];
-    __shared__ int idx[kGaMaxSort];
+    extern __shared__ __align__(16) unsigned char sel_smem[];
+    uint64_t* const ckey = reinterpret_cast<uint64_t*>(sel_smem);   // the children, sorted
+    uint64_t* const pkey = ckey + kGaMaxPop;                        // the parents
+    int* const cidx = reinterpret_cast<int*>(pkey + kGaMaxPop);
+    int* const idx = cidx + kGaMaxPop;                              // the entry at each new place
     GaJob& J = all[run[blockIdx.x]];
     const int P = J.P, ng = J.ng, nnew = J.nnew;
     const int g = J.gen[0];
@@ -502,29 +568,45 @@ __global__ void __launch_bounds__(kGaSortThreads) ga_select_kernel(GaJob* __rest
     double* const nxt_e = J.pop_e_next;
     // entries: parents [0, np_), then children; idx >= np_ names a child
     const int np_ = kInitial ? 0 : (J.steady ? P - nnew : P);
-    const int m = kInitial ? P : np_ + nnew;
-    int n = 1;
-    while (n < m) n <<= 1;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        double e = INFINITY;
-        int id = i;
-        if (i < m) {
-            // STEADY: the place P-1-c holds child c
-            const int c = kInitial ? i : (J.steady ? (P - 1 - i) : (i - np_));
-            e = i < np_ ? pe[i] : J.child_cf[c].evalue;
-            if (e != e) e = INFINITY;   // a NaN energy sorts last
-            id = i;
+    const int nc = kInitial ? P : nnew;
+    for (int i = threadIdx.x; i < nc; i += blockDim.x) {
+        const int id = np_ + i;
+        // STEADY: the place P-1-c holds child c
+        const int c = kInitial ? id : (J.steady ? (P - 1 - id) : i);
+        double e = J.child_cf[c].evalue;
+        if (e != e) e = INFINITY;   // a NaN energy sorts last
+        ckey[i] = order_key(e);
+        cidx[i] = id;
+    }
+    for (int i = threadIdx.x; i < np_; i += blockDim.x) pkey[i] = order_key(pe[i]);
+    block_sort(ckey, cidx, nc);
+    for (int i = threadIdx.x; i < np_; i += blockDim.x) {
+        const uint64_t k = pkey[i];
+        int lo = 0, hi = nc;   // children below k
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (ckey[mid] < k) lo = mid + 1;
+            else hi = mid;
         }
-        key[i] = order_key(e);
-        idx[i] = id;
+        if (i + lo < P) idx[i + lo] = i;
+    }
+    for (int i = threadIdx.x; i < nc; i += blockDim.x) {
+        const uint64_t k = ckey[i];
+        int lo = 0, hi = np_;   // parents at or below k
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (pkey[mid] <= k) lo = mid + 1;
+            else hi = mid;
+        }
+        if (i + lo < P) idx[i + lo] = cidx[i];
     }
     __syncthreads();
-    bitonic_sort(key, idx, n);
     // the new population, and (after a generation) its snapshot for the ensemble
     int32_t* const sg = kInitial ? nullptr : J.snap + (size_t)g * P * ng;
     double* const se = kInitial ? nullptr : J.snap_e + (size_t)g * P;
+    const unsigned inv = ng > 1 ? 0xffffffffu / (unsigned)ng + 1u : 0u;   // t / ng for these small t
     for (int t = threadIdx.x; t < P * ng; t += blockDim.x) {
-        const int r = t / ng, q = t - r * ng;
+        const int r = ng > 1 ? (int)__umulhi((unsigned)t, inv) : t, q = t - r * ng;
         const int src = idx[r];
         const int c = kInitial ? src : (J.steady ? (P - 1 - src) : (src - np_));
         const int32_t v = src < np_ ? pop[(size_t)src * ng + q] : J.child[(size_t)c * ng + q];
@@ -564,40 +646,113 @@ __global__ void __launch_bounds__(kGaThreads) ga_decode_kernel(const GaJob* __re
     }
 }
 
-constexpr int kNicheWarps = 8;
-constexpr int kNicheBlocks = (2048 + kNicheWarps - 1) / kNicheWarps;
+constexpr int kNicheRows = 8;              // chromosomes of a block
+constexpr int kNicheChunk = 256;           // others taken at a time (one per thread)
+constexpr int kNicheBlocks = (kGaMaxPop + kNicheRows - 1) / kNicheRows;
 
 // Niche count of chromosome i: the sum over all j of 1 - (rmsp / sig_share)^alpha where rmsp
 // (calc_rmsp, LIB/gaboom.cpp:2874-2885: root mean square of the IC differences) is within
-// sig_share (LIB/gaboom.cpp:1652-1661). One warp per i: the lanes form the terms of 32 j's at a
-// time, and the sum takes them in j order (a pair beyond sig_share adds 0, which changes no sum
-// of these non-negative terms), so every count is the one a thread walking j in order forms.
-__global__ void __launch_bounds__(kNicheWarps * 32) ga_niche_kernel(const GaJob* __restrict__ all, const int* __restrict__ run) {
+// sig_share (LIB/gaboom.cpp:1652-1661). A pair beyond sig_share adds 0, which changes no sum of
+// these non-negative terms, so only the pairs within it, in j order, need the double arithmetic:
+// every pair's distance is formed in single precision with a bound on its error, the pairs not
+// surely beyond sig_share are listed and evaluated in double by full warps, and each row's terms
+// are added in j order, the block's eight rows on eight lanes. The FP64 unit (2 lanes per clock and
+// SM) bounded the form that evaluated every pair in double: 0.87 ms per generation at P = 2,000.
+//
+// Bound: with coordinates truncated to float (2^-23 of them) the distance's square root moves by at
+// most 2^-23 (|x_i| + |x_j|) and its rounding by 2^-21 of it, so a pair whose float distance is above
+// sqrt(ng) sig + 2^-22 (|x_i|_1 + |x_j|_1), by one part in 10^5, is beyond sig_share also in double.
+__global__ void __launch_bounds__(kNicheChunk) ga_niche_kernel(const GaJob* __restrict__ all, const int* __restrict__ run) {
+    __shared__ float xi[kNicheRows][64];
+    __shared__ float ni[kNicheRows];
+    __shared__ uint32_t mask[kNicheRows][kNicheChunk / 32];   // pairs listed
+    __shared__ uint16_t list[kNicheRows * kNicheChunk];
+    __shared__ double term[kNicheRows][kNicheChunk + 1];
+    __shared__ int n_list;
     const GaJob& J = all[run[blockIdx.y]];
-    const int i = blockIdx.x * kNicheWarps + (int)(threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (J.fitness == kFitLinear || i >= J.P) return;
-    const int ng = J.ng, P = J.P;
-    const double* xi = J.pic + (size_t)i * ng;
+    const int ng = J.ng, P = J.P, i0 = blockIdx.x * kNicheRows;
+    if (J.fitness == kFitLinear || i0 >= P) return;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int rows = min(kNicheRows, P - i0);
     const double sig = J.sig_share, alpha = J.share_alpha;
-    double s = 0.0;
-    for (int j0 = 0; j0 < P; j0 += 32) {
-        const int j = j0 + lane;
-        double term = 0.0;
-        if (j < P) {
-            const double* xj = J.pic + (size_t)j * ng;
-            double acc = 0.0;
-            for (int q = 0; q < ng; ++q) {
-                const double dq = xi[q] - xj[q];
-                acc += dq * dq;
-            }
-            const double r = sqrt(acc / (double)ng);
-            if (r <= sig) term = 1.0 - (alpha == 1.0 ? r / sig : pow(r / sig, alpha));
-        }
-        const int m = P - j0 < 32 ? P - j0 : 32;
-        for (int k = 0; k < m; ++k) s += __shfl_sync(0xffffffffu, term, k);
+    const float lim0 = (float)(sqrt((double)ng) * sig) * 1.00001f;
+    const bool f32 = ng <= 64;          // (longer rows than the staging's: every pair in double)
+    for (int k = t; f32 && k < rows * ng; k += kNicheChunk) {
+        const int r = k / ng;
+        xi[r][k - r * ng] = d2f_trunc(J.pic[(size_t)i0 * ng + k]);
     }
-    if (lane == 0) J.share[i] = s;
+    __syncthreads();
+    if (t < rows) {
+        float n = 0.0f;
+        for (int q = 0; f32 && q < ng; ++q) n += fabsf(xi[t][q]);
+        ni[t] = n;
+    }
+    double sum = 0.0;   // warp 0, lane r: row r
+    for (int j0 = 0; j0 < P; j0 += kNicheChunk) {
+        const int j = j0 + t;
+        float acc[kNicheRows];
+#pragma unroll
+        for (int r = 0; r < kNicheRows; ++r) acc[r] = 0.0f;
+        float nj = 0.0f;
+        if (t == 0) n_list = 0;
+        __syncthreads();
+        if (f32 && j < P) {
+            const double* xj = J.pic + (size_t)j * ng;
+            for (int q = 0; q < ng; ++q) {
+                const float x = d2f_trunc(xj[q]);
+                nj += fabsf(x);
+#pragma unroll
+                for (int r = 0; r < kNicheRows; ++r) {
+                    const float d = xi[r][q] - x;
+                    acc[r] = fmaf(d, d, acc[r]);
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < kNicheRows; ++r) {
+            const float lim = lim0 + 0x1.0p-22f * 1.00001f * (r < rows ? ni[r] + nj : 0.0f);
+            const bool near = j < P && r < rows && !(f32 && acc[r] > lim * lim * 1.00002f);
+            const unsigned m = __ballot_sync(0xffffffffu, near);
+            int at = 0;
+            if (lane == 0) {
+                mask[r][warp] = m;
+                if (m) at = atomicAdd(&n_list, __popc(m));
+            }
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (near) list[at + __popc(m & lanemask_lt())] = (uint16_t)(r << 8 | t);
+        }
+        __syncthreads();
+        const int n = n_list;
+        for (int k = t; k < n; k += kNicheChunk) {
+            const int r = list[k] >> 8, c = list[k] & 255;
+            const double* a = J.pic + (size_t)(i0 + r) * ng;
+            const double* b = J.pic + (size_t)(j0 + c) * ng;
+            double s = 0.0;
+            for (int q = 0; q < ng; ++q) {
+                const double dq = a[q] - b[q];
+                s = __fma_rn(dq, dq, s);
+            }
+            bool slow;
+            double v = div_short(s, (double)ng, &slow);
+            if (slow) v = plain_div(s, (double)ng);
+            double d = sqrt_short(v, &slow);
+            if (slow) d = plain_sqrt(v);
+            double w = 0.0;
+            if (d <= sig) {
+                double x = div_short(d, sig, &slow);
+                if (slow) x = plain_div(d, sig);
+                w = 1.0 - (alpha == 1.0 ? x : pow(x, alpha));
+            }
+            term[r][c] = w;
+        }
+        __syncthreads();
+        if (warp == 0 && lane < rows) {
+            for (int w = 0; w < kNicheChunk / 32; ++w)
+                for (uint32_t m = mask[lane][w]; m; m &= m - 1) sum += term[lane][32 * w + __ffs(m) - 1];
+        }
+        __syncthreads();
+    }
+    if (warp == 0 && lane < rows) J.share[i0 + lane] = sum;
 }
 
 // Running sums of the fitness in roulette order (roullete_wheel's walk, LIB/gaboom.cpp:1158-1186)
@@ -627,13 +782,18 @@ __device__ void fitness_sums(const GaJob& J, const double* fit, int P) {
 }
 
 // Fitness of the population (sorted by energy), the roulette order, running sums and
-// fitness_stats. kInitial: the initial population, walked in energy order whatever the model.
+// fitness_stats. kInitial: the initial population, walked in energy order whatever the model. The
+// running sum is a chain of additions in the reference's order (70 cycles each): one thread makes
+// nothing else, out of and into shared memory, while the block finds the maximum.
 template <bool kInitial>
 __global__ void __launch_bounds__(kGaSortThreads) ga_fitness_kernel(const GaJob* __restrict__ all, const int* __restrict__ run) {
-    // P <= kGaMaxSort / 2: the fitness, the sort keys (then the sorted fitness) and the order
-    __shared__ double fval[kGaMaxSort / 2];
-    __shared__ uint64_t key[kGaMaxSort / 2];
-    __shared__ int idx[kGaMaxSort / 2];
+    // the fitness (then its running sums), the sort keys (then the sorted fitness) and the order
+    extern __shared__ __align__(16) unsigned char fit_smem[];
+    double* const fval = reinterpret_cast<double*>(fit_smem);
+    uint64_t* const key = reinterpret_cast<uint64_t*>(fval + kGaMaxPop);
+    int* const idx = reinterpret_cast<int*>(key + kGaMaxPop);
+    __shared__ uint64_t max_key[kGaSortThreads / 32];
+    __shared__ int max_at[kGaSortThreads / 32];
     const GaJob& J = all[run[blockIdx.x]];
     const int P = J.P, model = J.fitness;
     const bool rank_only = model == kFitLinear || (model == kFitSmfree && !(J.beta > 0.0));
@@ -660,52 +820,106 @@ __global__ void __launch_bounds__(kGaSortThreads) ga_fitness_kernel(const GaJob*
     const bool sorted = !kInitial && model == kFitPshare;
     if (sorted) {
         // QuickSort by fitness, descending (LIB/gaboom.cpp:499); equal fitness keeps energy order
-        int n = 1;
-        while (n < P) n <<= 1;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            key[i] = i < P ? order_key(-fval[i]) : order_key(INFINITY);
-            idx[i] = i;
-        }
-        __syncthreads();
-        bitonic_sort(key, idx, n);
+        for (int i = threadIdx.x; i < P; i += blockDim.x) key[i] = order_key(-fval[i]);
+        block_sort(key, idx, P);
     }
     double* const fs = reinterpret_cast<double*>(key);   // the fitness in roulette order
-    for (int i = threadIdx.x; i < P; i += blockDim.x) {
-        const double f = fval[sorted ? idx[i] : i];
+    double mine[2] = {0.0, 0.0};
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int i = threadIdx.x + kGaSortThreads * e;
+        if (i < P) mine[e] = fval[sorted ? idx[i] : i];
+    }
+    __syncthreads();
+    // the largest value, the first of equal ones, on the order keys (a NaN never compares greater;
+    // one in the first place stays)
+    uint64_t mk = 0;
+    int mi = 0x7fffffff;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int i = threadIdx.x + kGaSortThreads * e;
+        if (i >= P) continue;
+        const double f = mine[e];
         fs[i] = f;
         J.fit[i] = f;
         J.ford[i] = idx[i];
+        const bool nan = ((uint64_t)__double_as_longlong(f) << 1) > (0x7FF0000000000000ull << 1);
+        const uint64_t k = i == 0 && nan ? ~0ull : order_key(f);
+        if ((!nan || i == 0) && (k > mk || (k == mk && i < mi))) {
+            mk = k;
+            mi = i;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const uint64_t k2 = __shfl_xor_sync(0xffffffffu, (unsigned long long)mk, o);
+        const int i2 = __shfl_xor_sync(0xffffffffu, mi, o);
+        if (k2 > mk || (k2 == mk && i2 < mi)) {
+            mk = k2;
+            mi = i2;
+        }
+    }
+    if ((threadIdx.x & 31) == 0) {
+        max_key[threadIdx.x >> 5] = mk;
+        max_at[threadIdx.x >> 5] = mi;
     }
     __syncthreads();
-    if (threadIdx.x == 0) fitness_sums(J, fs, P);
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kGaSortThreads / 32; ++w)
+            if (max_key[w] > mk || (max_key[w] == mk && max_at[w] < mi)) {
+                mk = max_key[w];
+                mi = max_at[w];
+            }
+        double cum = 0.0;
+#pragma unroll 8
+        for (int i = 0; i < P; ++i) {
+            cum += fs[i];
+            fval[i] = cum;
+        }
+        J.fstat[0] = cum;
+        J.fstat[1] = fs[mi];
+        J.fstat[2] = cum / (double)P;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < P; i += blockDim.x) J.fcum[i] = fval[i];
 }
 
-void launch_ga_fitness(const GaJob* all, const int* run, int n_jobs, bool initial, cudaStream_t st) {
-    ga_decode_kernel<<<dim3(8, n_jobs), kGaThreads, 0, st>>>(all, run);
-    ga_niche_kernel<<<dim3(kNicheBlocks, n_jobs), kNicheWarps * 32, 0, st>>>(all, run);
-    if (initial) ga_fitness_kernel<true><<<n_jobs, kGaSortThreads, 0, st>>>(all, run);
-    else ga_fitness_kernel<false><<<n_jobs, kGaSortThreads, 0, st>>>(all, run);
-}
+constexpr int kDecodeBlocks = 152;
+constexpr size_t kFitSmem = (size_t)kGaMaxPop * (2 * sizeof(uint64_t) + sizeof(int));
+constexpr size_t kSelSmem = (size_t)kGaMaxPop * (2 * sizeof(uint64_t) + 2 * sizeof(int));
 
-// The acceptance kernels' shared memory (beyond the default 48 KB), allowed once per device.
-static void accept_smem_attribute() {
+// The acceptance and selection kernels' shared memory (at or beyond the default 48 KB), allowed once
+// per device.
+static void ga_smem_attributes() {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
     static bool done[64] = {false};
     if (done[dev]) return;
     cudaFuncSetAttribute(ga_accept_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAcceptSmem);
     cudaFuncSetAttribute(ga_accept_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAcceptSmem);
+    cudaFuncSetAttribute(ga_select_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSelSmem);
+    cudaFuncSetAttribute(ga_select_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSelSmem);
+    cudaFuncSetAttribute(ga_fitness_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFitSmem);
+    cudaFuncSetAttribute(ga_fitness_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFitSmem);
     done[dev] = true;
+}
+
+void launch_ga_fitness(const GaJob* all, const int* run, int n_jobs, bool initial, cudaStream_t st) {
+    // (a gene's decode is a chain of table reads: a thread each keeps more of them in flight)
+    ga_decode_kernel<<<dim3(kDecodeBlocks, n_jobs), kGaThreads, 0, st>>>(all, run);
+    ga_niche_kernel<<<dim3(kNicheBlocks, n_jobs), kNicheChunk, 0, st>>>(all, run);
+    if (initial) ga_fitness_kernel<true><<<n_jobs, kGaSortThreads, kFitSmem, st>>>(all, run);
+    else ga_fitness_kernel<false><<<n_jobs, kGaSortThreads, kFitSmem, st>>>(all, run);
 }
 
 void launch_ga_init(const GaJob* all, const int* run, int n_jobs, cudaStream_t st) {
     ga_init_kernel<<<dim3(2 * kGaBatchBlocks, n_jobs), kGaThreads, 0, st>>>(all, run);
-    accept_smem_attribute();
+    ga_smem_attributes();
     ga_accept_kernel<true><<<n_jobs, kAcceptThreads, kAcceptSmem, st>>>(all, run);
 }
 void launch_ga_breed(const GaJob* all, const int* run, int n_jobs, cudaStream_t st) {
-    ga_breed_kernel<<<dim3(kGaBatchBlocks, n_jobs), kGaThreads, 0, st>>>(all, run);
-    accept_smem_attribute();
+    ga_breed_kernel<<<dim3(kBreedBlocks, n_jobs), kGaThreads, 0, st>>>(all, run);
+    ga_smem_attributes();
     ga_accept_kernel<false><<<n_jobs, kAcceptThreads, kAcceptSmem, st>>>(all, run);
 }
 // Breeding with the caller's draws (fxe_ga_breed_draws): J.fit and J.ford given, one block forms
@@ -728,7 +942,6 @@ __global__ void __launch_bounds__(kGaThreads) ga_breed_draws_kernel(const GaJob*
             if (d >= stride) { over = true; return 0.0; }
             return row[d++];
         }
-        __device__ bool below(const DrawThreshold& t) { return (*this)() < t.p; }
     } draw{draws + (size_t)k * stride, stride, 0, false};
     int32_t* john = J.child + (size_t)(2 * k) * J.ng;
     breed_pair_with(J, draw, john, john + J.ng);
@@ -744,12 +957,13 @@ void launch_ga_breed_draws(const GaJob* J, const double* draws, long long stride
 // Niche counts of a population whose ICs are given (fxe_ga_niche_counts): the generation's kernel
 // on one job.
 void launch_ga_niche(const GaJob* all, const int* run, cudaStream_t st) {
-    ga_niche_kernel<<<dim3(kNicheBlocks, 1), kNicheWarps * 32, 0, st>>>(all, run);
+    ga_niche_kernel<<<dim3(kNicheBlocks, 1), kNicheChunk, 0, st>>>(all, run);
 }
 
 void launch_ga_select(GaJob* all, const int* run, int n_jobs, bool initial, cudaStream_t st) {
-    if (initial) ga_select_kernel<true><<<n_jobs, kGaSortThreads, 0, st>>>(all, run);
-    else ga_select_kernel<false><<<n_jobs, kGaSortThreads, 0, st>>>(all, run);
+    ga_smem_attributes();
+    if (initial) ga_select_kernel<true><<<n_jobs, kGaSortThreads, kSelSmem, st>>>(all, run);
+    else ga_select_kernel<false><<<n_jobs, kGaSortThreads, kSelSmem, st>>>(all, run);
 }
 
 }  // namespace fxe
