@@ -112,6 +112,8 @@ __device__ __forceinline__ void build_pose(const DevSystem& S, const DevWork& W,
     if (lane == 0) {
         W.pose_grid[p] = make_int4(alter ? 1 : 0, dim, sh.bad, 0);
         W.pose_gmin[p] = make_float4(gmin[0], gmin[1], gmin[2], 0.0f);
+        W.pose_cost[p] = 0;
+        W.pose_clash[p] = 0.0f;
     }
 }
 

@@ -663,6 +663,8 @@ fxe_status context_create(const fxe_receptor_desc* rec, const fxe_context* share
         FXE_TRY(ctx->alloc(&W.pose_rec, P * fxe::kMaxLig * fxe::kMaskWords), "workspace");
         FXE_TRY(ctx->alloc(&W.out, P), "workspace");
         FXE_TRY(ctx->alloc(&W.counters, 8), "workspace");   // [4]: the pose queue of pose_kernel
+        FXE_TRY(ctx->alloc(&W.pose_cost, P), "workspace");
+        FXE_TRY(ctx->alloc(&W.pose_clash, P), "workspace");
         FXE_TRY(ctx->alloc(&W.pose_order, P), "workspace");
         FXE_TRY(ctx->alloc(&ctx->d_genes, P * (ng > 0 ? ng : 1)), "staging");
         FXE_TRY(ctx->alloc(&ctx->d_icin, P * (ng > 0 ? ng : 1)), "staging");

@@ -154,6 +154,9 @@ struct DevWork {
     uint32_t* pose_rec;    // [P * kMaxLig * kMaskWords] mobile partners each processed atom kept
     fxe_cf* out;           // [P]
     int* counters;         // [4]: unused, hull failures, capacity, no-partner faces
+    int* pose_cost;        // [P] sum over the pose's atoms of the squared candidate count (zeroed by the
+                           // build, added up by the contact scan; for the pose order only)
+    float* pose_clash;     // [P] sum of clash_part, likewise
     int* pose_order;       // [P] poses in the order pose_kernel takes them (costliest first)
 };
 

@@ -15,6 +15,7 @@
 // L1 and L2), or staged first in shared memory by bulk copies (cp.async.bulk, one per contiguous
 // row of three cells, completing on an mbarrier). Results are the same.
 #include "fxe_common.cuh"
+#include "fxe_sort.cuh"
 
 namespace fxe {
 
@@ -258,6 +259,7 @@ __device__ __forceinline__ void contacts_atom(const DevSystem& S, const DevWork&
             consider(in, pos, k, pj);
         }
     }
+    const int n_rigid = nc;   // (in order already, unless the grid was re-derived)
     // the mobile atoms (side-chain atoms and the ligand) in the 27 cells
 #pragma unroll
     for (int s = 0; s < kMaxLig / 32; ++s) {
@@ -272,8 +274,33 @@ __device__ __forceinline__ void contacts_atom(const DevSystem& S, const DevWork&
         consider(pos >= 0, pos, m < nm ? slot_of(S, m) : 0, pj);
     }
     if (__any_sync(kFull, clash != 0.0)) clash = warp_sum_d(clash);
-    // into the reference's order: bitonic sort of the staged keys
-    if (nc <= kMaxCand) {
+    // into the reference's order
+    if (nc > kMaxCand) {
+        // (over capacity: nothing reads the list)
+    } else if (!pg.x) {
+        // The rigid candidates come in order (cells in scan order, Calc order within a cell): a
+        // candidate's place is the rigid ones before it (its own place, or by binary search) plus the
+        // mobile ones before it (all of them compared: a dozen). A bitonic sort of the list took a
+        // third of the kernel's instructions.
+        __syncwarp();
+        for (int i = lane; i < nc; i += 32) {
+            const int key = cs.key[i];
+            int place = i;
+            if (i >= n_rigid) {
+                int lo = 0, hi = n_rigid;
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    if (cs.key[mid] < key) lo = mid + 1;
+                    else hi = mid;
+                }
+                place = lo;
+            }
+            for (int t = n_rigid; t < nc; ++t) place += cs.key[t] < key;
+            W.cand_idx[cb + place] = cs.idx[i];
+            W.cand_d2[cb + place] = cs.d2[i];
+        }
+    } else {
+        // bitonic sort of the staged keys
         int len = 32;
         while (len < nc) len <<= 1;
         for (int i = nc + lane; i < len; i += 32) cs.key[i] = 0x7FFFFFFF;
@@ -307,6 +334,9 @@ __device__ __forceinline__ void contacts_atom(const DevSystem& S, const DevWork&
     if (lane == 0) {
         W.cand_n[lb + a] = nc > kMaxCand ? -nc : nc;
         W.clash_part[lb + a] = clash;
+        // the pose order's cost and clash sum
+        atomicAdd(&W.pose_cost[p], nc * nc);
+        if (clash != 0.0) atomicAdd(&W.pose_clash[p], (float)clash);
     }
 }
 
@@ -375,119 +405,62 @@ __device__ __forceinline__ int deal_tiles(int m, int n_scored, int deal, int til
     return deal > 0 && (deal == m / tile || n_scored < deal * tile) ? deal : 0;
 }
 
-// The sort key of pose p: minus its cost, or 1 for a pose the polyhedron launch rejects at once.
-__device__ __forceinline__ long long pose_order_key(const DevWork& W, int nm, int p) {
-    if (W.pose_grid[p].z) return 1;
-    const int* cn = W.cand_n + (size_t)p * nm;
-    const double* cp = W.clash_part + (size_t)p * nm;
-    long long cost = 0;
-    double clash = 0.0;
-    for (int a = 0; a < nm; ++a) {
-        const int k = cn[a];
-        if (k > 0) cost += (long long)k * k;
-        clash += cp[a];
-    }
-    // (the launch's own test sums the same terms in another order: a pose within rounding of the
-    // threshold may be placed on the other side, which only moves it in the queue)
-    if (clash >= kClashThreshold) return 1;
+// The sort key of pose p: the complement of its atoms and cost, the top bit set for a pose the
+// polyhedron launch rejects at once.
+constexpr uint64_t kRejected = 1ull << 63;
+__device__ __forceinline__ uint64_t pose_order_key(const DevWork& W, int nm, int p) {
+    // (the launch's own test sums the clash terms in double in another order: a pose within rounding
+    // of the threshold may be placed on the other side, which only moves it in the queue)
+    if (W.pose_grid[p].z || (double)W.pose_clash[p] >= kClashThreshold) return kRejected;
     // scored poses with more atoms first (a lockstep block steps through as many atoms as its
     // largest pose has), then the costliest
-    return -(((long long)nm << 40) | cost);
+    return ~kRejected & ~(((uint64_t)nm << 40) | (uint64_t)(unsigned)W.pose_cost[p]);
 }
 
-__global__ void __launch_bounds__(1024) order_poses_kernel(DevWork W, int nm, int n, int* __restrict__ order, int deal,
-                                                           int tile) {
-    __shared__ long long key[kOrderSeg];
+// Sorts the segment's m keys and writes its order.
+__device__ __forceinline__ void write_order(uint64_t* key, int* idx, int* n_scored, int base, int m, int* __restrict__ order, int deal,
+                                            int tile) {
+    int c = 0;
+    for (int i = threadIdx.x; i < m; i += blockDim.x) c += key[i] < kRejected;
+    c = __reduce_add_sync(kFull, c);
+    if ((threadIdx.x & 31) == 0 && c) atomicAdd(n_scored, c);
+    block_sort(key, idx, m);
+    const int dl = deal_tiles(m, *n_scored, deal, tile);
+    for (int i = threadIdx.x; i < m; i += blockDim.x) order[base + dealt_position(i, dl, tile)] = base + idx[i];
+}
+
+__global__ void __launch_bounds__(kSortThreads) order_poses_kernel(DevWork W, int nm, int n, int* __restrict__ order, int deal, int tile) {
+    __shared__ uint64_t key[kOrderSeg];
     __shared__ int idx[kOrderSeg];
     __shared__ int n_scored;
     if (threadIdx.x == 0) n_scored = 0;
     const int base = blockIdx.x * kOrderSeg;
     const int m = min(kOrderSeg, n - base);
-    int len = 1;
-    while (len < m) len <<= 1;
-    for (int i = threadIdx.x; i < len; i += blockDim.x) {
-        long long c = 0x7FFFFFFFFFFFFFFFll;   // padding sorts last
-        if (i < m) c = pose_order_key(W, nm, base + i);
-        key[i] = c;
+    for (int i = threadIdx.x; i < m; i += blockDim.x) {
+        key[i] = pose_order_key(W, nm, base + i);
         idx[i] = i;
     }
     __syncthreads();
-    for (int k = 2; k <= len; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < len; i += blockDim.x) {
-                const int l = i ^ j;
-                if (l > i) {
-                    const bool up = (i & k) == 0;
-                    const long long a = key[i], b = key[l];
-                    const bool gt = a > b || (a == b && idx[i] > idx[l]);
-                    if (gt == up) {
-                        key[i] = b;
-                        key[l] = a;
-                        const int t = idx[i];
-                        idx[i] = idx[l];
-                        idx[l] = t;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    // the scored poses (keys <= 0) of the segment
-    int c = 0;
-    for (int i = threadIdx.x; i < m; i += blockDim.x) c += key[i] <= 0;
-    if (c) atomicAdd(&n_scored, c);
-    __syncthreads();
-    const int dl = deal_tiles(m, n_scored, deal, tile);
-    for (int i = threadIdx.x; i < m; i += blockDim.x) order[base + dealt_position(i, dl, tile)] = base + idx[i];
+    write_order(key, idx, &n_scored, base, m, order, deal, tile);
 }
 
 // The same over the poses of several jobs (global pose index gp of the launch).
-__global__ void __launch_bounds__(1024) order_poses_jobs_kernel(const Job* __restrict__ jobs, int n_jobs, int n,
-                                                                int* __restrict__ order, int deal, int tile) {
-    __shared__ long long key[kOrderSeg];
+__global__ void __launch_bounds__(kSortThreads) order_poses_jobs_kernel(const Job* __restrict__ jobs, int n_jobs, int n,
+                                                                        int* __restrict__ order, int deal, int tile) {
+    __shared__ uint64_t key[kOrderSeg];
     __shared__ int idx[kOrderSeg];
     __shared__ int n_scored;
     if (threadIdx.x == 0) n_scored = 0;
     const int base = blockIdx.x * kOrderSeg;
     const int m = min(kOrderSeg, n - base);
-    int len = 1;
-    while (len < m) len <<= 1;
-    for (int i = threadIdx.x; i < len; i += blockDim.x) {
-        long long c = 0x7FFFFFFFFFFFFFFFll;
-        if (i < m) {
-            const int gp = base + i;
-            const Job& J = jobs[find_job(jobs, n_jobs, gp, false)];
-            c = pose_order_key(J.W, J.S.n_sc + J.S.n_lig, gp - J.pose0);
-        }
-        key[i] = c;
+    for (int i = threadIdx.x; i < m; i += blockDim.x) {
+        const int gp = base + i;
+        const Job& J = jobs[find_job(jobs, n_jobs, gp, false)];
+        key[i] = pose_order_key(J.W, J.S.n_sc + J.S.n_lig, gp - J.pose0);
         idx[i] = i;
     }
     __syncthreads();
-    for (int k = 2; k <= len; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < len; i += blockDim.x) {
-                const int l = i ^ j;
-                if (l > i) {
-                    const bool up = (i & k) == 0;
-                    const long long a = key[i], b = key[l];
-                    const bool gt = a > b || (a == b && idx[i] > idx[l]);
-                    if (gt == up) {
-                        key[i] = b;
-                        key[l] = a;
-                        const int t = idx[i];
-                        idx[i] = idx[l];
-                        idx[l] = t;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    // the scored poses (keys <= 0) of the segment
-    int c = 0;
-    for (int i = threadIdx.x; i < m; i += blockDim.x) c += key[i] <= 0;
-    if (c) atomicAdd(&n_scored, c);
-    __syncthreads();
-    const int dl = deal_tiles(m, n_scored, deal, tile);
-    for (int i = threadIdx.x; i < m; i += blockDim.x) order[base + dealt_position(i, dl, tile)] = base + idx[i];
+    write_order(key, idx, &n_scored, base, m, order, deal, tile);
 }
 
 // deal: full tiles to deal the sorted poses over (one segment only; 0 keeps the sorted order);
@@ -495,13 +468,13 @@ __global__ void __launch_bounds__(1024) order_poses_jobs_kernel(const Job* __res
 void launch_order_poses_jobs(const Job* jobs, int n_jobs, int total, int* order, cudaStream_t st, int deal,
                              int tile) {
     if (total > kOrderSeg || tile < 1) deal = 0;
-    order_poses_jobs_kernel<<<(total + kOrderSeg - 1) / kOrderSeg, 1024, 0, st>>>(jobs, n_jobs, total, order, deal,
+    order_poses_jobs_kernel<<<(total + kOrderSeg - 1) / kOrderSeg, kSortThreads, 0, st>>>(jobs, n_jobs, total, order, deal,
                                                                                   tile);
 }
 
 void launch_order_poses(const DevSystem& S, const DevWork& W, int n, cudaStream_t st, int deal, int tile) {
     if (n > kOrderSeg || tile < 1) deal = 0;
-    order_poses_kernel<<<(n + kOrderSeg - 1) / kOrderSeg, 1024, 0, st>>>(W, S.n_sc + S.n_lig, n, W.pose_order, deal,
+    order_poses_kernel<<<(n + kOrderSeg - 1) / kOrderSeg, kSortThreads, 0, st>>>(W, S.n_sc + S.n_lig, n, W.pose_order, deal,
                                                                          tile);
 }
 
