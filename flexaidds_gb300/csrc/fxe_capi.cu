@@ -21,7 +21,7 @@
 namespace fxe {
 void launch_build(const DevSystem&, const DevWork&, int, const int32_t*, const double*, cudaStream_t);
 void launch_contacts(const DevSystem&, const DevWork&, int, cudaStream_t, bool);
-void launch_order_poses(const DevSystem&, const DevWork&, int, cudaStream_t, int, int);
+void launch_order_poses(const DevSystem&, const DevWork&, int, cudaStream_t);
 namespace f32 {
 void launch_poses(const DevSystem&, const DevWork&, int, int*, uint8_t*, size_t, int, cudaStream_t);
 cudaError_t configure_voronoi();
@@ -33,22 +33,8 @@ void launch_poses(const DevSystem&, const DevWork&, int, int*, uint8_t*, size_t,
 cudaError_t configure_voronoi();
 size_t pose_hist_bytes();
 int pose_max_blocks_per_sm();
-int pose_tile_for(int, size_t, int);
-int pose_launch_blocks(int, size_t, int);
 }
 
-// How the pose order of a polyhedron launch over n poses may be dealt: {full tiles that start
-// together (0: none, the order stays sorted), poses per tile}; the order kernel deals when those
-// tiles are all the launch has or its scored poses do not fill them (launch_order_poses). Only
-// reference-precision launches have tiles.
-struct Deal {
-    int deal, tile;
-};
-inline Deal order_deal(int precision, int n, size_t hist_bytes, int blocks_per_sm) {
-    if (precision == FXE_PRECISION_FAST) return {0, 0};
-    const int tile = f64::pose_tile_for(n, hist_bytes, blocks_per_sm);
-    return {std::min(n / tile, f64::pose_launch_blocks(n, hist_bytes, blocks_per_sm)), tile};
-}
 // Face history of a polyhedron launch, large enough for either precision's launch: the warps the
 // device holds at once, kHistStride bytes each (configure_voronoi first).
 inline size_t pose_hist_bytes() {
@@ -661,6 +647,7 @@ fxe_status context_create(const fxe_receptor_desc* rec, const fxe_context* share
         FXE_TRY(ctx->alloc(&W.clash_part, PL), "workspace");
         FXE_TRY(ctx->alloc(&W.pose_seed, P * fxe::kMaxLig * 3), "workspace");
         FXE_TRY(ctx->alloc(&W.pose_rec, P * fxe::kMaxLig * fxe::kMaskWords), "workspace");
+        FXE_TRY(ctx->alloc(&W.atom_terms, PL * 4), "workspace");
         FXE_TRY(ctx->alloc(&W.out, P), "workspace");
         FXE_TRY(ctx->alloc(&W.counters, 8), "workspace");   // [4]: the pose queue of pose_kernel
         FXE_TRY(ctx->alloc(&W.pose_cost, P), "workspace");
@@ -716,8 +703,7 @@ fxe_status run_chunk(fxe_context* ctx, int nb, const int32_t* d_genes, const dou
     if (t) cudaEventRecord(ctx->ev[2], s);
     uint8_t* hist = ctx->face_order == FXE_FACE_ORDER_REFERENCE ? ctx->d_hist : nullptr;
     const int bpsm = tuned_blocks(ctx->precision, ctx->S.n_sc + ctx->S.n_lig, nb);
-    const fxe::Deal dl = fxe::order_deal(ctx->precision, nb, hist ? ctx->hist_bytes : 0, bpsm);
-    fxe::launch_order_poses(ctx->S, ctx->W, nb, s, dl.deal, dl.tile);
+    fxe::launch_order_poses(ctx->S, ctx->W, nb, s);
     if (ctx->precision == FXE_PRECISION_FAST)
         fxe::f32::launch_poses(ctx->S, ctx->W, nb, ctx->W.counters + 4, hist, ctx->hist_bytes, bpsm, s);
     else fxe::f64::launch_poses(ctx->S, ctx->W, nb, ctx->W.counters + 4, hist, ctx->hist_bytes, bpsm, s);
@@ -1232,7 +1218,7 @@ extern "C" fxe_status fxe_thermo_compute_device_fixed(const double* d_energies, 
 namespace fxe {
 void launch_build_jobs(const Job*, int, int, cudaStream_t);
 void launch_contacts_jobs(const Job*, int, long long, cudaStream_t, bool);
-void launch_order_poses_jobs(const Job*, int, int, int*, cudaStream_t, int, int);
+void launch_order_poses_jobs(const Job*, int, int, int*, cudaStream_t);
 namespace f32 {
 void launch_poses_jobs(const Job*, int, int, int*, const int*, uint8_t*, size_t, int, cudaStream_t);
 }
@@ -1351,8 +1337,7 @@ fxe_status batch_launch(fxe_batch* b, const fxe_job* jobs, int32_t n_jobs, cudaS
     fxe::launch_contacts_jobs(b->d_jobs, k, items, s, resolve_staged(cells, prec, mobile, total));
     uint8_t* hist = order == FXE_FACE_ORDER_REFERENCE ? b->d_hist : nullptr;
     const int bpsm = tuned_blocks(prec, mobile, total);
-    const fxe::Deal dl = fxe::order_deal(prec, total, hist ? b->hist_bytes : 0, bpsm);
-    fxe::launch_order_poses_jobs(b->d_jobs, k, total, b->d_order, s, dl.deal, dl.tile);
+    fxe::launch_order_poses_jobs(b->d_jobs, k, total, b->d_order, s);
     if (prec == FXE_PRECISION_FAST)
         fxe::f32::launch_poses_jobs(b->d_jobs, k, total, b->d_next, b->d_order, hist, b->hist_bytes, bpsm, s);
     else fxe::f64::launch_poses_jobs(b->d_jobs, k, total, b->d_next, b->d_order, hist, b->hist_bytes, bpsm, s);
@@ -1764,8 +1749,7 @@ extern "C" fxe_status fxe_ga_step(fxe_ga* e) {
         for (int sl : e->run) ref_order = ref_order && e->slots[sl].ctx->face_order == FXE_FACE_ORDER_REFERENCE;
         uint8_t* hist = ref_order ? e->d_hist : nullptr;
         const int bpsm = tuned_blocks(e->precision, mobile, total);
-        const fxe::Deal dl = fxe::order_deal(e->precision, total, hist ? e->hist_bytes : 0, bpsm);
-        fxe::launch_order_poses_jobs(e->d_eval, n, total, e->d_order, e->stream, dl.deal, dl.tile);
+        fxe::launch_order_poses_jobs(e->d_eval, n, total, e->d_order, e->stream);
         if (e->precision == FXE_PRECISION_FAST)
             fxe::f32::launch_poses_jobs(e->d_eval, n, total, e->d_next, e->d_order, hist, e->hist_bytes, bpsm, e->stream);
         else fxe::f64::launch_poses_jobs(e->d_eval, n, total, e->d_next, e->d_order, hist, e->hist_bytes, bpsm,
@@ -2197,8 +2181,7 @@ static fxe_status autotune_sweep(fxe_context* ctx, int32_t n, const int32_t* d_g
     // the candidates' work: this batch built, its contact candidates listed and ordered once
     fxe::launch_build(ctx->S, ctx->W, n, d_genes, nullptr, s);
     fxe::launch_contacts(ctx->S, ctx->W, n, s, false);
-    const fxe::Deal dl = fxe::order_deal(ctx->precision, n, hist ? ctx->hist_bytes : 0, 0);
-    fxe::launch_order_poses(ctx->S, ctx->W, n, s, dl.deal, dl.tile);
+    fxe::launch_order_poses(ctx->S, ctx->W, n, s);
     FXE_TRY(cudaGetLastError(), "autotune launch");
     cudaEvent_t a = nullptr, b = nullptr;
     FXE_TRY(cudaEventCreate(&a), "cudaEventCreate");

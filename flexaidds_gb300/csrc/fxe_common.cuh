@@ -152,6 +152,7 @@ struct DevWork {
     double* clash_part;    // [P * n_mob]
     int* pose_seed;        // [P * kMaxLig * 3] polyhedron seeds left by earlier atoms
     uint32_t* pose_rec;    // [P * kMaxLig * kMaskWords] mobile partners each processed atom kept
+    double* atom_terms;    // [P * n_mob * 4] terms of each scored atom (reference precision)
     fxe_cf* out;           // [P]
     int* counters;         // [4]: unused, hull failures, capacity, no-partner faces
     int* pose_cost;        // [P] sum over the pose's atoms of the squared candidate count (zeroed by the

@@ -380,30 +380,10 @@ contacts_kernel_jobs(const Job* __restrict__ jobs, int n_jobs, long long total) 
 // The order pose_kernel takes the poses in: the poses with the most scored atoms first, among
 // them the costliest first (sum over the pose's atoms of the squared candidate count, which the
 // hull walk's plane tests grow with), so that the slowest poses start early and the launch does
-// not end on one of them while the SMs run dry, and the poses a lockstep block steps through
-// together have as many atoms; then the
-// poses that need no polyhedra (the clash pre-filter rejects them, or they left the grid), so
-// that the warps of a block, which step through the atoms together, are not held by poses that
-// have nothing to do. Sorted in segments of kOrderSeg poses, one block each. The order changes
-// no result.
-// A launch of lockstep blocks takes tiles of `tile` neighbouring queue entries; its first `deal`
-// tiles (as many full tiles as the device runs at once) start together. When they are all the
-// launch has, or when its scored poses do not fill them, the launch lasts about as long as its
-// slowest first tile: there the sorted poses are dealt round-robin over those tiles (tile t gets
-// sorted entries t, t + deal, ...), so each holds one of the costliest poses and the scored poses
-// spread over every SM, the rejected ones taking the tiles' last slots and the later tiles.
-// Otherwise (the scored poses fill more than the first tiles) the sorted order stands.
+// not end on one of them while the SMs run dry; then the poses that need no polyhedra (the clash
+// pre-filter rejects them, or they left the grid). Sorted in segments of kOrderSeg poses, one block
+// each. The order changes no result.
 constexpr int kOrderSeg = 4096;
-
-// Queue position of sorted entry i of a segment.
-__device__ __forceinline__ int dealt_position(int i, int deal, int tile) {
-    return deal > 0 && i < deal * tile ? (i % deal) * tile + i / deal : i;
-}
-
-// Whether a sorted single segment of m poses, n_scored of them scored, is dealt over `deal` tiles.
-__device__ __forceinline__ int deal_tiles(int m, int n_scored, int deal, int tile) {
-    return deal > 0 && (deal == m / tile || n_scored < deal * tile) ? deal : 0;
-}
 
 // The sort key of pose p: the complement of its atoms and cost, the top bit set for a pose the
 // polyhedron launch rejects at once.
@@ -412,45 +392,28 @@ __device__ __forceinline__ uint64_t pose_order_key(const DevWork& W, int nm, int
     // (the launch's own test sums the clash terms in double in another order: a pose within rounding
     // of the threshold may be placed on the other side, which only moves it in the queue)
     if (W.pose_grid[p].z || (double)W.pose_clash[p] >= kClashThreshold) return kRejected;
-    // scored poses with more atoms first (a lockstep block steps through as many atoms as its
-    // largest pose has), then the costliest
+    // scored poses with more atoms first, then the costliest
     return ~kRejected & ~(((uint64_t)nm << 40) | (uint64_t)(unsigned)W.pose_cost[p]);
 }
 
-// Sorts the segment's m keys and writes its order.
-__device__ __forceinline__ void write_order(uint64_t* key, int* idx, int* n_scored, int base, int m, int* __restrict__ order, int deal,
-                                            int tile) {
-    int c = 0;
-    for (int i = threadIdx.x; i < m; i += blockDim.x) c += key[i] < kRejected;
-    c = __reduce_add_sync(kFull, c);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(n_scored, c);
-    block_sort(key, idx, m);
-    const int dl = deal_tiles(m, *n_scored, deal, tile);
-    for (int i = threadIdx.x; i < m; i += blockDim.x) order[base + dealt_position(i, dl, tile)] = base + idx[i];
-}
-
-__global__ void __launch_bounds__(kSortThreads) order_poses_kernel(DevWork W, int nm, int n, int* __restrict__ order, int deal, int tile) {
+__global__ void __launch_bounds__(kSortThreads) order_poses_kernel(DevWork W, int nm, int n, int* __restrict__ order) {
     __shared__ uint64_t key[kOrderSeg];
     __shared__ int idx[kOrderSeg];
-    __shared__ int n_scored;
-    if (threadIdx.x == 0) n_scored = 0;
     const int base = blockIdx.x * kOrderSeg;
     const int m = min(kOrderSeg, n - base);
     for (int i = threadIdx.x; i < m; i += blockDim.x) {
         key[i] = pose_order_key(W, nm, base + i);
         idx[i] = i;
     }
-    __syncthreads();
-    write_order(key, idx, &n_scored, base, m, order, deal, tile);
+    block_sort(key, idx, m);
+    for (int i = threadIdx.x; i < m; i += blockDim.x) order[base + i] = base + idx[i];
 }
 
 // The same over the poses of several jobs (global pose index gp of the launch).
 __global__ void __launch_bounds__(kSortThreads) order_poses_jobs_kernel(const Job* __restrict__ jobs, int n_jobs, int n,
-                                                                        int* __restrict__ order, int deal, int tile) {
+                                                                        int* __restrict__ order) {
     __shared__ uint64_t key[kOrderSeg];
     __shared__ int idx[kOrderSeg];
-    __shared__ int n_scored;
-    if (threadIdx.x == 0) n_scored = 0;
     const int base = blockIdx.x * kOrderSeg;
     const int m = min(kOrderSeg, n - base);
     for (int i = threadIdx.x; i < m; i += blockDim.x) {
@@ -459,23 +422,16 @@ __global__ void __launch_bounds__(kSortThreads) order_poses_jobs_kernel(const Jo
         key[i] = pose_order_key(J.W, J.S.n_sc + J.S.n_lig, gp - J.pose0);
         idx[i] = i;
     }
-    __syncthreads();
-    write_order(key, idx, &n_scored, base, m, order, deal, tile);
+    block_sort(key, idx, m);
+    for (int i = threadIdx.x; i < m; i += blockDim.x) order[base + i] = base + idx[i];
 }
 
-// deal: full tiles to deal the sorted poses over (one segment only; 0 keeps the sorted order);
-// tile: poses per tile.
-void launch_order_poses_jobs(const Job* jobs, int n_jobs, int total, int* order, cudaStream_t st, int deal,
-                             int tile) {
-    if (total > kOrderSeg || tile < 1) deal = 0;
-    order_poses_jobs_kernel<<<(total + kOrderSeg - 1) / kOrderSeg, kSortThreads, 0, st>>>(jobs, n_jobs, total, order, deal,
-                                                                                  tile);
+void launch_order_poses_jobs(const Job* jobs, int n_jobs, int total, int* order, cudaStream_t st) {
+    order_poses_jobs_kernel<<<(total + kOrderSeg - 1) / kOrderSeg, kSortThreads, 0, st>>>(jobs, n_jobs, total, order);
 }
 
-void launch_order_poses(const DevSystem& S, const DevWork& W, int n, cudaStream_t st, int deal, int tile) {
-    if (n > kOrderSeg || tile < 1) deal = 0;
-    order_poses_kernel<<<(n + kOrderSeg - 1) / kOrderSeg, kSortThreads, 0, st>>>(W, S.n_sc + S.n_lig, n, W.pose_order, deal,
-                                                                         tile);
+void launch_order_poses(const DevSystem& S, const DevWork& W, int n, cudaStream_t st) {
+    order_poses_kernel<<<(n + kOrderSeg - 1) / kOrderSeg, kSortThreads, 0, st>>>(W, S.n_sc + S.n_lig, n, W.pose_order);
 }
 
 void launch_contacts(const DevSystem& S, const DevWork& W, int n, cudaStream_t st, bool staged) {

@@ -18,17 +18,20 @@
 // atom centre lies outside its own cell, so a start from the closest plane can lie outside the
 // cell and trace another polyhedron. Parallelism is across poses (one warp each), across the
 // planes, edges, vertices and faces of each polyhedron (the 32 lanes), and, for the triangles and
-// arcs of the areas, across the block: the poses of a block step through their atoms together and
-// pool those items.
+// arcs of the areas, across a group of warps: the poses of a group step through their atoms together
+// and pool those items. Stepping together also keeps the group's warps at the same place of 170 KB of
+// code, more than the instruction caches hold: sixteen warps each on its own took 11.1 ms where the
+// lockstep took 8.0 (2,000 poses of the benchmark's system).
 //
 // What bounds it: the FP64 unit, which takes one warp instruction per 64 cycles and SM quarter
 // whatever its active lanes. Hence
 //   * quotients and roots in five FP64 instructions (fxe_dmath.cuh);
 //   * comparisons on the integer units (the bit patterns of doubles order like the doubles);
 //   * the three coordinates of a vertex or a direction on three lanes, one instruction for all;
-//   * the triangles and arcs of all the block's poses packed into full warps (25 and 7 per atom on
+//   * the triangles and arcs of all the group's poses packed into full warps (25 and 7 per atom on
 //     the benchmark's systems, of a warp's 32 lanes);
 //   * plane tests decided in single precision with an error bound wherever that is certain.
+#include <algorithm>
 #include <cfloat>
 #include <climits>
 
@@ -42,24 +45,22 @@ constexpr unsigned kFull = 0xffffffffu;
 constexpr int kFaceWords = (kMaxCand + 31) / 32;
 constexpr uint8_t kNone = 255;
 constexpr int kAtomNone = 5;     // an atom without contacts
-constexpr int kAtomWalking = 4;  // the hull walk goes on in the block's next step
+constexpr int kAtomWalking = 4;  // the hull walk goes on in the group's next step
 constexpr int kAtomRetry = 3;    // the atom outgrew this shape's capacities: score the pose with the large one
 
-// Warps of a block, one block per SM.
+// Warps of a block, one block per SM, in groups that step through their poses' atoms together.
 constexpr int kWarps = 16;
-// Batches of edges a hull walk may step before its warp meets the block (it goes on in the block's
-// next step).
-#ifndef FXE_WALK_BUDGET
-#define FXE_WALK_BUDGET 8
-#endif
-constexpr int kWalkBudget = FXE_WALK_BUDGET;
+// Batches of edges a hull walk may step before its warp meets its group (it goes on in the group's
+// next step): a walk takes 5.4 on average, forty when it fails. 2,000 poses of the benchmark's system
+// take 7.77 ms with 8, 7.59 with 10, 7.40 with 12, 7.37 with 16, 7.36 with 20.
+constexpr int kWalkBudget = 16;
 
 // Capacities of one polyhedron. The compact shape holds the polyhedra of ordinary poses (on the
 // benchmark's systems at most 44 vertices inside the sphere, 125 face points and 125 area items over
 // 2,300 atoms; means 17, 43 and 33) and any hull walk and its arc points (176 vertices: those past
 // `verts` lie in storage the faces use later), in 14.1 KB per pose, so that sixteen poses fit an SM. A
 // pose one of whose atoms outgrows it is scored again, from its start, in the large shape when its
-// block is through with its tile.
+// group has no other pose.
 template <int kV, int kX, int kP, int kI, int kN>
 struct Shape {
     static constexpr int verts = kV;         // of the faces; vertex indices are bytes (255 means "none")
@@ -659,10 +660,105 @@ __device__ __forceinline__ uchar4* hist_vp(uint8_t* h) {
     return reinterpret_cast<uchar4*>(h + kHistBytes + kMaxCand * sizeof(real4));
 }
 
+// The smallest of the lanes' values (not negative), with the lowest index among equal ones and its
+// upper bound; false when another entry's lower bound (lo1 / lo2: each lane's two smallest, lo1i the
+// first's index) does not lie above that, or a lane is undecided.
+__device__ __forceinline__ bool certain_min(float best, float hi, int bi, float lo1, float lo2, int lo1i, bool undecided, int* at) {
+    const unsigned b = __float_as_uint(best), m = __reduce_min_sync(kFull, b);
+    const int i = __reduce_min_sync(kFull, b == m ? bi : INT_MAX);
+    const unsigned own = __ballot_sync(kFull, b == m && bi == i);
+    const float h = __shfl_sync(kFull, hi, __ffs(own) - 1);
+    *at = i;
+    return !__any_sync(kFull, undecided || !((lo1i == i ? lo2 : lo1) > h)) && i != INT_MAX;
+}
+
+// get_firstvert's search (see first_planes_exact) decided in single precision, false when an error
+// bound does not allow it (3 % of the searches). The search starts a fifth of the atoms, so nearly
+// every step of a group waited for one: 25,000 - 38,000 cycles in double precision of some 230,000.
+//  Two planes' line lies at d^2 = (wa^2 + wb^2 - 2 wa wb cos) / sin^2 of unit
+// normals with cosine cos; inputs truncated by 2^-23 of them leave cos within 6e-7, so the numerator
+// within 3e-6 (|wa| + |wb|)^2 and the denominator within 1.5e-6.
+template <class Sh>
+__device__ __noinline__ bool first_planes_fast(const Vor<Sh>& sh, int NC, int lane, int* pA, int* pB, int* pC) {
+    constexpr float kBig = 3.0e38f;
+    long long bv = bits(9.9e9);
+    int iA = INT_MAX;
+    #pragma unroll 1
+    for (int c = lane; c < NC; c += 32) {
+        const long long d = bits(fabs(sh.pl[c].w));
+        if (d < bv) { bv = d; iA = c; }
+    }
+    warp_argmin(bv, iA);
+    if (iA == INT_MAX) return false;
+    const float4 A = sh.plf[iA];
+    float best = kBig, hi = kBig, lo1 = kBig, lo2 = kBig;
+    int bi = INT_MAX, lo1i = INT_MAX;
+    bool undecided = false;
+    #pragma unroll 1
+    for (int c = lane; c < NC + 4; c += 32) {
+        if (c == iA) continue;
+        float4 C = sh.plf[c];
+        if (c >= NC) {   // the bounding planes' normals are 1.224683 long
+            C.x *= 0.816538f; C.y *= 0.816538f; C.z *= 0.816538f; C.w *= 0.816538f;
+        }
+        const float cs = A.x * C.x + A.y * C.y + A.z * C.z, s2 = 1.0f - cs * cs;
+        const float w2 = (fabsf(A.w) + fabsf(C.w)) * (fabsf(A.w) + fabsf(C.w));
+        const float n = fmaxf(A.w * A.w + C.w * C.w - 2.0f * A.w * C.w * cs, 0.0f), en = 3e-6f * w2;
+        if (!(s2 > 1e-4f)) {
+            undecided = true;
+            continue;
+        }
+        const float d2 = n / s2, h = (n + en) / (s2 - 1.5e-6f) * 1.000001f, l = (n - en) / (s2 + 1.5e-6f) * 0.999999f - 1e-12f;
+        if (d2 < best) { best = d2; hi = h; bi = c; }
+        if (l < lo1) { lo2 = lo1; lo1 = l; lo1i = c; }
+        else if (l < lo2) lo2 = l;
+    }
+    int iB;
+    if (!certain_min(best, hi, bi, lo1, lo2, lo1i, undecided, &iB)) return false;
+    // the point of the line closest to the centre, and the plane the line meets first
+    float4 B = sh.plf[iB];
+    if (iB >= NC) {
+        B.x *= 0.816538f; B.y *= 0.816538f; B.z *= 0.816538f; B.w *= 0.816538f;
+    }
+    const float cs = A.x * B.x + A.y * B.y + A.z * B.z, is2 = 1.0f / (1.0f - cs * cs);
+    const float ka = -(A.w - B.w * cs) * is2, kb = -(B.w - A.w * cs) * is2;
+    const float px = ka * A.x + kb * B.x, py = ka * A.y + kb * B.y, pz = ka * A.z + kb * B.z;
+    const float es = start_err(px, py, pz) + 8e-6f * (fabsf(A.w) + fabsf(B.w)) * is2 * is2;
+    const float3 v = cross_f(A, B);
+    best = hi = lo1 = lo2 = kBig;
+    bi = lo1i = INT_MAX;
+    #pragma unroll 1
+    for (int c = lane; c < NC + 4; c += 32) {
+        if (c == iA || c == iB) continue;
+        const float4 C = sh.plf[c];
+        float er;
+        bool ok;
+        const float vt = fabsf(vt_pretest(C, px, py, pz, v.x, v.y, v.z, es, &er, &ok));
+        float l = vt - er;
+        if (ok) {
+            if (vt < best) { best = vt; hi = vt + er; bi = c; }
+        } else {
+            // nearly parallel to the line: beyond |numerator| over the largest such denominator
+            const float num = fabsf(fmaf(C.x, px, fmaf(C.y, py, fmaf(C.z, pz, C.w))));
+            const float left = num - fmaf(fabsf(C.w), 0x1.0p-20f, es);
+            if (!(left > 0.0f)) undecided = true;
+            l = left * (0.9f / (17.0f * kDenErr));
+        }
+        if (l < lo1) { lo2 = lo1; lo1 = l; lo1i = c; }
+        else if (l < lo2) lo2 = l;
+    }
+    int iC;
+    if (!certain_min(best, hi, bi, lo1, lo2, lo1i, undecided, &iC)) return false;
+    *pA = iA;
+    *pB = iB;
+    *pC = iC;
+    return true;
+}
+
 // get_firstvert's search from the plane closest to the centre (LIB/Vcontacts.cpp:498-592): the
 // first vertex's planes, false when a step finds none.
 template <class Sh>
-__device__ __noinline__ bool first_planes(const Vor<Sh>& sh, int NC, int lane, int* pA, int* pB, int* pC) {
+__device__ __noinline__ bool first_planes_exact(const Vor<Sh>& sh, int NC, int lane, int* pA, int* pB, int* pC) {
     long long bv = bits(9.9e9);
     int bi = INT_MAX;
     #pragma unroll 1
@@ -1366,25 +1462,34 @@ __device__ __forceinline__ int area_items(Vor<Sh>& sh, int NC, int NV, double ra
     return kAtomOk;
 }
 
-// A block's state besides its poses' workspaces.
-struct BlockState {
-    int2 items[kWarps];      // per pose: triangle items, arc items
-    int base;                // first queue entry of the block's tile
-    int n_retry;             // poses to score again in the large shape
-    int retry[kWarps];
+// The warps of a block that step together: kSize of them, of which this warp is `slot`.
+template <int kSize>
+struct Group {
+    static constexpr int size = kSize;
+    int slot, barrier;
+    int4* step;              // per pose: triangle items, arc items, whether the pose goes on
+    int* n_retry;            // poses to score again in the large shape
+    int* retry;              // [2 * size]
 };
 
-// The block's area items, pooled: every pose's triangles as one list, then every pose's arcs as
-// another, 32 at a time to the block's warps. Block barriers around it keep the items' owners out.
-template <class Sh>
-__device__ __forceinline__ void pooled_areas(PoseShared<Sh>* all, const int2* items, int warp, int lane) {
+// The group's barrier (a named one: 1 ..; 0 is the block's own).
+template <int kSize>
+__device__ __forceinline__ void group_sync(const Group<kSize>& g) {
+    __syncwarp();
+    asm volatile("bar.sync %0, %1;" ::"r"(g.barrier), "n"(kSize * 32) : "memory");
+}
+
+// The group's area items, pooled: every pose's triangles as one list, then every pose's arcs as
+// another, 32 at a time to the group's warps. Group barriers around it keep the items' owners out.
+template <class Sh, int kSize>
+__device__ __forceinline__ void pooled_areas(PoseShared<Sh>* all, const Group<kSize>& g, int lane) {
     static_assert(kWarps <= 32, "one lane per pose in the prefix sums");
-    const int2 n = lane < Sh::poses ? items[lane] : make_int2(0, 0);
+    const int4 n = lane < g.size ? g.step[lane] : make_int4(0, 0, 0, 0);
     int T, A;
     const int tpre = warp_excl_scan(n.x, lane, &T), apre = warp_excl_scan(n.y, lane, &A);
     const int tch = (T + 31) >> 5, ach = (A + 31) >> 5;
     #pragma unroll 1
-    for (int ch = warp; ch < tch + ach; ch += kWarps) {
+    for (int ch = g.slot; ch < tch + ach; ch += g.size) {
         const bool tri = ch < tch;
         const int k = (tri ? ch : ch - tch) * 32 + lane, pre = tri ? tpre : apre;
         // the pose of item k: the last one whose first item is at or before it (a pose without
@@ -1539,101 +1644,100 @@ __device__ __forceinline__ double matrix_term(const DevSystem& S, int idx, doubl
                                    (double)(S.em_y[k + 1] - S.em_y[k]);
 }
 
-// vcfunction (LIB/vcfunction.cpp:84-513) for one pose: scored atoms in Calc order (side-chain
-// atoms, then the ligand), their kept contacts; each residue's terms are summed on their own and
-// the records added up ligand first, then the side chains in order (LIB/ic2cf.cpp:133-245).
-__device__ __noinline__ void score_contacts(const DevSystem& S, const DevWork& W, int p, int lane) {
-    const int nl = n_mobile(S);
-    const size_t lb = (size_t)p * nl;
+// vcfunction (LIB/vcfunction.cpp:84-513) for scored atom i of a pose (mobile atoms lb ..): the terms of
+// its kept contacts and its solvent term into W.atom_terms (complementarity, wall, solvent, and the
+// accessible surface). Called as each atom is saved, so that no pose's scoring holds its group.
+__device__ __noinline__ void score_atom(const DevSystem& S, const DevWork& W, size_t lb, int i, int lane) {
     const int T = S.ntypes, nsc = S.n_sc;
-    double com = 0.0, wal = 0.0, sas = 0.0, totsas = 0.0;
-    // lane r keeps side chain r's record
-    double res_com = 0.0, res_wal = 0.0, res_sas = 0.0;
-    int cur_res = -1;
+    const int NC = W.cand_n[lb + i];
+    const size_t cb = (lb + i) * kMaxCand;
+    const bool side = i < nsc;
+    const float radf = W.mob_pos[lb + i].w;
+    const double radA = f2d(radf);
+    const double radoA = radA + (double)kRw;
+    const double surfA = 4.0 * kPi * radoA * radoA;
+    const int ti = side ? S.rec_type[S.sc_slot[i]] : S.lig_type[i - nsc];
+    double c_com = 0.0, c_wal = 0.0, c_area = 0.0;
     #pragma unroll 1
-    for (int i = 0; i < nl; ++i) {
-        const int NC = W.cand_n[lb + i];
-        const size_t cb = (lb + i) * kMaxCand;
-        const bool side = i < nsc;
-        const int res = side ? S.sc_res[i] : kMaxFlex;
-        if (res != cur_res) {
-            if (lane == cur_res) {
-                res_com = com;
-                res_wal = wal;
-                res_sas = sas;
-            }
-            com = wal = sas = 0.0;
-            cur_res = res;
-        }
-        const float radf = W.mob_pos[lb + i].w;
-        const double radA = f2d(radf);
-        const double radoA = radA + (double)kRw;
-        const double surfA = 4.0 * kPi * radoA * radoA;
-        const int ti = side ? S.rec_type[S.sc_slot[i]] : S.lig_type[i - nsc];
-        double c_com = 0.0, c_wal = 0.0, c_area = 0.0;
-        #pragma unroll 1
-        for (int c = lane; c < NC; c += 32) {
-            if (!(W.cand_flag[cb + c] & kRecorded)) continue;
-            const int j = W.cand_idx[cb + c];
-            const double area = W.cand_area[cb + c];
-            c_area += area;
-            const int rel = residue_pair(S, i, j);
-            if (rel == 1) continue;                      // bonded within the residue
-            const int mj = mobile_of(S, j);
-            if (mj >= 0 && mj < i) continue;             // FA->contacts: scored from that atom
-            const bool lig_j = j >= S.n_rec;
-            const float rj = lig_j ? S.lig_radius[j - S.n_rec] : (mj >= 0 ? W.mob_pos[lb + mj].w : S.rec_pos[j].w);
-            const int tj = lig_j ? S.lig_type[j - S.n_rec] : S.rec_type[j];
-            // intramolecular: one residue, or two protein residues (LIB/vcfunction.cpp:283-291)
-            const bool intra = rel != 0 || (side && !lig_j);
-            if (S.intramolecular || !intra) c_com += matrix_term(S, (ti - 1) * T + (tj - 1), area, surfA);
-            const float d2 = W.cand_d2[cb + c];
-            const float cdf = S.permeability * (radf + rj);   // the clash distance, to single precision
-            if (d2 < cdf * cdf * 1.0002f) {
-                const double permea = (double)S.permeability;
-                const double rAB = radA + (double)rj;
-                const float clash_distance = (float)(permea * rAB);
-                if (d2 < clash_distance * clash_distance * 1.0001f) {
-                    const double dd = sqrt((double)d2);
-                    if (dd < (double)clash_distance) {
-                        const double q2 = dd * dd, q4 = q2 * q2, q6 = q4 * q2;
-                        const double cr = permea * rAB;
-                        const double r2 = cr * cr, r4 = r2 * r2, r6 = r4 * r2;
-                        c_wal += (double)kKwall * (1.0 / (q6 * q6) - 1.0 / (r6 * r6));
-                    }
+    for (int c = lane; c < NC; c += 32) {
+        if (!(W.cand_flag[cb + c] & kRecorded)) continue;
+        const int j = W.cand_idx[cb + c];
+        const double area = W.cand_area[cb + c];
+        c_area += area;
+        const int rel = residue_pair(S, i, j);
+        if (rel == 1) continue;                      // bonded within the residue
+        const int mj = mobile_of(S, j);
+        if (mj >= 0 && mj < i) continue;             // FA->contacts: scored from that atom
+        const bool lig_j = j >= S.n_rec;
+        const float rj = lig_j ? S.lig_radius[j - S.n_rec] : (mj >= 0 ? W.mob_pos[lb + mj].w : S.rec_pos[j].w);
+        const int tj = lig_j ? S.lig_type[j - S.n_rec] : S.rec_type[j];
+        // intramolecular: one residue, or two protein residues (LIB/vcfunction.cpp:283-291)
+        const bool intra = rel != 0 || (side && !lig_j);
+        if (S.intramolecular || !intra) c_com += matrix_term(S, (ti - 1) * T + (tj - 1), area, surfA);
+        const float d2 = W.cand_d2[cb + c];
+        const float cdf = S.permeability * (radf + rj);   // the clash distance, to single precision
+        if (d2 < cdf * cdf * 1.0002f) {
+            const double permea = (double)S.permeability;
+            const double rAB = radA + (double)rj;
+            const float clash_distance = (float)(permea * rAB);
+            if (d2 < clash_distance * clash_distance * 1.0001f) {
+                const double dd = sqrt((double)d2);
+                if (dd < (double)clash_distance) {
+                    const double q2 = dd * dd, q4 = q2 * q2, q6 = q4 * q2;
+                    const double cr = permea * rAB;
+                    const double r2 = cr * cr, r4 = r2 * r2, r6 = r4 * r2;
+                    c_wal += (double)kKwall * (1.0 / (q6 * q6) - 1.0 / (r6 * r6));
                 }
             }
         }
-        // both sums in one reduction: after the first exchange the lower half holds c_com's
-        // partial sums, the upper half c_area's (the additions are warp_sum's)
-        {
-            const bool up = lane >= 16;
-            double x = (up ? c_area : c_com) + __shfl_xor_sync(kFull, up ? c_com : c_area, 16);
-#pragma unroll
-            for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(kFull, x, o);
-            c_com = __shfl_sync(kFull, x, 0);
-            c_area = __shfl_sync(kFull, x, 16);
-        }
-        if (__any_sync(kFull, !is0(c_wal))) wal += warp_sum(c_wal);
-        double SAS = surfA - c_area;
-        if (lt0(SAS)) SAS = 0.0;
-        if (!side) totsas += SAS;
-        com += c_com;
-        sas += S.solventterm != 0.0f ? (double)S.solventterm * SAS : matrix_term(S, (ti - 1) * T + (T - 1), SAS, surfA);
     }
-    // the ligand's record (com/wal/sas hold it now), then each side chain's
-    #pragma unroll 1
-    for (int r = 0; r < S.n_flex; ++r) {
-        com += __shfl_sync(kFull, res_com, r);
-        wal += __shfl_sync(kFull, res_wal, r);
-        sas += __shfl_sync(kFull, res_sas, r);
+    // both sums in one reduction: after the first exchange the lower half holds c_com's
+    // partial sums, the upper half c_area's (the additions are warp_sum's)
+    {
+        const bool up = lane >= 16;
+        double x = (up ? c_area : c_com) + __shfl_xor_sync(kFull, up ? c_com : c_area, 16);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(kFull, x, o);
+        c_com = __shfl_sync(kFull, x, 0);
+        c_area = __shfl_sync(kFull, x, 16);
+    }
+    if (__any_sync(kFull, !is0(c_wal))) c_wal = warp_sum(c_wal);
+    double SAS = surfA - c_area;
+    if (lt0(SAS)) SAS = 0.0;
+    const double sas = S.solventterm != 0.0f ? (double)S.solventterm * SAS : matrix_term(S, (ti - 1) * T + (T - 1), SAS, surfA);
+    if (lane == 0) {
+        double* t = W.atom_terms + (lb + i) * 4;
+        t[0] = c_com;
+        t[1] = c_wal;
+        t[2] = sas;
+        t[3] = SAS;
+    }
+}
+
+// The pose's record from its atoms' terms, in Calc order (side-chain atoms, then the ligand): each
+// residue's are summed on their own and the records added up ligand first, then the side chains in
+// order (LIB/ic2cf.cpp:133-245). One term per lane.
+__device__ __noinline__ void finish_scored(const DevSystem& S, const DevWork& W, int p, int lane) {
+    const int nl = n_mobile(S), nsc = S.n_sc;
+    const double* t = W.atom_terms + (size_t)p * nl * 4 + (lane & 3);
+    double sum = 0.0;
+    for (int i = nsc; i < nl; ++i) sum += t[4 * i];
+    if ((lane & 3) < 3) {
+        double res = 0.0;
+        for (int i = 0; i < nsc; ++i) {
+            res += t[4 * i];
+            if (i + 1 == nsc || S.sc_res[i + 1] != S.sc_res[i]) {
+                sum += res;
+                res = 0.0;
+            }
+        }
     }
     fxe_cf cf;
     memset(&cf, 0, sizeof(cf));
-    cf.com = com;
-    cf.wal = wal;
-    cf.sas = sas;
-    cf.totsas = totsas;
+    cf.com = __shfl_sync(kFull, sum, 0);
+    cf.wal = __shfl_sync(kFull, sum, 1);
+    cf.sas = __shfl_sync(kFull, sum, 2);
+    cf.totsas = __shfl_sync(kFull, sum, 3);
     cf.evalue = cf.com + cf.wal + cf.sas + cf.con + cf.elec + cf.hbond + cf.gist_desolv + cf.metal_coord;
     cf.status = FXE_POSE_SCORED;
     if (lane == 0) W.out[p] = cf;
@@ -1672,6 +1776,8 @@ __device__ __forceinline__ int start_atom(const DevSystem& S, const DevWork& W, 
             W.cand_area[cb + c] = 0.0;
             W.cand_flag[cb + c] = 0;
         }
+        __syncwarp();
+        score_atom(S, W, (size_t)p * n_mobile(S), a, lane);
         return kAtomNone;
     }
     const float4 me = W.mob_pos[(size_t)p * n_mobile(S) + a];
@@ -1694,227 +1800,294 @@ __device__ __forceinline__ int start_atom(const DevSystem& S, const DevWork& W, 
             if (m2) sC = c0 + 31 - __clz(m2);
         }
     }
-    if ((sA < 0 || sB < 0 || sC < 0) && !first_planes(sh, NC, lane, &sA, &sB, &sC)) return kAtomCapacity;
+    if (sA < 0 || sB < 0 || sC < 0)
+        if (!first_planes_fast(sh, NC, lane, &sA, &sB, &sC) && !first_planes_exact(sh, NC, lane, &sA, &sB, &sC)) return kAtomCapacity;
     walk_start(sh, lane, sA, sB, sC, walk);
     return kAtomOk;
 }
 
-// Scores pose p (p < 0: none; the warp only helps with the others' areas) together with the block's
-// other poses, step by step: in each step every pose takes its next atom (or goes on with its walk),
-// the block evaluates the areas' items, and each pose saves its atom. Returns kAtomRetry for a pose
-// that outgrew the shape, else kAtomOk.
-template <class Sh>
-__device__ __forceinline__ int score_pose(const DevSystem& S, const DevWork& W, int p, int lane, PoseShared<Sh>* all,
-                                          BlockState& block, uint8_t* hist) {
-    const int warp = (int)(threadIdx.x >> 5);
-    PoseShared<Sh>& ps = all[warp];
-    Vor<Sh>& sh = ps.v;
-    int result = kAtomOk;
-    bool alive = p >= 0;
-    if (p < 0) p = 0;
-    const int nl = alive ? n_mobile(S) : 0;      // the scored atoms: side-chain atoms, then the ligand
-    // polyhedron seeds (Calc indices, -1 = none), and for each atom the processed atoms that kept a
-    // contact with it
-    int (*const seed)[3] = reinterpret_cast<int (*)[3]>(W.pose_seed + (size_t)p * kMaxLig * 3);
-    uint32_t (*const kept)[kMaskWords] = reinterpret_cast<uint32_t (*)[kMaskWords]>(W.pose_rec + (size_t)p * kMaxLig * kMaskWords);
-    const size_t lb = (size_t)p * nl;
-    if (alive && W.pose_grid[p].z) {
+// A warp's pose: its place and its current atom's state.
+struct Pose {
+    int p, entry, job;       // index in the workspace, queue entry, job
+    int r, a, n_cand, NC;    // the atom's place in Calclist order, the atom, its candidates and contacts
+    int miss, lost;          // per lane: faces without a neighbour, and those not replayed
+    bool alive, walking;     // walking: the atom's hull walk goes on
+    Walk walk;
+};
+
+// Where a launch's poses lie: one system's, or several jobs' (their descriptors are read from the job
+// table and stay in L1, keeping shared memory for the polyhedron workspace).
+struct OneJob {
+    const DevSystem& s;
+    const DevWork& w;
+    __device__ __forceinline__ const DevSystem& S(const Pose&) const { return s; }
+    __device__ __forceinline__ const DevWork& W(const Pose&) const { return w; }
+    __device__ __forceinline__ void place(Pose& q) const { q.p = q.entry; }
+};
+struct ManyJobs {
+    const Job* jobs;
+    int n;
+    __device__ __forceinline__ const DevSystem& S(const Pose& q) const { return jobs[q.job].S; }
+    __device__ __forceinline__ const DevWork& W(const Pose& q) const { return jobs[q.job].W; }
+    __device__ __forceinline__ void place(Pose& q) const {
+        q.job = find_job(jobs, n, q.entry, false);
+        q.p = q.entry - jobs[q.job].pose0;
+    }
+};
+
+// Takes pose q.p up: false when it is done already (clash pre-filter, or it left the grid).
+template <class Sh, class Jobs>
+__device__ __forceinline__ bool begin_pose(const Jobs& jobs, Pose& q, int lane, PoseShared<Sh>& ps, uint8_t* hist) {
+    const DevSystem& S = jobs.S(q);
+    const DevWork& W = jobs.W(q);
+    const int p = q.p, nl = n_mobile(S);
+    if (W.pose_grid[p].z) {
         finish_failed(W, p, lane, FXE_POSE_CAPACITY, 0.0);
-        alive = false;
+        return false;
     }
     // clash pre-filter (LIB/Vcontacts.cpp:36-51)
-    if (alive) {
-        const double clash = pose_clash_sum(S, W, p, lane);
-        if (clash >= kClashThreshold) {
-            finish_failed(W, p, lane, FXE_POSE_CLASHED, clash);
-            alive = false;
-        }
+    const double clash = pose_clash_sum(S, W, p, lane);
+    if (clash >= kClashThreshold) {
+        finish_failed(W, p, lane, FXE_POSE_CLASHED, clash);
+        return false;
     }
-    if (alive) {
+    const size_t lb = (size_t)p * nl;
+    #pragma unroll 1
+    for (int l = lane; l < nl; l += 32) {
+        ps.order[W.mob_rank[lb + l]] = (uint8_t)l;
+        int* seed = W.pose_seed + ((size_t)p * kMaxLig + l) * 3;
+        seed[0] = seed[1] = seed[2] = -1;
+        *reinterpret_cast<uint4*>(W.pose_rec + ((size_t)p * kMaxLig + l) * kMaskWords) = make_uint4(0u, 0u, 0u, 0u);
+    }
+    if (lane < kMaskWords) ps.done[lane] = 0;
+    // the face history starts the pose at zero, as the reference's ptorder does on a workspace
+    // cleared before the pose
+    if (hist) {
+        uint4* h4 = reinterpret_cast<uint4*>(hist);
         #pragma unroll 1
-        for (int l = lane; l < nl; l += 32) {
-            ps.order[W.mob_rank[lb + l]] = (uint8_t)l;
-            seed[l][0] = seed[l][1] = seed[l][2] = -1;
-#pragma unroll
-            for (int w = 0; w < kMaskWords; ++w) kept[l][w] = 0;
-        }
-        if (lane < kMaskWords) ps.done[lane] = 0;
-        // the face history starts the pose at zero, as the reference's ptorder does on a workspace
-        // cleared before the pose
-        if (hist) {
-            uint4* h4 = reinterpret_cast<uint4*>(hist);
-            #pragma unroll 1
-            for (int k = lane; k < kHistBytes / 16; k += 32) h4[k] = make_uint4(0u, 0u, 0u, 0u);
-        }
+        for (int k = lane; k < kHistBytes / 16; k += 32) h4[k] = make_uint4(0u, 0u, 0u, 0u);
     }
     __syncwarp();
-    bool scored = false;             // every atom done
-    int miss = 0, lost = 0;          // per lane: faces without a neighbour, and those not replayed
-    // calc_region: atoms in Calclist order (LIB/Vcontacts.cpp:74-139); the current atom's state
-    int r = 0, a = 0, n_cand = 0, NC = 0;
-    size_t cb = 0;
-    Walk walk{0, 0, 0};
-    bool walking = false;
-    #pragma unroll 1
-    for (;;) {
-        bool pending = false;        // the atom has areas to sum
-        if (alive) {
-            int st = kAtomOk;
-            if (!walking) {
-                a = ps.order[r];
-                n_cand = W.cand_n[lb + a];
-                cb = (lb + a) * kMaxCand;
-                if (n_cand < 0) st = kAtomCapacity;
-                else st = start_atom(S, W, p, a, lane, ps, cb, n_cand, kept[a], seed[a], &NC, walk);
-            }
-            if (st == kAtomNone) {   // no contacts: SAS -1, nothing saved, the atom is not marked done
-                ++r;
-            } else {
-                const double rr = f2d(sh.rr);
-                if (st == kAtomOk) st = hull_walk(sh, NC, rr, lane, walk);
-                walking = st == kAtomWalking;
-                if (st == kAtomOk) {
-                    int NV = 0;
-                    const double rado = sh.rado;
-                    st = arc_points(sh, rado, rr, lane, walk.vn, walk.edges, &NV);
-                    if (st == kAtomOk) st = order_faces(sh, NC, NV, rado, lane, hist, miss, lost);
-                    if (st == kAtomOk) st = area_items(sh, NC, NV, rado, rr, lane);
-                    pending = st == kAtomOk;
-                }
-                if (!pending && !walking) {
-                    alive = false;
-                    if (st == kAtomRetry) {
-                        result = kAtomRetry;
-                    } else if (st == kAtomHullFail) {
-                        if (lane == 0) atomicAdd(&W.counters[1], 1);
-                        finish_failed(W, p, lane, FXE_POSE_POLYHEDRON_FAILED, (double)kPolyPenalty);
-                    } else {
-                        if (lane == 0) atomicAdd(&W.counters[2], 1);
-                        finish_failed(W, p, lane, FXE_POSE_CAPACITY, 0.0);
-                    }
-                }
-            }
-        }
-        if (lane == 0 && warp < Sh::poses) block.items[warp] = pending ? make_int2(sh.nt, sh.na + sh.ne) : make_int2(0, 0);
-        __syncthreads();
-        pooled_areas(all, block.items, warp, lane);
-        const bool more = __syncthreads_or(alive && r + (pending ? 1 : 0) < nl);
-        if (pending) {
-            ++r;
-            // save_areas (LIB/Vcontacts.cpp:1149-1220): contacts with area > 0 on a contact plane;
-            // candidates outside the contact list record nothing
-            #pragma unroll 1
-            for (int c = lane; c < n_cand; c += 32) {
-                if (bit(sh.excl, c)) {
-                    W.cand_area[cb + c] = 0.0;
-                    W.cand_flag[cb + c] = 0;
-                }
-            }
-            const int az = slot_of(S, a);
-            #pragma unroll 1
-            for (int k = lane; k < NC; k += 32) {
-                const double ar = face_area(sh, k);
-                const uint8_t f = sh.flag[k];
-                const bool keep = gt0(ar) && (f & (kOnHull | kEngulf));
-                const int c = sh.cslot[k];
-                W.cand_area[cb + c] = ar;
-                W.cand_flag[cb + c] = (uint8_t)(f | (keep ? kRecorded : 0));
-                const int m = sh.cmob[k];
-                if (m != kNone) {
-                    if (keep) kept[m][a >> 5] |= 1u << (a & 31);
-                    // save_seeds (LIB/Vcontacts.cpp:601-629): the first vertex naming a later atom's plane
-                    const int vi = sh.fseed[k];
-                    if (vi != kNone && seed[m][0] == -1) {
-                        const uchar4 q = sh.vp[vi];
-                        const int p1 = q.x == k ? q.y : q.x, p2 = q.z == k ? q.y : q.z;
-                        seed[m][0] = az;
-                        seed[m][1] = sh.cidx[p1];
-                        seed[m][2] = sh.cidx[p2];
-                    }
-                }
-            }
-            if (lane == 0) ps.done[a >> 5] |= 1u << (a & 31);
-            __syncwarp();
-        }
-        if (!more) break;
-        if (alive && r == nl) {
-            scored = true;
-            alive = false;
-        }
-    }
-    if (result != kAtomRetry) {
-        miss = warp_sum(miss);
-        lost = warp_sum(lost);
-        if (lane == 0 && miss) atomicAdd(&W.counters[3], miss);
-        if (lane == 0 && lost) atomicAdd(&W.counters[0], lost);
-    }
-    if (alive || scored) score_contacts(S, W, p, lane);
-    return result;
+    q.r = q.miss = q.lost = 0;
+    q.walking = false;
+    return true;
 }
 
-constexpr size_t kPoseSmem = sizeof(PoseShared<Compact>) * Compact::poses;
-static_assert(kPoseSmem + 512 <= 227 * 1024, "sixteen poses per SM");
-static_assert(sizeof(PoseShared<Large>) * Large::poses <= kPoseSmem, "the large shape's poses fit the same block");
+// The pose's share of a group step up to the area items: its next atom (or more of its walk).
+// kAtomOk: the atom has items and areas to sum; kAtomWalking; kAtomNone: an atom without contacts;
+// else the pose ends here.
+template <class Sh, class Jobs>
+__device__ __forceinline__ int step_pose(const Jobs& jobs, Pose& q, int lane, PoseShared<Sh>& ps, uint8_t* hist) {
+    static_assert(kMaskWords == 4, "an atom's mask is read as one uint4");
+    const DevSystem& S = jobs.S(q);
+    const DevWork& W = jobs.W(q);
+    Vor<Sh>& sh = ps.v;
+    const size_t lb = (size_t)q.p * n_mobile(S);
+    if (!q.walking) {
+        q.a = ps.order[q.r];
+        q.n_cand = W.cand_n[lb + q.a];
+        if (q.n_cand < 0) return kAtomCapacity;
+        const int st = start_atom(S, W, q.p, q.a, lane, ps, (lb + q.a) * kMaxCand, q.n_cand,
+                                  W.pose_rec + ((size_t)q.p * kMaxLig + q.a) * kMaskWords,
+                                  W.pose_seed + ((size_t)q.p * kMaxLig + q.a) * 3, &q.NC, q.walk);
+        if (st != kAtomOk) return st;
+    }
+    const double rr = f2d(sh.rr), rado = sh.rado;
+    int st = hull_walk(sh, q.NC, rr, lane, q.walk), NV = 0;
+    q.walking = st == kAtomWalking;
+    if (st == kAtomOk) st = arc_points(sh, rado, rr, lane, q.walk.vn, q.walk.edges, &NV);
+    if (st == kAtomOk) st = order_faces(sh, q.NC, NV, rado, lane, hist, q.miss, q.lost);
+    if (st == kAtomOk) st = area_items(sh, q.NC, NV, rado, rr, lane);
+    return st;
+}
 
-// Poses are handed out from a queue (`next`, zeroed before the launch; order: n poses): the launch
-// keeps only as many blocks as the SMs hold at once, and each takes `tile` neighbouring poses at a
-// time (its first `tile` warps score them; the others help with their areas). job_of(entry, &S, &W)
-// gives a queue entry's system and workspace and its index there.
-template <typename JobOf>
-__device__ __forceinline__ void score_queue(int n, int* next, const int* __restrict__ order, uint8_t* hist_all, int tile, JobOf job_of) {
+// Saves the atom whose areas are in: save_areas (LIB/Vcontacts.cpp:1149-1220: contacts with area > 0 on
+// a contact plane; candidates outside the contact list record nothing), save_seeds (:601-629: the first
+// vertex naming a later atom's plane), and its terms.
+template <class Sh, class Jobs>
+__device__ __forceinline__ void save_atom(const Jobs& jobs, const Pose& q, int lane, PoseShared<Sh>& ps) {
+    const DevSystem& S = jobs.S(q);
+    const DevWork& W = jobs.W(q);
+    Vor<Sh>& sh = ps.v;
+    const size_t lb = (size_t)q.p * n_mobile(S), cb = (lb + q.a) * kMaxCand;
+    const int az = slot_of(S, q.a);
+    #pragma unroll 1
+    for (int c = lane; c < q.n_cand; c += 32) {
+        if (bit(sh.excl, c)) {
+            W.cand_area[cb + c] = 0.0;
+            W.cand_flag[cb + c] = 0;
+        }
+    }
+    #pragma unroll 1
+    for (int k = lane; k < q.NC; k += 32) {
+        const double ar = face_area(sh, k);
+        const uint8_t f = sh.flag[k];
+        const bool keep = gt0(ar) && (f & (kOnHull | kEngulf));
+        const int c = sh.cslot[k];
+        W.cand_area[cb + c] = ar;
+        W.cand_flag[cb + c] = (uint8_t)(f | (keep ? kRecorded : 0));
+        const int m = sh.cmob[k];
+        if (m != kNone) {
+            if (keep) W.pose_rec[((size_t)q.p * kMaxLig + m) * kMaskWords + (q.a >> 5)] |= 1u << (q.a & 31);
+            int* seed = W.pose_seed + ((size_t)q.p * kMaxLig + m) * 3;
+            const int vi = sh.fseed[k];
+            if (vi != kNone && seed[0] == -1) {
+                const uchar4 v = sh.vp[vi];
+                const int p1 = v.x == k ? v.y : v.x, p2 = v.z == k ? v.y : v.z;
+                seed[0] = az;
+                seed[1] = sh.cidx[p1];
+                seed[2] = sh.cidx[p2];
+            }
+        }
+    }
+    if (lane == 0) ps.done[q.a >> 5] |= 1u << (q.a & 31);
+    __syncwarp();
+    score_atom(S, W, lb, q.a, lane);
+}
+
+// The launch's counters of a finished pose.
+__device__ __forceinline__ void count_faces(const DevWork& W, const Pose& q, int lane) {
+    const int miss = warp_sum(q.miss), lost = warp_sum(q.lost);
+    if (lane == 0 && miss) atomicAdd(&W.counters[3], miss);
+    if (lane == 0 && lost) atomicAdd(&W.counters[0], lost);
+}
+
+// Scores poses group step by group step: in each step every pose of the group takes its next atom (or
+// goes on with its walk), the group evaluates the areas' items, and each pose saves its atom. A warp
+// whose pose is through takes another (next_pose(&q): false when it gets none; warps without a pose
+// help with the others' areas). Returns when no warp has one. all: the group's workspaces, for its
+// first `poses` warps.
+template <class Sh, int kSize, class Jobs, typename NextPose>
+__device__ __forceinline__ void score_poses(const Jobs& jobs, int lane, PoseShared<Sh>* all, int poses, const Group<kSize>& g,
+                                            uint8_t* hist, NextPose next_pose) {
+    PoseShared<Sh>& ps = all[g.slot < poses ? g.slot : 0];
+    Pose q;
+    q.alive = false;
+    bool more = g.slot < poses;          // poses may be left for this warp
+    #pragma unroll 1
+    for (;;) {
+        while (!q.alive && more) {
+            more = next_pose(q);
+            if (more) q.alive = begin_pose(jobs, q, lane, ps, hist);
+        }
+        int st = kAtomNone;
+        if (q.alive) {
+            st = step_pose(jobs, q, lane, ps, hist);
+            if (st == kAtomNone) {
+                __syncwarp();
+                ++q.r;
+            } else if (st == kAtomRetry) {
+                q.alive = false;
+                if (lane == 0) g.retry[atomicAdd(g.n_retry, 1)] = q.entry;
+            } else if (st != kAtomOk && st != kAtomWalking) {
+                const DevWork& W = jobs.W(q);
+                q.alive = false;
+                if (lane == 0) atomicAdd(&W.counters[st == kAtomHullFail ? 1 : 2], 1);
+                if (st == kAtomHullFail) finish_failed(W, q.p, lane, FXE_POSE_POLYHEDRON_FAILED, (double)kPolyPenalty);
+                else finish_failed(W, q.p, lane, FXE_POSE_CAPACITY, 0.0);
+                count_faces(W, q, lane);
+            }
+        }
+        const bool pending = q.alive && st == kAtomOk;
+        if (lane == 0) g.step[g.slot] = make_int4(pending ? ps.v.nt : 0, pending ? ps.v.na + ps.v.ne : 0, q.alive || more, 0);
+        group_sync(g);
+        if (!__any_sync(kFull, lane < g.size && g.step[lane].z != 0)) break;
+        pooled_areas(all, g, lane);
+        group_sync(g);
+        if (pending) {
+            save_atom(jobs, q, lane, ps);
+            ++q.r;
+        }
+        if (q.alive && !q.walking && q.r == n_mobile(jobs.S(q))) {
+            __syncwarp();
+            finish_scored(jobs.S(q), jobs.W(q), q.p, lane);
+            count_faces(jobs.W(q), q, lane);
+            q.alive = false;
+        }
+    }
+    group_sync(g);
+}
+
+constexpr size_t kPoseSmem = sizeof(PoseShared<Compact>) * kWarps;
+static_assert(kPoseSmem + 512 <= 227 * 1024, "sixteen poses per SM");
+static_assert(sizeof(PoseShared<Large>) * Large::poses <= kPoseSmem && sizeof(PoseShared<Large>) <= kPoseSmem / 4,
+              "the large shape's poses fit a block, and one fits the smallest group's share");
+
+// Poses are handed out from a queue (order: n entries): the launch keeps only as many blocks as the
+// SMs hold at once. The first `active` warps of each group score poses: their first ones are dealt,
+// costliest first, over the launch's groups and back, so that each group gets costly and cheap ones;
+// then each takes the next (`next`, zeroed before the launch) when it is through with one, at the
+// group's next step. (When a block took sixteen poses at a time and waited for the last of them, 30,011
+// poses of a screen took 19.4 ms; 13.8 so.)
+template <int kSize, class Jobs>
+__device__ __forceinline__ void score_queue(const Jobs& jobs, int n, int* next, const int* __restrict__ order, uint8_t* hist_all,
+                                            int active) {
     extern __shared__ __align__(32) unsigned char smem[];
-    __shared__ BlockState b;
+    __shared__ int4 step[kWarps];
+    __shared__ int n_retry_of[kWarps], retry[2 * kWarps];
     const int lane = threadIdx.x & 31, warp = (int)(threadIdx.x >> 5);
+    constexpr int groups = kWarps / kSize;
+    const int group = warp / kSize;
+    Group<kSize> g;
+    g.slot = (warp + group * (4 / groups)) % kSize;   // (a group's first slots: each in another quarter of the SM)
+    g.barrier = group + 1;
+    g.step = step + group * kSize;
+    g.n_retry = n_retry_of + group;
+    g.retry = retry + 2 * group * kSize;
+    unsigned char* const mem = smem + sizeof(PoseShared<Compact>) * kSize * group;
+    constexpr int large = kSize * Large::poses / kWarps;
     // the warp's face history (hist_all: kHistStride bytes per warp of the launch), or null
     uint8_t* hist = hist_all ? hist_all + (size_t)(blockIdx.x * kWarps + warp) * kHistStride : nullptr;
-    const DevSystem* S;
-    const DevWork* W;
+    const int all_groups = groups * gridDim.x, at = group * gridDim.x + blockIdx.x;
+    int dealt = g.slot * all_groups + (g.slot & 1 ? all_groups - 1 - at : at);
+    bool empty = g.slot >= active;       // no more poses for this warp
     #pragma unroll 1
     for (;;) {
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            b.base = atomicAdd(next, tile);
-            b.n_retry = 0;
-        }
-        __syncthreads();
-        const int q = b.base + warp;
-        if (b.base >= n) break;
-        const int entry = warp < tile && q < n ? order[q] : -1;
-        const int p = job_of(entry, &S, &W);
-        if (score_pose(*S, *W, p, lane, reinterpret_cast<PoseShared<Compact>*>(smem), b, hist) == kAtomRetry && lane == 0)
-            b.retry[atomicAdd(&b.n_retry, 1)] = entry;
-        __syncthreads();
-        const int n_retry = b.n_retry;
-        #pragma unroll 1
-        for (int i = 0; i < n_retry; i += Large::poses) {
-            const int again = warp < Large::poses && i + warp < n_retry ? b.retry[i + warp] : -1;
-            const int pa = job_of(again, &S, &W);
-            score_pose(*S, *W, pa, lane, reinterpret_cast<PoseShared<Large>*>(smem), b, hist);
-            __syncthreads();
-        }
+        if (g.slot == 0 && lane == 0) *g.n_retry = 0;
+        group_sync(g);
+        score_poses(jobs, lane, reinterpret_cast<PoseShared<Compact>*>(mem), kSize, g, hist, [&](Pose& q) {
+            if (empty) return false;
+            int e = dealt;
+            dealt = -1;
+            if (e < 0) {
+                // (the list of poses to score again has room for those under way)
+                if (lane == 0 && *(volatile int*)g.n_retry <= g.size) e = active * all_groups + atomicAdd(next, 1);
+                e = __shfl_sync(kFull, e, 0);
+                if (e < 0) return false;
+                empty = e >= n;
+                if (empty) return false;
+            } else if (e >= n) {
+                empty = true;
+                return false;
+            }
+            q.entry = order[e];
+            jobs.place(q);
+            return true;
+        });
+        const int n_retry = *g.n_retry;
+        if (n_retry == 0) break;
+        int i = g.slot;
+        score_poses(jobs, lane, reinterpret_cast<PoseShared<Large>*>(mem), large, g, hist, [&](Pose& q) {
+            if (i >= n_retry) return false;
+            q.entry = g.retry[i];
+            i += large;
+            jobs.place(q);
+            return true;
+        });
     }
 }
 
+template <int kSize>
 __global__ void __launch_bounds__(kWarps * 32)
-pose_kernel(const __grid_constant__ DevSystem S, const __grid_constant__ DevWork W, int n, int* next, uint8_t* hist_all, int tile) {
-    score_queue(n, next, W.pose_order, hist_all, tile, [&](int entry, const DevSystem** s, const DevWork** w) {
-        *s = &S;
-        *w = &W;
-        return entry;
-    });
+pose_kernel(const __grid_constant__ DevSystem S, const __grid_constant__ DevWork W, int n, int* next, uint8_t* hist_all, int active) {
+    score_queue<kSize>(OneJob{S, W}, n, next, W.pose_order, hist_all, active);
 }
 
-// The same over the poses of several jobs; the job's system and workspace descriptors are read
-// from the job table (they stay in L1), keeping shared memory for the polyhedron workspace.
+template <int kSize>
 __global__ void __launch_bounds__(kWarps * 32)
 pose_kernel_jobs(const Job* __restrict__ jobs, int n_jobs, int n, int* next, const int* __restrict__ order, uint8_t* hist_all,
-                 int tile) {
-    score_queue(n, next, order, hist_all, tile, [&](int entry, const DevSystem** s, const DevWork** w) {
-        const Job& job = jobs[entry >= 0 ? find_job(jobs, n_jobs, entry, false) : 0];
-        *s = &job.S;
-        *w = &job.W;
-        return entry >= 0 ? entry - job.pose0 : -1;
-    });
+                 int active) {
+    score_queue<kSize>(ManyJobs{jobs, n_jobs}, n, next, order, hist_all, active);
 }
 
 static int g_sms = 0, g_per_sm = 0;   // SMs, and blocks of pose_kernel one SM holds
@@ -1933,20 +2106,21 @@ static int max_blocks(size_t hist_bytes, int blocks_per_sm) {
     return b > 0 ? b : 1;
 }
 
-// Poses a block takes at a time: one per warp, or fewer when the launch's poses would not reach every
-// block the device runs at once, so that they spread over more SMs (a pose's time is its chain of
-// atoms, shorter with fewer warps sharing the SM's double-precision unit).
-int pose_tile_for(int n, size_t hist_bytes, int blocks_per_sm) {
+// A launch's blocks, its groups' size, and the warps of each group that take poses: all of them, or
+// fewer when the launch's poses would not reach every block the device runs at once, so that they
+// spread over more SMs (a pose's time is its chain of atoms, shorter with fewer warps sharing the
+// SM's double-precision unit). Up to kSplitPoses poses per block two groups of eight warps share it: a
+// pose waits for fewer others (500 poses of 40 atoms: 1,861 us, one group of sixteen 1,998); with the
+// block full their code no longer meets in the instruction cache (2,000 poses: 8.7 ms against 7.8).
+constexpr int kSplitPoses = 4;
+static void launch_shape(int n, size_t hist_bytes, int blocks_per_sm, int* blocks, int* group, int* active) {
     const int r = max_blocks(hist_bytes, blocks_per_sm);
-    const int t = (int)(((long long)n + r - 1) / r);
-    return t < 1 ? 1 : (t > kWarps ? kWarps : t);
-}
-
-// The blocks of a launch over n poses: one per tile of poses, no more than run at once.
-int pose_launch_blocks(int n, size_t hist_bytes, int blocks_per_sm) {
-    const int per = pose_tile_for(n, hist_bytes, blocks_per_sm);
-    const int b = (n + per - 1) / per, r = max_blocks(hist_bytes, blocks_per_sm);
-    return b > r ? r : (b > 0 ? b : 1);
+    const int t = std::max(1, std::min((n + r - 1) / r, kWarps));
+    *group = t <= kSplitPoses ? kWarps / 2 : kWarps;
+    const int groups = kWarps / *group;
+    *active = (t + groups - 1) / groups;
+    const int per = *active * groups;
+    *blocks = std::max(1, std::min((n + per - 1) / per, r));
 }
 
 int pose_max_blocks_per_sm() { return g_per_sm; }
@@ -1956,30 +2130,34 @@ int pose_max_blocks_per_sm() { return g_per_sm; }
 void launch_poses(const DevSystem& S, const DevWork& W, int n, int* next, uint8_t* hist, size_t hist_bytes,
                   int blocks_per_sm, cudaStream_t st) {
     if (hist_bytes < kWarps * kHistStride) hist = nullptr;
-    if (!hist) hist_bytes = 0;
+    int blocks, group, active;
+    launch_shape(n, hist ? hist_bytes : 0, blocks_per_sm, &blocks, &group, &active);
     cudaMemsetAsync(next, 0, sizeof(int), st);
-    pose_kernel<<<pose_launch_blocks(n, hist_bytes, blocks_per_sm), kWarps * 32, kPoseSmem, st>>>(
-        S, W, n, next, hist, pose_tile_for(n, hist_bytes, blocks_per_sm));
+    auto* kernel = group == kWarps ? pose_kernel<kWarps> : pose_kernel<kWarps / 2>;
+    kernel<<<blocks, kWarps * 32, kPoseSmem, st>>>(S, W, n, next, hist, active);
 }
 
 void launch_poses_jobs(const Job* jobs, int n_jobs, int total, int* next, const int* order, uint8_t* hist,
                        size_t hist_bytes, int blocks_per_sm, cudaStream_t st) {
     if (hist_bytes < kWarps * kHistStride) hist = nullptr;
-    if (!hist) hist_bytes = 0;
+    int blocks, group, active;
+    launch_shape(total, hist ? hist_bytes : 0, blocks_per_sm, &blocks, &group, &active);
     cudaMemsetAsync(next, 0, sizeof(int), st);
-    pose_kernel_jobs<<<pose_launch_blocks(total, hist_bytes, blocks_per_sm), kWarps * 32, kPoseSmem, st>>>(
-        jobs, n_jobs, total, next, order, hist, pose_tile_for(total, hist_bytes, blocks_per_sm));
+    auto* kernel = group == kWarps ? pose_kernel_jobs<kWarps> : pose_kernel_jobs<kWarps / 2>;
+    kernel<<<blocks, kWarps * 32, kPoseSmem, st>>>(jobs, n_jobs, total, next, order, hist, active);
 }
 
 cudaError_t configure_voronoi() {
-    cudaError_t e = cudaFuncSetAttribute(pose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPoseSmem);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(pose_kernel_jobs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPoseSmem);
-    if (e != cudaSuccess) return e;
+    for (const void* k : {(const void*)pose_kernel<kWarps>, (const void*)pose_kernel<kWarps / 2>,
+                          (const void*)pose_kernel_jobs<kWarps>, (const void*)pose_kernel_jobs<kWarps / 2>}) {
+        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPoseSmem);
+        if (e != cudaSuccess) return e;
+    }
+    cudaError_t e;
     int dev = 0, sms = 0, per_sm = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pose_kernel, kWarps * 32, kPoseSmem)) != cudaSuccess) return e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pose_kernel<kWarps>, kWarps * 32, kPoseSmem)) != cudaSuccess) return e;
     g_sms = sms;
     g_per_sm = per_sm > 0 ? per_sm : 1;
     return cudaSuccess;
