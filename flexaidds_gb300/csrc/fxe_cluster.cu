@@ -27,36 +27,50 @@ namespace fxe {
 // limits, so the two agree). Each thread forms its atoms' ICs without replaying the assignment:
 // the host's replay names the gene (or grid point, or base IC) that sets each distance, angle and
 // dihedral last, and the atoms whose shifts a dihedral cascade adds (dis_src, trig_src, cas_*).
-// Shared memory, per block: the placed atoms [3 * n_lig][kThreadBuild], and per gene its value as
-// a float and its bin [n_genes][kThreadBuild] each.
-constexpr int kThreadBuild = 64;
+// What bounds it is latency, an atom's chain of table look-ups and its placement from three earlier
+// atoms, so the SM has to hold many warps: the placed atoms stay in the coordinates in global memory
+// (a thread reads back its own; its references are recent and hit the caches), and shared memory holds
+// what is the same for all chromosomes (BuildAtom, by build order) and the genes as floats,
+// [n_genes][kThreadBuild], little enough to leave the rest to the L1 cache. 200,000 chromosomes of 19
+// genes: 500 us with the atoms in shared memory (12 warps an SM), 263 so (40 warps; serialised launches).
+constexpr int kThreadBuild = 128;
 constexpr int kPassThreads = 256;
 
+struct __align__(16) BuildAtom {
+    float4 base;       // base distance, angle, dihedral
+    int4 ref;          // the atoms it is placed from
+    int l, dis, angle, dihedral;       // the atom, and the genes (-2: grid, -1: base) that set its ICs
+    int cas_lo, cas_hi;                // the atoms whose shifts its dihedral adds
+    int tab_a, tab_d, cnt_a, cnt_d;    // its angle's and its dihedral's table: first entry, entries
+    int pad[2];
+};
+
 size_t thread_build_smem(const DevSystem& S) {
-    return sizeof(float) * kThreadBuild * (3 * (size_t)S.n_lig + 2 * (size_t)S.n_genes);
+    return sizeof(BuildAtom) * (size_t)S.n_build + sizeof(float) * kThreadBuild * (size_t)S.n_genes;
 }
 
-__global__ void __launch_bounds__(kThreadBuild)
-cluster_build_thread_kernel(DevSystem S, int n, const double* __restrict__ ic, float* __restrict__ xyz,
-                            int* __restrict__ bad) {
-    extern __shared__ __align__(16) float tsm[];
+__global__ void __launch_bounds__(kThreadBuild, 10)
+cluster_build_thread_kernel(DevSystem S, int n, const double* __restrict__ ic, float* xyz, int* __restrict__ bad) {
+    extern __shared__ __align__(16) unsigned char tsm[];
     const int t = threadIdx.x, ng = S.n_genes, nl = S.n_lig;
-    float* pos = tsm;                                    // [(3 l + k) * kThreadBuild + t]
-    float* fv = pos + (size_t)3 * nl * kThreadBuild;     // [g * kThreadBuild + t]
-    int* gb = reinterpret_cast<int*>(fv + (size_t)ng * kThreadBuild);
+    BuildAtom* atoms = reinterpret_cast<BuildAtom*>(tsm);
+    float* fv = reinterpret_cast<float*>(atoms + S.n_build);   // [g * kThreadBuild + t]
+    for (int an = t; an < S.n_build; an += kThreadBuild) {
+        const int l = S.build_order[an];
+        atoms[an] = {S.lig_ic[l], S.lig_rec[l], l, S.dis_src[l], S.trig_src[2 * l], S.trig_src[2 * l + 1],
+                     S.cas_off[l], S.cas_off[l + 1], S.trig_off[2 * l], S.trig_off[2 * l + 1], S.trig_cnt[2 * l],
+                     S.trig_cnt[2 * l + 1], {0, 0}};
+    }
+    __syncthreads();
     const int p = blockIdx.x * kThreadBuild + t;
     if (p >= n) return;   // no block-wide barrier follows
+    float* const pos = xyz + p;                                // [(3 l + k) * n]
     const double* row = ic + (size_t)p * ng;
     int gi = -1, st = 0;
     for (int g = 0; g < ng; ++g) {
         const double v = row[g];
         if (!(v >= S.gene_min[g] && v <= S.gene_max[g])) st |= 2;
-        // a guess, in single precision, of the bin this value comes from; a table entry is used
-        // only if its angle matches, and a miss retries with the bin formed in double precision
-        const float f = (float)v;
-        const float b = (f - S.gene_minf[g]) * S.gene_idelf[g];
-        gb[g * kThreadBuild + t] = (b >= 0.0f && b < 2.0e9f) ? (int)rintf(b) : -1;
-        fv[g * kThreadBuild + t] = f;
+        fv[g * kThreadBuild + t] = (float)v;
         if (S.gene_type[g] == -1) {
             // the grid gene (LIB/ic2cf.cpp:60-67); an index past the grid is an error and leaves
             // the anchor's base ICs
@@ -66,38 +80,48 @@ cluster_build_thread_kernel(DevSystem S, int n, const double* __restrict__ ic, f
         }
     }
     if (st) atomicOr(bad, st);
-    for (int k = 0; k < 3 * nl; ++k) pos[k * kThreadBuild + t] = 0.0f;
+    // atoms that are never placed, or referenced before they are, read as zero (none of either when the
+    // build order has levels and holds every atom)
+    if (S.n_levels == 0 || S.n_build < nl)
+        for (int k = 0; k < 3 * nl; ++k) pos[(size_t)k * n] = 0.0f;
     const float4 grid = gi >= 0 ? S.grid_ic[gi] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     for (int an = 0; an < S.n_build; ++an) {
-        const int l = S.build_order[an];
-        const float4 base = S.lig_ic[l];
+        const BuildAtom& at = atoms[an];
+        const int l = at.l;
+        const float4 base = at.base;
         // distance, angle and dihedral as the IC assignment leaves them
-        const int sd = S.dis_src[l], sa = S.trig_src[2 * l], sx = S.trig_src[2 * l + 1];
+        const int sd = at.dis, sa = at.angle, sx = at.dihedral;
         const float dis = sd == -2 ? (gi >= 0 ? grid.x : base.x) : (sd >= 0 ? fv[sd * kThreadBuild + t] : base.x);
         const float ang = sa == -2 ? (gi >= 0 ? grid.y : base.y) : (sa >= 0 ? fv[sa * kThreadBuild + t] : base.y);
         float dih = sx == -2 ? (gi >= 0 ? grid.z : base.z) : (sx >= 0 ? fv[sx * kThreadBuild + t] : base.z);
         if (sx >= 0)
-            for (int q = S.cas_off[l]; q < S.cas_off[l + 1]; ++q) dih = dih + S.lig_shift[S.cas_atom[q]];
+            for (int q = at.cas_lo; q < at.cas_hi; ++q) dih = dih + S.lig_shift[S.cas_atom[q]];
         float ca, sn_a, cd, sn_d;
-        auto trig = [&](int c, int src, float deg, float* cs, float* sn) {
-            if (trig_table(S, l, c, gi, src >= 0 ? gb[src * kThreadBuild + t] : -1, deg, cs, sn)) return;
-            if (src >= 0) {
-                const double b = (row[src] - S.gene_min[src]) / S.gene_del[src];
-                const int exact = (b >= 0.0 && b < 2147483647.0) ? (int)rint(b) : -1;
-                if (exact != gb[src * kThreadBuild + t] && trig_table(S, l, c, gi, exact, deg, cs, sn)) return;
+        auto trig = [&](int c, int src, int tab, int cnt, float deg, float* cs, float* sn) {
+            auto entry = [&](int idx) { return (unsigned)idx < (unsigned)cnt && trig_match(S.trig_tab[tab + idx], deg, cs, sn); };
+            if (src == -2) {
+                if (gi >= 0 && trig_match(c == 0 ? S.grid_trig_a[gi] : S.grid_trig_d[gi], deg, cs, sn)) return;
+            } else if (src < 0) {
+                if (entry(0)) return;
+            } else {
+                // a guess, in single precision, of the bin the gene's value comes from; an entry is used
+                // only if its angle matches, and a miss retries with the bin formed in double precision
+                const float b = (fv[src * kThreadBuild + t] - S.gene_minf[src]) * S.gene_idelf[src];
+                const int guess = (b >= 0.0f && b < 2.0e9f) ? (int)rintf(b) : -1;
+                if (entry(guess)) return;
+                const double bd = (row[src] - S.gene_min[src]) / S.gene_del[src];
+                const int exact = (bd >= 0.0 && bd < 2147483647.0) ? (int)rint(bd) : -1;
+                if (exact != guess && entry(exact)) return;
             }
             trig_exact(deg, cs, sn);
         };
-        trig(0, sa, ang, &ca, &sn_a);
-        trig(1, sx, dih, &cd, &sn_d);
+        trig(0, sa, at.tab_a, at.cnt_a, ang, &ca, &sn_a);
+        trig(1, sx, at.tab_d, at.cnt_d, dih, &cd, &sn_d);
         float x[4], y[4], z[4], out[3];
-        buildcc_refs(S, S.lig_rec[l], [&](int j, int k) { return pos[(3 * j + k) * kThreadBuild + t]; }, x, y, z);
+        buildcc_refs(S, at.ref, [&](int j, int k) { return pos[(size_t)(3 * j + k) * n]; }, x, y, z);
         buildcc_place(x, y, z, dis, ca, sn_a, cd, sn_d, out);
-        pos[(3 * l) * kThreadBuild + t] = out[0];
-        pos[(3 * l + 1) * kThreadBuild + t] = out[1];
-        pos[(3 * l + 2) * kThreadBuild + t] = out[2];
+        for (int k = 0; k < 3; ++k) pos[(size_t)(3 * l + k) * n] = out[k];
     }
-    for (int k = 0; k < 3 * nl; ++k) xyz[(size_t)k * n + p] = pos[k * kThreadBuild + t];
 }
 
 // Partition function of the clustering step: sum of exp(-beta * app_evalue)
@@ -117,24 +141,34 @@ cluster_z_kernel(int n, const double* __restrict__ e, double beta, double* __res
     if (threadIdx.x == 0) part[blockIdx.x] = red[0];
 }
 
-__device__ __forceinline__ double sum_partials(const double* __restrict__ part, int nb) {
-    double z = 0.0;
-    for (int b = 0; b < nb; ++b) z += part[b];
+// The partials' sum, by one warp.
+template <typename T>
+__device__ __forceinline__ T sum_partials(const T* __restrict__ part, int nb, int lane) {
+    T z = 0;
+    for (int b = lane; b < nb; b += 32) z += part[b];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
     return z;
 }
+
+// What bounds a pass is the latency of its loads, repeated until the farthest-going lane of a warp gives
+// its chromosome up: the atoms come kPassAtoms at a time. (Most far chromosomes share the head's place and
+// differ in orientation: a test of the centroids first gave nothing up soon enough to pay.) 200,000
+// chromosomes: 42 us with an atom at a time, 24 so.
+constexpr int kPassAtoms = 4;
 
 // Cluster c. Its head is next[c]: 0 for the first cluster, else the first chromosome the pass of
 // cluster c - 1 left unclustered (n: none left, no cluster). Every later unclustered chromosome
 // whose RMSD to the head is at most thr joins (member, rmsd); the others bid for next[c + 1].
 // Each block leaves its members' count and their share of the cluster's ACF in part_cnt/part_acf
 // at [c * gridDim.x + block].
-__global__ void __launch_bounds__(kPassThreads)
+__global__ void __launch_bounds__(kPassThreads, 6)
 cluster_pass_kernel(int n, int nl, int c, const float* __restrict__ xyz, float thr, float exit_sum,
                     const double* __restrict__ e, int temperature, double beta,
                     const double* __restrict__ part_z, int nb_z, int* __restrict__ member,
                     float* __restrict__ rmsd, int* __restrict__ next, double* __restrict__ part_acf,
                     int* __restrict__ part_cnt) {
-    __shared__ float head_xyz[3 * kMaxLig];
+    __shared__ float head_xyz[3 * (kMaxLig + kPassAtoms)];
     __shared__ double red[kPassThreads];
     __shared__ int red_n[kPassThreads / 32], red_next[kPassThreads / 32];
     __shared__ double z_sh;
@@ -142,7 +176,10 @@ cluster_pass_kernel(int n, int nl, int c, const float* __restrict__ xyz, float t
     if (head >= n) return;
     const int m3 = 3 * nl;
     for (int k = threadIdx.x; k < m3; k += kPassThreads) head_xyz[k] = xyz[(size_t)k * n + head];
-    if (threadIdx.x == 0) z_sh = temperature > 0 ? sum_partials(part_z, nb_z) : 0.0;
+    if (threadIdx.x < 32) {
+        const double zs = temperature > 0 ? sum_partials(part_z, nb_z, threadIdx.x) : 0.0;
+        if (threadIdx.x == 0) z_sh = zs;
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         member[head] = head;
         rmsd[head] = 0.0f;
@@ -157,18 +194,19 @@ cluster_pass_kernel(int n, int nl, int c, const float* __restrict__ xyz, float t
         // the sum of squared coordinate differences in the reference's order
         // (flexaids::sum_sq_distances_f's scalar form, LIB/simd_distance.h:712-713); partial sums
         // only grow, so a chromosome is given up once its partial sum is past exit_sum, a bound
-        // above every sum whose RMSD is within thr
+        // above every sum whose RMSD is within thr. kPassAtoms atoms' loads are under way at a time.
         float s = 0.0f;
         bool far = false;
-        for (int a = 0; a < nl; ++a) {
-            for (int k = 3 * a; k < 3 * a + 3; ++k) {
-                const float d = xyz[(size_t)k * n + i] - head_xyz[k];
-                s = s + d * d;
+        for (int a = 0; a < nl && !far; a += kPassAtoms) {
+            float v[3 * kPassAtoms];
+#pragma unroll
+            for (int k = 0; k < 3 * kPassAtoms; ++k) v[k] = a + k / 3 < nl ? xyz[(size_t)(3 * a + k) * n + i] : 0.0f;
+#pragma unroll
+            for (int k = 0; k < 3 * kPassAtoms; ++k) {
+                const float d = v[k] - head_xyz[3 * a + k];
+                if (a + k / 3 < nl) s = s + d * d;
             }
-            if (s > exit_sum) {
-                far = true;
-                break;
-            }
+            far = s > exit_sum;
         }
         const float r = far ? 0.0f : sqrtf(s / nf);
         if (!far && r <= thr) {
@@ -225,47 +263,48 @@ cluster_finish_kernel(int n, int nl, int R, int nb, const float* __restrict__ xy
                       double* __restrict__ acf, float* __restrict__ head_rmsd, double* __restrict__ z_out) {
     __shared__ double z_sh;
     __shared__ int nc_sh;
-    if (threadIdx.x == 0) {
-        z_sh = temperature > 0 ? sum_partials(part_z, nb_z) : 0.0;
-        int nc = 0;
-        while (nc < R && next[nc] < n) ++nc;
-        nc_sh = nc;
-        *z_out = z_sh;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp == 0) {
+        const double zs = temperature > 0 ? sum_partials(part_z, nb_z, lane) : 0.0;
+        int nc = R;      // the first cluster without a head
+        for (int c = lane; c < R; c += 32)
+            if (next[c] >= n) nc = min(nc, c);
+        nc = __reduce_min_sync(0xffffffffu, nc);
+        if (lane == 0) {
+            z_sh = zs;
+            nc_sh = nc;
+            *z_out = zs;
+        }
     }
     __syncthreads();
     const int nc = nc_sh;
     const double z = z_sh, T = (double)temperature;
-    for (int c = threadIdx.x; c < R; c += kPassThreads) {
-        if (c >= nc) {
-            top[c] = 0;
-            freq[c] = 0;
-            tcf[c] = 0.0;
-            acf[c] = 0.0;
-            continue;
+    for (int c = warp; c < R; c += kPassThreads / 32) {      // a warp per cluster
+        double lead = 0.0, s = 0.0;
+        int h = 0, f = 0;
+        if (c < nc) {
+            h = next[c];
+            if (temperature > 0) {
+                const double pj = exp(-1.0 * beta * e[h]) / z;
+                lead = (double)((pj * e[h]) - (T * pj * log(pj)));
+            } else {
+                lead = e[h];
+            }
+            s = lead + sum_partials(part_acf + (size_t)c * nb, nb, lane);
+            f = 1 + sum_partials(part_cnt + (size_t)c * nb, nb, lane);
         }
-        const int h = next[c];
-        double lead;
-        if (temperature > 0) {
-            const double pj = exp(-1.0 * beta * e[h]) / z;
-            lead = (double)((pj * e[h]) - (T * pj * log(pj)));
-        } else {
-            lead = e[h];
+        if (lane == 0) {
+            top[c] = h;
+            freq[c] = f;
+            tcf[c] = lead;
+            acf[c] = s;
         }
-        double s = lead;
-        int f = 1;
-        for (int b = 0; b < nb; ++b) {
-            s += part_acf[(size_t)c * nb + b];
-            f += part_cnt[(size_t)c * nb + b];
-        }
-        top[c] = h;
-        freq[c] = f;
-        tcf[c] = lead;
-        acf[c] = s;
     }
     for (int q = threadIdx.x; q < nc * nc; q += kPassThreads) {
         const int a = q / nc, b = q % nc;
         const int ha = next[a], hb = next[b];
         float s = 0.0f;
+#pragma unroll 4
         for (int l = 0; l < nl; ++l) {
             const float d0 = xyz[(size_t)(3 * l) * n + ha] - xyz[(size_t)(3 * l) * n + hb];
             const float d1 = xyz[(size_t)(3 * l + 1) * n + ha] - xyz[(size_t)(3 * l + 1) * n + hb];
@@ -278,18 +317,17 @@ cluster_finish_kernel(int n, int nl, int R, int nb, const float* __restrict__ xy
 
 int cluster_blocks(int n) {
     const int want = (n + kPassThreads - 1) / kPassThreads;
-    return want < 4 * 152 ? (want < 1 ? 1 : want) : 4 * 152;
+    return want < 8 * 152 ? (want < 1 ? 1 : want) : 8 * 152;
 }
 
 cudaError_t launch_cluster(const DevSystem& S, const ClusterWork& C, cudaStream_t st) {
     const int n = C.n, nl = S.n_lig, nb = cluster_blocks(n);
-    // at most 128 atoms and 100 genes (checked by the caller): 146 KB for 64 chromosomes
+    // at most 128 atoms and 100 genes (checked by the caller): 61 KB for 128 chromosomes
     const size_t tsmem = thread_build_smem(S);
     cudaError_t e = cudaFuncSetAttribute(cluster_build_thread_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)tsmem);
     if (e != cudaSuccess) return e;
-    cluster_build_thread_kernel<<<(n + kThreadBuild - 1) / kThreadBuild, kThreadBuild, tsmem, st>>>(S, n, C.ic,
-                                                                                                  C.xyz, C.status);
+    cluster_build_thread_kernel<<<(n + kThreadBuild - 1) / kThreadBuild, kThreadBuild, tsmem, st>>>(S, n, C.ic, C.xyz, C.status);
     if (C.temperature > 0) cluster_z_kernel<<<nb, kPassThreads, 0, st>>>(n, C.e, C.beta, C.part_z);
     for (int c = 0; c < C.max_results; ++c)
         cluster_pass_kernel<<<nb, kPassThreads, 0, st>>>(n, nl, c, C.xyz, C.thr, C.exit_sum, C.e, C.temperature,

@@ -30,6 +30,15 @@ struct BuildShared {
 // double precision as buildcc forms it and the entry is used if its x equals x; else the
 // correctly rounded values. gi is the pose's grid point, bin the bin of the gene that sets the
 // angle (-1: none known); trig_table answers whether a table entry gave the pair.
+__device__ __forceinline__ bool trig_match(const float4& e, float deg, float* cs, float* sn) {
+    if (__float_as_int(e.w) == __float_as_int(deg) || __float_as_int(e.x) == __float_as_int((float)(deg * kPi / 180.0f))) {
+        *cs = e.y;
+        *sn = e.z;
+        return true;
+    }
+    return false;
+}
+
 __device__ __forceinline__ bool trig_table(const DevSystem& S, int l, int c, int gi, int bin, float deg, float* cs,
                                            float* sn) {
     const int k = 2 * l + c, src = S.trig_src[k];
@@ -47,13 +56,7 @@ __device__ __forceinline__ bool trig_table(const DevSystem& S, int l, int c, int
             have = true;
         }
     }
-    if (!have) return false;
-    if (__float_as_int(e.w) == __float_as_int(deg) || __float_as_int(e.x) == __float_as_int((float)(deg * kPi / 180.0f))) {
-        *cs = e.y;
-        *sn = e.z;
-        return true;
-    }
-    return false;
+    return have && trig_match(e, deg, cs, sn);
 }
 
 // Correctly rounded cos and sin of the build angle, for angles no table entry holds.
