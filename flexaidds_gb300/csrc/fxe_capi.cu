@@ -97,6 +97,33 @@ struct CallBuffers {
     }
 };
 
+// The same in one allocation (an allocation and its release cost 80 - 170 us from a megabyte up, about
+// alike for one of 1 MB and one of 128 MB): the buffers are laid out twice with take(), first to count
+// the bytes, then, after allocate(), for their addresses.
+struct CallBlock {
+    unsigned char* base = nullptr;
+    size_t bytes = 0;
+    template <typename T>
+    T* take(size_t count) {
+        T* q = base ? reinterpret_cast<T*>(base + bytes) : nullptr;
+        bytes += (count * sizeof(T) + 255) & ~(size_t)255;
+        return q;
+    }
+    cudaError_t allocate() {
+        void* q = nullptr;
+        const cudaError_t e = cudaMalloc(&q, bytes ? bytes : 256);
+        if (e == cudaSuccess) base = static_cast<unsigned char*>(q);
+        bytes = 0;
+        return e;
+    }
+    CallBlock() = default;
+    CallBlock(const CallBlock&) = delete;
+    CallBlock& operator=(const CallBlock&) = delete;
+    ~CallBlock() {
+        if (base) cudaFree(base);
+    }
+};
+
 
 }  // namespace
 
@@ -931,21 +958,19 @@ fxe_status thermo_host(const double* e, const int32_t* mult, int64_t n, double T
     double *d_e = nullptr, *d_w = nullptr;
     int32_t* d_m = nullptr;
     cudaStream_t s = nullptr;
-    auto cleanup = [&]() {
-        if (d_e) cudaFree(d_e);
-        if (d_w) cudaFree(d_w);
-        if (d_m) cudaFree(d_m);
-        if (s) cudaStreamDestroy(s);
+    CallBlock m;
+    auto layout = [&]() {
+        d_e = m.take<double>(n);
+        d_w = w ? m.take<double>(n) : nullptr;
+        d_m = mult ? m.take<int32_t>(n) : nullptr;
     };
     fxe_status st = [&]() -> fxe_status {
         FXE_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "stream");
-        FXE_TRY(cudaMalloc(&d_e, n * sizeof(double)), "thermo input");
+        layout();
+        FXE_TRY(m.allocate(), "thermo input");
+        layout();
         FXE_TRY(cudaMemcpyAsync(d_e, e, n * sizeof(double), cudaMemcpyHostToDevice, s), "thermo input");
-        if (mult) {
-            FXE_TRY(cudaMalloc(&d_m, n * sizeof(int32_t)), "thermo input");
-            FXE_TRY(cudaMemcpyAsync(d_m, mult, n * sizeof(int32_t), cudaMemcpyHostToDevice, s), "thermo input");
-        }
-        if (w) FXE_TRY(cudaMalloc(&d_w, n * sizeof(double)), "thermo output");
+        if (mult) FXE_TRY(cudaMemcpyAsync(d_m, mult, n * sizeof(int32_t), cudaMemcpyHostToDevice, s), "thermo input");
         fxe_status r = thermo_run(d_e, d_m, n, T, out, d_w, s);
         if (r != FXE_OK) return r;
         if (w) {
@@ -954,7 +979,7 @@ fxe_status thermo_host(const double* e, const int32_t* mult, int64_t n, double T
         }
         return FXE_OK;
     }();
-    cleanup();
+    if (s) cudaStreamDestroy(s);
     return st;
 }
 
@@ -1021,21 +1046,6 @@ void quicksort_clusters(int* top, int* fre, double* tcf, double* acf, int* perm,
     }
 }
 
-struct DevScratch {
-    std::vector<void*> p;
-    template <typename T>
-    cudaError_t get(T** out, size_t count) {
-        void* q = nullptr;
-        cudaError_t e = cudaMalloc(&q, count * sizeof(T) + 16);
-        if (e == cudaSuccess) p.push_back(q);
-        *out = reinterpret_cast<T*>(q);
-        return e;
-    }
-    ~DevScratch() {
-        for (void* q : p) cudaFree(q);
-    }
-};
-
 }  // namespace
 
 extern "C" fxe_status fxe_cluster(fxe_context* ctx, int64_t n, const double* ic, const double* app_evalue,
@@ -1055,7 +1065,7 @@ extern "C" fxe_status fxe_cluster(fxe_context* ctx, int64_t n, const double* ic,
     const int N = (int)n, R = max_results, ng = ctx->S.n_genes, nl = ctx->S.n_lig;
     const int nb = fxe::cluster_blocks(N);
     cudaStream_t st = ctx->stream;
-    DevScratch m;
+    CallBlock m;
     fxe::ClusterWork C{};
     C.n = N;
     C.temperature = temperature;
@@ -1072,24 +1082,33 @@ extern "C" fxe_status fxe_cluster(fxe_context* ctx, int64_t n, const double* ic,
     C.max_results = R;
     double* d_ic = nullptr;
     double* d_e = nullptr;
-    FXE_TRY(m.get(&d_ic, (size_t)N * ng), "cluster ICs");
-    FXE_TRY(m.get(&d_e, (size_t)N), "cluster energies");
+    // the results lie together and come back in one copy (res_bytes from C.z on)
+    size_t res_at = 0, res_bytes = 0;
+    auto layout = [&]() {
+        d_ic = m.take<double>((size_t)N * ng);
+        d_e = m.take<double>((size_t)N);
+        C.xyz = m.take<float>((size_t)3 * nl * N);
+        C.part_z = m.take<double>((size_t)nb);
+        C.member = m.take<int>((size_t)N);
+        C.rmsd = m.take<float>((size_t)N);
+        C.part_acf = m.take<double>((size_t)R * nb);
+        C.part_cnt = m.take<int>((size_t)R * nb);
+        res_at = m.bytes;
+        C.z = m.take<double>(1);
+        C.status = m.take<int>(1);
+        C.next = m.take<int>((size_t)R + 1);
+        C.top = m.take<int>((size_t)R);
+        C.freq = m.take<int>((size_t)R);
+        C.tcf = m.take<double>((size_t)R);
+        C.acf = m.take<double>((size_t)R);
+        C.head_rmsd = m.take<float>((size_t)R * R);
+        res_bytes = m.bytes - res_at;
+    };
+    layout();
+    FXE_TRY(m.allocate(), "cluster buffers");
+    layout();
     C.ic = d_ic;
     C.e = d_e;
-    FXE_TRY(m.get(&C.xyz, (size_t)3 * nl * N), "cluster coordinates");
-    FXE_TRY(m.get(&C.status, 1), "cluster status");
-    FXE_TRY(m.get(&C.part_z, (size_t)nb), "cluster partials");
-    FXE_TRY(m.get(&C.member, (size_t)N), "cluster members");
-    FXE_TRY(m.get(&C.rmsd, (size_t)N), "cluster rmsd");
-    FXE_TRY(m.get(&C.next, (size_t)R + 1), "cluster heads");
-    FXE_TRY(m.get(&C.part_acf, (size_t)R * nb), "cluster partials");
-    FXE_TRY(m.get(&C.part_cnt, (size_t)R * nb), "cluster partials");
-    FXE_TRY(m.get(&C.top, (size_t)R), "cluster results");
-    FXE_TRY(m.get(&C.freq, (size_t)R), "cluster results");
-    FXE_TRY(m.get(&C.tcf, (size_t)R), "cluster results");
-    FXE_TRY(m.get(&C.acf, (size_t)R), "cluster results");
-    FXE_TRY(m.get(&C.head_rmsd, (size_t)R * R), "cluster results");
-    FXE_TRY(m.get(&C.z, 1), "cluster results");
     std::vector<int> h_next(R + 1, N);
     h_next[0] = 0;
     cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -1120,18 +1139,23 @@ extern "C" fxe_status fxe_cluster(fxe_context* ctx, int64_t n, const double* ic,
     std::vector<float> h_hr((size_t)R * R);
     int status = 0;
     double z = 0.0;
-    FXE_TRY(cudaMemcpyAsync(h_next.data(), C.next, sizeof(int) * (R + 1), cudaMemcpyDeviceToHost, st), "cluster results");
-    FXE_TRY(cudaMemcpyAsync(h_top.data(), C.top, sizeof(int) * R, cudaMemcpyDeviceToHost, st), "cluster results");
-    FXE_TRY(cudaMemcpyAsync(h_freq.data(), C.freq, sizeof(int) * R, cudaMemcpyDeviceToHost, st), "cluster results");
-    FXE_TRY(cudaMemcpyAsync(h_tcf.data(), C.tcf, sizeof(double) * R, cudaMemcpyDeviceToHost, st), "cluster results");
-    FXE_TRY(cudaMemcpyAsync(h_acf.data(), C.acf, sizeof(double) * R, cudaMemcpyDeviceToHost, st), "cluster results");
-    FXE_TRY(cudaMemcpyAsync(h_hr.data(), C.head_rmsd, sizeof(float) * R * R, cudaMemcpyDeviceToHost, st), "cluster results");
-    FXE_TRY(cudaMemcpyAsync(&status, C.status, sizeof(int), cudaMemcpyDeviceToHost, st), "cluster results");
-    FXE_TRY(cudaMemcpyAsync(&z, C.z, sizeof(double), cudaMemcpyDeviceToHost, st), "cluster results");
+    std::vector<unsigned char> res(res_bytes);
+    FXE_TRY(cudaMemcpyAsync(res.data(), m.base + res_at, res_bytes, cudaMemcpyDeviceToHost, st), "cluster results");
     if (member_of)
         FXE_TRY(cudaMemcpyAsync(member_of, C.member, sizeof(int) * N, cudaMemcpyDeviceToHost, st), "cluster members");
     if (rmsd) FXE_TRY(cudaMemcpyAsync(rmsd, C.rmsd, sizeof(float) * N, cudaMemcpyDeviceToHost, st), "cluster rmsd");
     FXE_TRY(cudaStreamSynchronize(st), "cluster");
+    auto result = [&](void* to, const void* from, size_t bytes) {
+        std::memcpy(to, res.data() + (static_cast<const unsigned char*>(from) - (m.base + res_at)), bytes);
+    };
+    result(h_next.data(), C.next, sizeof(int) * (R + 1));
+    result(h_top.data(), C.top, sizeof(int) * R);
+    result(h_freq.data(), C.freq, sizeof(int) * R);
+    result(h_tcf.data(), C.tcf, sizeof(double) * R);
+    result(h_acf.data(), C.acf, sizeof(double) * R);
+    result(h_hr.data(), C.head_rmsd, sizeof(float) * R * R);
+    result(&status, C.status, sizeof(int));
+    result(&z, C.z, sizeof(double));
     float ms = 0.0f;
     FXE_TRY(cudaEventElapsedTime(&ms, ev[0], ev[1]), "cluster events");
     ctx->cluster_ms = ms;
@@ -2059,17 +2083,24 @@ extern "C" fxe_status fxe_ensemble_dedup(int64_t n, int32_t n_genes, const doubl
     if (n == 0) return FXE_OK;
     int dc = 0;
     if (cudaGetDeviceCount(&dc) != cudaSuccess || dc == 0) return fail(FXE_ERR_NO_DEVICE, "no CUDA device");
-    CallBuffers b;
+    CallBlock b;
     double *d_ic = nullptr, *d_e = nullptr, *d_eo = nullptr;
     long long* d_idx = nullptr;
     unsigned char* scratch = nullptr;
     int* d_cnt = nullptr;
-    FXE_TRY(b.put(&d_ic, ic, (size_t)n * n_genes), "ensemble input");
-    FXE_TRY(b.put(&d_e, energies, (size_t)n), "ensemble input");
-    FXE_TRY(b.get(&d_eo, (size_t)n), "ensemble output");
-    FXE_TRY(b.get(&d_idx, (size_t)n), "ensemble output");
-    FXE_TRY(b.get(&d_cnt, 1), "ensemble output");
-    FXE_TRY(b.get(&scratch, fxe::ensemble_scratch_bytes(n, n_genes)), "ensemble scratch");
+    auto layout = [&]() {
+        d_ic = b.take<double>((size_t)n * n_genes);
+        d_e = b.take<double>((size_t)n);
+        d_eo = b.take<double>((size_t)n);
+        d_idx = b.take<long long>((size_t)n);
+        d_cnt = b.take<int>(1);
+        scratch = b.take<unsigned char>(fxe::ensemble_scratch_bytes(n, n_genes));
+    };
+    layout();
+    FXE_TRY(b.allocate(), "ensemble buffers");
+    layout();
+    FXE_TRY(cudaMemcpy(d_e, energies, sizeof(double) * n, cudaMemcpyHostToDevice), "ensemble input");
+    FXE_TRY(cudaMemcpy(d_ic, ic, sizeof(double) * n * n_genes, cudaMemcpyHostToDevice), "ensemble input");
     FXE_TRY(fxe::launch_ensemble(n, n_genes, d_e, d_ic, nullptr, nullptr, scratch, d_idx, d_eo, nullptr, d_cnt, nullptr),
             "ensemble launch");
     int cnt = 0;
@@ -2077,9 +2108,8 @@ extern "C" fxe_status fxe_ensemble_dedup(int64_t n, int32_t n_genes, const doubl
     if (cnt < 0 || cnt > n) return fail(FXE_ERR_INTERNAL, "ensemble size out of range");
     *n_kept = cnt;
     if (cnt > 0 && kept_index) {
-        std::vector<long long> idx(cnt);
-        FXE_TRY(cudaMemcpy(idx.data(), d_idx, sizeof(long long) * cnt, cudaMemcpyDeviceToHost), "kept indices");
-        for (int i = 0; i < cnt; ++i) kept_index[i] = idx[i];
+        static_assert(sizeof(long long) == sizeof(int64_t), "copied as they are");
+        FXE_TRY(cudaMemcpy(kept_index, d_idx, sizeof(int64_t) * cnt, cudaMemcpyDeviceToHost), "kept indices");
     }
     if (cnt > 0 && kept_energy) FXE_TRY(cudaMemcpy(kept_energy, d_eo, sizeof(double) * cnt, cudaMemcpyDeviceToHost), "kept energies");
     return FXE_OK;
