@@ -3,17 +3,23 @@
 // (QuickSort, :520; ties here keep snapshot order), then remove_dups (:2728-2747): a chromosome is
 // dropped when every decoded gene lies within 0.1 of the last chromosome kept.
 //
-// Sort: least-significant-digit radix sort of the energies' order-preserving 64-bit images, 4 bits
-// a pass (16 passes), each pass a per-block digit count, one scan of the counts and a stable
-// scatter (a block's elements ranked by warp match and per-warp counts), so equal energies keep
-// their input order.
+// Sort: least-significant-digit radix sort of the energies' order-preserving 64-bit images, 8 bits
+// a pass (8 passes), each pass a launch that counts every block's digits and one that scatters, stable
+// (each block adds up the counts before its own, and ranks its elements by warp match and per-warp
+// counts), so equal energies keep their input order.
 //
 // remove_dups is a chain: whether chromosome i is kept depends on which one was kept last. Runs of
 // identical chromosomes (a survivor sits in the population for many generations) are collapsed
 // first: a chromosome identical to its predecessor is always dropped and never becomes the last one
 // kept. Over the remaining run heads, next(t) = the first later head that is not within 0.1 of head
 // t (a bounded scan per thread, then one warp per unresolved head scanning 32 at a time); the kept
-// heads are the path 0, next(0), next(next(0)), ..., marked by pointer jumping in log2(M) rounds.
+// heads are the path 0, next(0), next(next(0)), .... The heads are cut into segments that fit a block's
+// shared memory: one launch finds by pointer jumping where the path leaves the segment from each of its
+// heads, the next follows those exits to its segment and marks the path inside.
+//
+// What bounds the assembly is its number of dependent launches more than the bytes (12 per chromosome
+// and pass, the genes once): 4-bit digits with a three-launch scan each and log2(n) launches of pointer
+// jumping made 130 of them.
 #include <cstdint>
 
 #include "fxe_place.cuh"
@@ -31,14 +37,6 @@ __device__ __forceinline__ unsigned long long order_key(double e) {
     if (e == 0.0) return 0x8000000000000000ull;   // -0 and +0 compare equal
     const unsigned long long b = (unsigned long long)__double_as_longlong(e);
     return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
-}
-
-__global__ void ens_keys_kernel(const double* __restrict__ e, long long n, unsigned long long* __restrict__ key,
-                                int* __restrict__ val) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        key[i] = order_key(e[i]);
-        val[i] = (int)i;
-    }
 }
 
 // --- exclusive scan of int counts (n entries, total written to out[n]) -------------------------
@@ -115,38 +113,112 @@ void scan_ints(const int* in, int* out, long long n, int* tmp, cudaStream_t st) 
 
 // --- radix sort passes --------------------------------------------------------------------------
 
-__global__ void __launch_bounds__(kEnsThreads) radix_hist_kernel(const unsigned long long* __restrict__ key, long long n, int shift,
-                                                                 int* __restrict__ hist) {
-    __shared__ int cnt[16];
-    if (threadIdx.x < 16) cnt[threadIdx.x] = 0;
-    __syncthreads();
-    const long long i = blockIdx.x * (long long)kEnsThreads + threadIdx.x;
-    if (i < n) atomicAdd(&cnt[(int)((key[i] >> shift) & 15ull)], 1);
-    __syncthreads();
-    if (threadIdx.x < 16) hist[(long long)threadIdx.x * gridDim.x + blockIdx.x] = cnt[threadIdx.x];
+constexpr int kRadix = 256;
+constexpr int kRadixItems = 8;                                // keys a thread holds
+constexpr int kRadixTile = kEnsThreads * kRadixItems;
+constexpr int kRadixBlocks = 4 * 152;                         // at most; then a block takes several tiles
+static_assert(kEnsThreads == kRadix, "a digit per thread");
+
+static long long radix_tiles_per_block(long long n) {
+    const long long tiles = (n + kRadixTile - 1) / kRadixTile;
+    return (tiles + kRadixBlocks - 1) / kRadixBlocks;
+}
+static int radix_blocks(long long n) {
+    const long long per = radix_tiles_per_block(n) * kRadixTile;
+    return (int)((n + per - 1) / per);
 }
 
-__global__ void __launch_bounds__(kEnsThreads) radix_scatter_kernel(const unsigned long long* __restrict__ kin, const int* __restrict__ vin,
-                                                                    unsigned long long* __restrict__ kout, int* __restrict__ vout,
-                                                                    long long n, int shift, const int* __restrict__ offs) {
-    __shared__ int wcnt[kEnsThreads / 32][16];
-    const long long i = blockIdx.x * (long long)kEnsThreads + threadIdx.x;
+// The digit counts of each block's run of `per` keys, hist[block * kRadix + digit]. kFirst: the keys
+// are formed from the energies and stored.
+template <bool kFirst>
+__global__ void __launch_bounds__(kEnsThreads)
+radix_count_kernel(const double* __restrict__ e, unsigned long long* __restrict__ key, long long n, long long per, int shift,
+                   int* __restrict__ hist) {
+    __shared__ int cnt[kEnsThreads / 32][kRadix];
     const int w = threadIdx.x >> 5;
-    const bool ok = i < n;
-    const unsigned long long k = ok ? kin[i] : 0ull;
-    const int dg = ok ? (int)((k >> shift) & 15ull) : 16;
-    const unsigned peers = __match_any_sync(0xffffffffu, dg);
-    const int rank = __popc(peers & lanemask_lt());
-    if (threadIdx.x < (kEnsThreads / 32) * 16) wcnt[threadIdx.x >> 4][threadIdx.x & 15] = 0;
+    for (int k = threadIdx.x; k < kEnsThreads / 32 * kRadix; k += kEnsThreads) (&cnt[0][0])[k] = 0;
     __syncthreads();
-    if (ok && rank == 0) wcnt[w][dg] = __popc(peers);
+    const long long lo = (long long)blockIdx.x * per, hi = lo + per < n ? lo + per : n;
+    for (long long i0 = lo; i0 < hi; i0 += kRadixTile) {
+        unsigned long long k[kRadixItems];
+#pragma unroll
+        for (int j = 0; j < kRadixItems; ++j) {
+            const long long i = i0 + j * kEnsThreads + threadIdx.x;
+            if (i < hi) k[j] = kFirst ? order_key(e[i]) : key[i];
+        }
+#pragma unroll
+        for (int j = 0; j < kRadixItems; ++j) {
+            const long long i = i0 + j * kEnsThreads + threadIdx.x;
+            if (i < hi) {
+                if (kFirst) key[i] = k[j];
+                atomicAdd(&cnt[w][(int)((k[j] >> shift) & (kRadix - 1))], 1);
+            }
+        }
+    }
     __syncthreads();
-    if (ok) {
-        int before = 0;
-        for (int u = 0; u < w; ++u) before += wcnt[u][dg];
-        const long long dst = (long long)offs[(long long)dg * gridDim.x + blockIdx.x] + before + rank;
-        kout[dst] = k;
-        vout[dst] = vin[i];
+    int s = 0;
+#pragma unroll
+    for (int u = 0; u < kEnsThreads / 32; ++u) s += cnt[u][threadIdx.x];
+    hist[blockIdx.x * kRadix + threadIdx.x] = s;
+}
+
+// Scatters each block's keys and values to their places, stable: a tile's elements in the order warp,
+// item, lane, which is their order in the tile. vin null: the values are the indices.
+__global__ void __launch_bounds__(kEnsThreads)
+radix_scatter_kernel(const unsigned long long* __restrict__ kin, const int* __restrict__ vin, unsigned long long* __restrict__ kout,
+                     int* __restrict__ vout, long long n, long long per, int shift, const int* __restrict__ hist) {
+    __shared__ int wcnt[kEnsThreads / 32][kRadix + 1];      // (digit kRadix: past the end)
+    __shared__ int wsum[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // where the block's first key of each digit goes
+    int all = 0, before = 0;
+#pragma unroll 8
+    for (int b = 0; b < (int)gridDim.x; ++b) {
+        const int c = hist[b * kRadix + threadIdx.x];
+        all += c;
+        before += b < (int)blockIdx.x ? c : 0;
+    }
+    int total;
+    int off = block_excl_scan(all, wsum, &total) + before;      // of digit threadIdx.x
+    const long long lo = (long long)blockIdx.x * per, hi = lo + per < n ? lo + per : n;
+    for (long long i0 = lo; i0 < hi; i0 += kRadixTile) {
+        const long long first = i0 + w * 32 * kRadixItems + lane;
+        unsigned long long k[kRadixItems];
+        int v[kRadixItems], rank[kRadixItems];
+#pragma unroll
+        for (int j = 0; j < kRadixItems; ++j) {
+            const long long i = first + 32 * j;
+            k[j] = i < hi ? kin[i] : 0ull;
+            v[j] = i < hi ? (vin ? vin[i] : (int)i) : 0;
+        }
+        for (int d = lane; d <= kRadix; d += 32) wcnt[w][d] = 0;
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < kRadixItems; ++j) {
+            const int dg = first + 32 * j < hi ? (int)((k[j] >> shift) & (kRadix - 1)) : kRadix;
+            const unsigned peers = __match_any_sync(0xffffffffu, dg);
+            const int base = wcnt[w][dg], under = __popc(peers & lanemask_lt());
+            rank[j] = base + under;
+            __syncwarp();
+            if (under == 0) wcnt[w][dg] = base + __popc(peers);
+            __syncwarp();
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < kEnsThreads / 32; ++u) {
+            const int c = wcnt[u][threadIdx.x];
+            wcnt[u][threadIdx.x] = off;
+            off += c;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kRadixItems; ++j) {
+            if (first + 32 * j >= hi) continue;
+            const long long dst = (long long)wcnt[w][(int)((k[j] >> shift) & (kRadix - 1))] + rank[j];
+            kout[dst] = k[j];
+            vout[dst] = v[j];
+        }
+        __syncthreads();
     }
 }
 
@@ -158,19 +230,17 @@ __device__ __forceinline__ bool within_tol(const double* __restrict__ a, const d
     return true;
 }
 
-// head[p] = 1 where sorted chromosome p differs from p - 1 in some decoded gene.
+// x / ng for a flat index x of [n][ng] (in 32 bits where they suffice).
+__device__ __forceinline__ long long row_of(long long x, int ng, bool small) {
+    return small ? (long long)((unsigned)x / (unsigned)ng) : x / ng;
+}
+
+// head[p] (zeroed before) = 1 where sorted chromosome p differs from p - 1 in some decoded gene.
 __global__ void ens_heads_kernel(const double* __restrict__ ic, long long n, int ng, int* __restrict__ head) {
-    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
-        int h = 1;
-        if (p > 0) {
-            h = 0;
-            const double* a = ic + p * ng;
-            const double* b = a - ng;
-            for (int q = 0; q < ng; ++q)
-                if (a[q] != b[q]) { h = 1; break; }
-        }
-        head[p] = h;
-    }
+    const long long total = n * ng;
+    const bool small = total <= 0xffffffffll;
+    for (long long x = blockIdx.x * (long long)blockDim.x + threadIdx.x; x < total; x += (long long)gridDim.x * blockDim.x)
+        if (x < ng || ic[x] != ic[x - ng]) head[row_of(x, ng, small)] = 1;
 }
 
 // H[t]: the sorted position of head t.
@@ -219,42 +289,111 @@ __global__ void ens_next_far_kernel(const double* __restrict__ ic, int ng, const
     }
 }
 
-__global__ void ens_path_init_kernel(const int* __restrict__ nxt, const int* __restrict__ Mp, int* __restrict__ jump,
-                                     uint8_t* __restrict__ on) {
+constexpr int kSegment = 8192;         // heads of a segment
+constexpr int kSegThreads = 1024;
+constexpr int kSegItems = kSegment / kSegThreads;
+constexpr size_t kSegSmem = sizeof(int) * kSegment + kSegment;
+
+// out[t]: the first head past t's segment on the path from t (M: none), by pointer jumping inside the
+// segment, at most log2(kSegment) rounds.
+__global__ void __launch_bounds__(kSegThreads)
+ens_exits_kernel(const int* __restrict__ nxt, const int* __restrict__ Mp, int* __restrict__ out) {
+    extern __shared__ int jump[];
     const int M = *Mp;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < M; t += gridDim.x * blockDim.x) {
-        jump[t] = nxt[t];
-        on[t] = t == 0;
+    const long long base = (long long)blockIdx.x * kSegment;
+    if (base >= M) return;
+    const long long end = base + kSegment < M ? base + kSegment : M;
+    int j[kSegItems];
+#pragma unroll
+    for (int k = 0; k < kSegItems; ++k) {
+        const long long t = base + k * kSegThreads + threadIdx.x;
+        j[k] = t < end ? nxt[t] : M;
+        jump[k * kSegThreads + threadIdx.x] = j[k];
+    }
+    __syncthreads();
+    for (;;) {
+        bool more = false;
+#pragma unroll
+        for (int k = 0; k < kSegItems; ++k)
+            if (j[k] < end) {
+                j[k] = jump[j[k] - base];
+                more = true;
+            }
+        if (!__syncthreads_or(more)) break;
+#pragma unroll
+        for (int k = 0; k < kSegItems; ++k) jump[k * kSegThreads + threadIdx.x] = j[k];
+        __syncthreads();
+    }
+#pragma unroll
+    for (int k = 0; k < kSegItems; ++k) {
+        const long long t = base + k * kSegThreads + threadIdx.x;
+        if (t < end) out[t] = j[k];
     }
 }
 
-// One pointer-jumping round: every marked head marks the head 2^r steps along the chain.
-__global__ void ens_path_round_kernel(const int* __restrict__ jin, int* __restrict__ jout, const uint8_t* __restrict__ oin,
-                                      uint8_t* __restrict__ oout, const int* __restrict__ Mp) {
+// flag[t] = 1 for the heads on the path from head 0, 0 for the others and for t from M to n: each block
+// follows the exits to its segment, then marks by pointer jumping inside (every marked head marks the
+// head 2^r steps along).
+__global__ void __launch_bounds__(kSegThreads)
+ens_mark_kernel(const int* __restrict__ nxt, const int* __restrict__ exits, const int* __restrict__ Mp, long long n,
+                int* __restrict__ flag) {
+    extern __shared__ int jump[];
+    volatile uint8_t* on = reinterpret_cast<uint8_t*>(jump + kSegment);
+    __shared__ int entry;
     const int M = *Mp;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < M; t += gridDim.x * blockDim.x) {
-        const int j = jin[t];
-        if (oin[t]) {
-            oout[t] = 1;
-            if (j < M) oout[j] = 1;
+    const long long base = (long long)blockIdx.x * kSegment;
+    const long long end = base + kSegment < M ? base + kSegment : M;
+    if (base < M) {
+        if (threadIdx.x == 0) {
+            int t = 0;
+            while (t < base) t = exits[t];
+            entry = t;
         }
-        jout[t] = j < M ? jin[j] : M;
+        int j[kSegItems];
+#pragma unroll
+        for (int k = 0; k < kSegItems; ++k) {
+            const int at = k * kSegThreads + threadIdx.x;
+            j[k] = base + at < end ? nxt[base + at] : M;
+            jump[at] = j[k];
+            on[at] = 0;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0 && entry < end) on[entry - base] = 1;
+        __syncthreads();
+        for (;;) {
+            bool more = false;
+            uint8_t mark = 0;
+#pragma unroll
+            for (int k = 0; k < kSegItems; ++k)
+                if (on[k * kSegThreads + threadIdx.x]) mark |= 1u << k;
+            __syncthreads();       // (a round marks from the heads marked before it)
+#pragma unroll
+            for (int k = 0; k < kSegItems; ++k)
+                if (j[k] < end) {
+                    if (mark >> k & 1) on[j[k] - base] = 1;
+                    j[k] = jump[j[k] - base];
+                    more = true;
+                }
+            if (!__syncthreads_or(more)) break;
+#pragma unroll
+            for (int k = 0; k < kSegItems; ++k) jump[k * kSegThreads + threadIdx.x] = j[k];
+            __syncthreads();
+        }
     }
-}
-
-// kept[t] = 1 for the kept heads (as ints, for the scan), 0 past M.
-__global__ void ens_kept_flags_kernel(const uint8_t* __restrict__ on, const int* __restrict__ Mp, long long n, int* __restrict__ flag) {
-    const int M = *Mp;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
-        flag[t] = t < M ? (int)on[t] : 0;
+#pragma unroll
+    for (int k = 0; k < kSegItems; ++k) {
+        const int at = k * kSegThreads + threadIdx.x;
+        if (base + at < n) flag[base + at] = base + at < end ? (int)on[at] : 0;
+    }
 }
 
 // Sorted ICs from ICs given in input order.
 __global__ void ens_gather_ic_kernel(const double* __restrict__ ic_in, const int* __restrict__ order, long long n, int ng,
                                      double* __restrict__ ic_out) {
     const long long total = n * ng;
+    const bool small = total <= 0xffffffffll;
     for (long long x = blockIdx.x * (long long)blockDim.x + threadIdx.x; x < total; x += (long long)gridDim.x * blockDim.x) {
-        const long long p = x / ng;
+        const long long p = row_of(x, ng, small);
         const int q = (int)(x - p * ng);
         ic_out[x] = ic_in[(long long)order[p] * ng + q];
     }
@@ -265,8 +404,9 @@ __global__ void ens_decode_kernel(DevSystem S, const int32_t* __restrict__ genes
                                   double* __restrict__ ic_out) {
     const int ng = S.n_genes;
     const long long total = n * ng;
+    const bool small = total <= 0xffffffffll;
     for (long long x = blockIdx.x * (long long)blockDim.x + threadIdx.x; x < total; x += (long long)gridDim.x * blockDim.x) {
-        const long long p = x / ng;
+        const long long p = row_of(x, ng, small);
         const int q = (int)(x - p * ng);
         double v = S.gene_min[q] + S.gene_del[q] * (double)gene_bin(S, q, genes[(long long)order[p] * ng + q]);
         if (v > S.gene_max[q]) v = S.gene_max[q];
@@ -307,7 +447,6 @@ struct EnsScratch {
     unsigned long long *k0, *k1;
     int *v0, *v1, *hist, *stmp, *head;
     double* ics;
-    uint8_t* oa;
     int* cnt;
     size_t bytes = 0;
 
@@ -318,18 +457,15 @@ struct EnsScratch {
         return q;
     }
     void carve(unsigned char* base, long long n, int ng) {
-        const long long nb = (n + kEnsThreads - 1) / kEnsThreads;
-        const long long st_n = 16 * nb > n + 1 ? 16 * nb : n + 1;
         bytes = 0;
         k0 = take<unsigned long long>(base, n);
         k1 = take<unsigned long long>(base, n);
         v0 = take<int>(base, n);
         v1 = take<int>(base, n);
-        hist = take<int>(base, 32 * nb + 1);          // digit counts [16 nb], their scan [16 nb + 1]
-        stmp = take<int>(base, scan_tmp_ints(st_n));
+        hist = take<int>(base, (size_t)kRadix * radix_blocks(n));
+        stmp = take<int>(base, scan_tmp_ints(n + 1));
         ics = take<double>(base, (size_t)n * ng);
-        head = take<int>(base, 6 * (n + 1));           // head flags, positions, H, next, two jump arrays
-        oa = take<uint8_t>(base, 2 * (size_t)n);       // two mark arrays
+        head = take<int>(base, 5 * (n + 1));           // head flags, positions, H, next, exits (far list)
         cnt = take<int>(base, 4);                      // M, far count
     }
 };
@@ -348,58 +484,49 @@ cudaError_t launch_ensemble(long long n, int ng, const double* e_in, const doubl
                             const int32_t* genes, void* scratch, long long* idx_out, double* e_out, double* ic_out,
                             int* d_kept, cudaStream_t st) {
     if (n <= 0) return cudaMemsetAsync(d_kept, 0, sizeof(int), st);
-    const long long nb = (n + kEnsThreads - 1) / kEnsThreads;
     EnsScratch sc;
     sc.carve(static_cast<unsigned char*>(scratch), n, ng);
     unsigned long long *k0 = sc.k0, *k1 = sc.k1;
     int *v0 = sc.v0, *v1 = sc.v1;
     int* hist = sc.hist;
-    int* hoff = hist + 16 * nb;
     int* stmp = sc.stmp;
     double* ics = sc.ics;
     int* head = sc.head;
     int* hpos = head + (n + 1);
     int* H = hpos + (n + 1);
     int* nxt = H + (n + 1);
-    int* ja = nxt + (n + 1);
-    int* jb = ja + (n + 1);
-    uint8_t* oa = sc.oa;
-    uint8_t* ob = oa + n;
+    int* exits = nxt + (n + 1);
     int* cnt = sc.cnt;                                       // [0] M, [1] far count
     int* kept_flag = head;                                   // reused once the heads are compacted
     int* kept_pos = hpos;
 
-    ens_keys_kernel<<<grid_for(n, kEnsThreads), kEnsThreads, 0, st>>>(e_in, n, k0, v0);
-    for (int pass = 0; pass < 16; ++pass) {
-        const int shift = 4 * pass;
-        radix_hist_kernel<<<(unsigned)nb, kEnsThreads, 0, st>>>(k0, n, shift, hist);
-        scan_ints(hist, hoff, 16 * nb, stmp, st);
-        radix_scatter_kernel<<<(unsigned)nb, kEnsThreads, 0, st>>>(k0, v0, k1, v1, n, shift, hoff);
+    const int nb = radix_blocks(n);
+    const long long per = radix_tiles_per_block(n) * kRadixTile;
+    for (int pass = 0; pass < 8; ++pass) {
+        const int shift = 8 * pass;
+        if (pass == 0) radix_count_kernel<true><<<nb, kEnsThreads, 0, st>>>(e_in, k0, n, per, shift, hist);
+        else radix_count_kernel<false><<<nb, kEnsThreads, 0, st>>>(nullptr, k0, n, per, shift, hist);
+        radix_scatter_kernel<<<nb, kEnsThreads, 0, st>>>(k0, pass == 0 ? nullptr : v0, k1, v1, n, per, shift, hist);
         unsigned long long* tk = k0; k0 = k1; k1 = tk;
         int* tv = v0; v0 = v1; v1 = tv;
     }
     // v0: input index at each sorted position
     if (ic_in) ens_gather_ic_kernel<<<grid_for(n * ng, kEnsThreads), kEnsThreads, 0, st>>>(ic_in, v0, n, ng, ics);
     else ens_decode_kernel<<<grid_for(n * ng, kEnsThreads), kEnsThreads, 0, st>>>(*S, genes, v0, n, ics);
-    ens_heads_kernel<<<grid_for(n, kEnsThreads), kEnsThreads, 0, st>>>(ics, n, ng, head);
+    cudaError_t e = cudaMemsetAsync(head, 0, sizeof(int) * (size_t)n, st);
+    if (e != cudaSuccess) return e;
+    ens_heads_kernel<<<grid_for(n * ng, kEnsThreads), kEnsThreads, 0, st>>>(ics, n, ng, head);
     scan_ints(head, hpos, n, stmp, st);
     ens_compact_kernel<<<grid_for(n, kEnsThreads), kEnsThreads, 0, st>>>(head, hpos, n, H);
-    cudaError_t e = cudaMemcpyAsync(cnt, hpos + n, sizeof(int), cudaMemcpyDeviceToDevice, st);
+    e = cudaMemcpyAsync(cnt, hpos + n, sizeof(int), cudaMemcpyDeviceToDevice, st);
     if (e != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(cnt + 1, 0, sizeof(int), st)) != cudaSuccess) return e;
     // heads: at most n; the kernels read M from the device
-    ens_next_kernel<<<grid_for(n, kEnsThreads), kEnsThreads, 0, st>>>(ics, ng, H, cnt, nxt, ja, cnt + 1);
-    ens_next_far_kernel<<<grid_for(n * 32, kEnsThreads), kEnsThreads, 0, st>>>(ics, ng, H, cnt, nxt, ja, cnt + 1);
-    ens_path_init_kernel<<<grid_for(n, kEnsThreads), kEnsThreads, 0, st>>>(nxt, cnt, ja, oa);
-    int rounds = 0;
-    while ((1ll << rounds) < n) ++rounds;
-    for (int r = 0; r < rounds; ++r) {
-        if ((e = cudaMemsetAsync(ob, 0, (size_t)n, st)) != cudaSuccess) return e;
-        ens_path_round_kernel<<<grid_for(n, kEnsThreads), kEnsThreads, 0, st>>>(ja, jb, oa, ob, cnt);
-        int* tj = ja; ja = jb; jb = tj;
-        uint8_t* to = oa; oa = ob; ob = to;
-    }
-    ens_kept_flags_kernel<<<grid_for(n, kEnsThreads), kEnsThreads, 0, st>>>(oa, cnt, n, kept_flag);
+    ens_next_kernel<<<grid_for(n, kEnsThreads), kEnsThreads, 0, st>>>(ics, ng, H, cnt, nxt, exits, cnt + 1);
+    ens_next_far_kernel<<<grid_for(n * 32, kEnsThreads), kEnsThreads, 0, st>>>(ics, ng, H, cnt, nxt, exits, cnt + 1);
+    const unsigned segments = (unsigned)((n + kSegment - 1) / kSegment);
+    ens_exits_kernel<<<segments, kSegThreads, kSegSmem, st>>>(nxt, cnt, exits);
+    ens_mark_kernel<<<segments, kSegThreads, kSegSmem, st>>>(nxt, exits, cnt, n, kept_flag);
     scan_ints(kept_flag, kept_pos, n, stmp, st);
     ens_emit_kernel<<<grid_for(n, kEnsThreads), kEnsThreads, 0, st>>>(H, kept_flag, kept_pos, cnt, v0, e_in, ics, ng, idx_out,
                                                                       e_out, ic_out);
