@@ -178,7 +178,6 @@ struct Vor {
         uint8_t elist[kMaxEdges + 8];      // before the faces: the hull edges with an end outside the sphere
     };
     uint8_t cslot[kMaxCand];           // the contact's slot in the atom's candidate list
-    uint8_t cmob[kMaxCand];            // the contact's mobile index (kNone: a rigid atom)
     uint8_t fnp[kMaxCand];
     uint8_t fseed[kMaxCand];           // the face's first vertex of three contact planes (kNone: none)
     uint8_t flag[kMaxPlanes];
@@ -1467,7 +1466,8 @@ template <int kSize>
 struct Group {
     static constexpr int size = kSize;
     int slot, barrier;
-    int4* step;              // per pose: triangle items, arc items, whether the pose goes on
+    int4* step;              // per pose: triangle items, arc items, whether the pose goes on, and an atom
+    int2* saved;             // saved in the step before whose terms are to be summed (-1: none); its pose, job
     int* n_retry;            // poses to score again in the large shape
     int* retry;              // [2 * size]
 };
@@ -1477,38 +1477,6 @@ template <int kSize>
 __device__ __forceinline__ void group_sync(const Group<kSize>& g) {
     __syncwarp();
     asm volatile("bar.sync %0, %1;" ::"r"(g.barrier), "n"(kSize * 32) : "memory");
-}
-
-// The group's area items, pooled: every pose's triangles as one list, then every pose's arcs as
-// another, 32 at a time to the group's warps. Group barriers around it keep the items' owners out.
-template <class Sh, int kSize>
-__device__ __forceinline__ void pooled_areas(PoseShared<Sh>* all, const Group<kSize>& g, int lane) {
-    static_assert(kWarps <= 32, "one lane per pose in the prefix sums");
-    const int4 n = lane < g.size ? g.step[lane] : make_int4(0, 0, 0, 0);
-    int T, A;
-    const int tpre = warp_excl_scan(n.x, lane, &T), apre = warp_excl_scan(n.y, lane, &A);
-    const int tch = (T + 31) >> 5, ach = (A + 31) >> 5;
-    #pragma unroll 1
-    for (int ch = g.slot; ch < tch + ach; ch += g.size) {
-        const bool tri = ch < tch;
-        const int k = (tri ? ch : ch - tch) * 32 + lane, pre = tri ? tpre : apre;
-        // the pose of item k: the last one whose first item is at or before it (a pose without
-        // items shares its successor's first item)
-        int w = 0;
-        #pragma unroll 1
-        for (int q = 1; q < Sh::poses; ++q)
-            if (__shfl_sync(kFull, pre, q) <= k) w = q;
-        const int first = __shfl_sync(kFull, pre, w);
-        if (k < (tri ? T : A)) {
-            Vor<Sh>& q = all[w].v;
-            const int i = k - first + (tri ? 0 : q.nt);
-            const uint32_t it = q.u.f.item[i];
-            double v;
-            if (tri) v = fan_triangle(q.vx[it & 0xffu], q.vx[(it >> 8) & 0xffu], q.vx[it >> 16], q.rado);
-            else v = sph_arc(centre_of(q.pl[it & 0xffu]), q.vx[(it >> 8) & 0xffu], q.vx[(it >> 16) & 0xffu], q.rado);
-            q.u.f.val[i] = v;
-        }
-    }
 }
 
 // The area of face X from its items' values, the sum in the reference's order (triangles, then
@@ -1576,7 +1544,6 @@ __device__ __forceinline__ int load_planes(Vor<Sh>& sh, const DevSystem& S, cons
             sh.cidx[r] = j;
             sh.cslot[r] = (uint8_t)c;
             const int mj = mobile_of(S, j);
-            sh.cmob[r] = (uint8_t)mj;      // (-1: kNone)
             const float4 pj = mj < 0 ? S.rec_pos[j] : W.mob_pos[(size_t)p * nm + mj];
             const double d = dsqrt(f2d(d2));
             const float q = kRw + pj.w;
@@ -1903,7 +1870,7 @@ __device__ __forceinline__ int step_pose(const Jobs& jobs, Pose& q, int lane, Po
 
 // Saves the atom whose areas are in: save_areas (LIB/Vcontacts.cpp:1149-1220: contacts with area > 0 on
 // a contact plane; candidates outside the contact list record nothing), save_seeds (:601-629: the first
-// vertex naming a later atom's plane), and its terms.
+// vertex naming a later atom's plane).
 template <class Sh, class Jobs>
 __device__ __forceinline__ void save_atom(const Jobs& jobs, const Pose& q, int lane, PoseShared<Sh>& ps) {
     const DevSystem& S = jobs.S(q);
@@ -1926,8 +1893,8 @@ __device__ __forceinline__ void save_atom(const Jobs& jobs, const Pose& q, int l
         const int c = sh.cslot[k];
         W.cand_area[cb + c] = ar;
         W.cand_flag[cb + c] = (uint8_t)(f | (keep ? kRecorded : 0));
-        const int m = sh.cmob[k];
-        if (m != kNone) {
+        const int m = mobile_of(S, sh.cidx[k]);
+        if (m >= 0) {
             if (keep) W.pose_rec[((size_t)q.p * kMaxLig + m) * kMaskWords + (q.a >> 5)] |= 1u << (q.a & 31);
             int* seed = W.pose_seed + ((size_t)q.p * kMaxLig + m) * 3;
             const int vi = sh.fseed[k];
@@ -1942,7 +1909,6 @@ __device__ __forceinline__ void save_atom(const Jobs& jobs, const Pose& q, int l
     }
     if (lane == 0) ps.done[q.a >> 5] |= 1u << (q.a & 31);
     __syncwarp();
-    score_atom(S, W, lb, q.a, lane);
 }
 
 // The launch's counters of a finished pose.
@@ -1950,6 +1916,57 @@ __device__ __forceinline__ void count_faces(const DevWork& W, const Pose& q, int
     const int miss = warp_sum(q.miss), lost = warp_sum(q.lost);
     if (lane == 0 && miss) atomicAdd(&W.counters[3], miss);
     if (lane == 0 && lost) atomicAdd(&W.counters[0], lost);
+}
+
+// Whether a saved atom's terms are summed by any of the group's warps in the next step, beside the areas,
+// or by its own warp at once. In the groups of few poses most warps have nothing else to do: one pose of
+// 24 atoms takes 1,283 us so and 1,355 otherwise, 500 poses 1,683 and 1,744. A full group's warps are busy
+// with the areas (2,000 poses: 7.53 ms and 7.37).
+template <int kSize>
+constexpr bool kScoreLater = kSize < kWarps;
+
+// What the group's warps share out in a step: every pose's triangles as one list, 32 at a time, then
+// every pose's arcs, then the atoms saved in the step before whose terms are still to be summed. Group
+// barriers around it keep the items' owners out.
+template <class Sh, int kSize, class Jobs>
+__device__ __forceinline__ void pooled_work(const Jobs& jobs, PoseShared<Sh>* all, const Group<kSize>& g, int lane) {
+    static_assert(kWarps <= 32, "one lane per pose in the prefix sums");
+    const int4 n = lane < g.size ? g.step[lane] : make_int4(0, 0, 0, -1);
+    const unsigned scores = kScoreLater<kSize> ? __ballot_sync(kFull, n.w >= 0) : 0u;
+    int T, A;
+    const int tpre = warp_excl_scan(n.x, lane, &T), apre = warp_excl_scan(n.y, lane, &A);
+    const int tch = (T + 31) >> 5, ach = (A + 31) >> 5;
+    #pragma unroll 1
+    for (int ch = g.slot; ch < tch + ach + __popc(scores); ch += g.size) {
+        if (kScoreLater<kSize> && ch >= tch + ach) {
+            unsigned m = scores;
+            for (int k = ch - tch - ach; k > 0; --k) m &= m - 1;
+            const int slot = __ffs(m) - 1;
+            Pose q;
+            q.p = g.saved[slot].x;
+            q.job = g.saved[slot].y;
+            score_atom(jobs.S(q), jobs.W(q), (size_t)q.p * n_mobile(jobs.S(q)), g.step[slot].w, lane);
+            continue;
+        }
+        const bool tri = ch < tch;
+        const int k = (tri ? ch : ch - tch) * 32 + lane, pre = tri ? tpre : apre;
+        // the pose of item k: the last one whose first item is at or before it (a pose without
+        // items shares its successor's first item)
+        int w = 0;
+        #pragma unroll 1
+        for (int q = 1; q < Sh::poses; ++q)
+            if (__shfl_sync(kFull, pre, q) <= k) w = q;
+        const int first = __shfl_sync(kFull, pre, w);
+        if (k < (tri ? T : A)) {
+            Vor<Sh>& q = all[w].v;
+            const int i = k - first + (tri ? 0 : q.nt);
+            const uint32_t it = q.u.f.item[i];
+            double v;
+            if (tri) v = fan_triangle(q.vx[it & 0xffu], q.vx[(it >> 8) & 0xffu], q.vx[it >> 16], q.rado);
+            else v = sph_arc(centre_of(q.pl[it & 0xffu]), q.vx[(it >> 8) & 0xffu], q.vx[(it >> 16) & 0xffu], q.rado);
+            q.u.f.val[i] = v;
+        }
+    }
 }
 
 // Scores poses group step by group step: in each step every pose of the group takes its next atom (or
@@ -1964,11 +1981,13 @@ __device__ __forceinline__ void score_poses(const Jobs& jobs, int lane, PoseShar
     Pose q;
     q.alive = false;
     bool more = g.slot < poses;          // poses may be left for this warp
+    int to_score = -1;                   // the atom saved in the step before
     #pragma unroll 1
     for (;;) {
         while (!q.alive && more) {
             more = next_pose(q);
             if (more) q.alive = begin_pose(jobs, q, lane, ps, hist);
+            to_score = -1;
         }
         int st = kAtomNone;
         if (q.alive) {
@@ -1989,14 +2008,23 @@ __device__ __forceinline__ void score_poses(const Jobs& jobs, int lane, PoseShar
             }
         }
         const bool pending = q.alive && st == kAtomOk;
-        if (lane == 0) g.step[g.slot] = make_int4(pending ? ps.v.nt : 0, pending ? ps.v.na + ps.v.ne : 0, q.alive || more, 0);
+        if (lane == 0) {
+            g.step[g.slot] = make_int4(pending ? ps.v.nt : 0, pending ? ps.v.na + ps.v.ne : 0, q.alive || more,
+                                       q.alive ? to_score : -1);
+            if (kScoreLater<kSize>) g.saved[g.slot] = make_int2(q.p, q.job);
+        }
+        to_score = -1;
         group_sync(g);
         if (!__any_sync(kFull, lane < g.size && g.step[lane].z != 0)) break;
-        pooled_areas(all, g, lane);
+        pooled_work(jobs, all, g, lane);
         group_sync(g);
         if (pending) {
             save_atom(jobs, q, lane, ps);
             ++q.r;
+            if (kScoreLater<kSize> && q.r < n_mobile(jobs.S(q)))
+                to_score = q.a;
+            else
+                score_atom(jobs.S(q), jobs.W(q), (size_t)q.p * n_mobile(jobs.S(q)), q.a, lane);
         }
         if (q.alive && !q.walking && q.r == n_mobile(jobs.S(q))) {
             __syncwarp();
@@ -2009,7 +2037,7 @@ __device__ __forceinline__ void score_poses(const Jobs& jobs, int lane, PoseShar
 }
 
 constexpr size_t kPoseSmem = sizeof(PoseShared<Compact>) * kWarps;
-static_assert(kPoseSmem + 512 <= 227 * 1024, "sixteen poses per SM");
+static_assert(kPoseSmem + 768 <= 227 * 1024, "sixteen poses per SM");
 static_assert(sizeof(PoseShared<Large>) * Large::poses <= kPoseSmem && sizeof(PoseShared<Large>) <= kPoseSmem / 4,
               "the large shape's poses fit a block, and one fits the smallest group's share");
 
@@ -2024,6 +2052,7 @@ __device__ __forceinline__ void score_queue(const Jobs& jobs, int n, int* next, 
                                             int active) {
     extern __shared__ __align__(32) unsigned char smem[];
     __shared__ int4 step[kWarps];
+    __shared__ int2 saved[kWarps];
     __shared__ int n_retry_of[kWarps], retry[2 * kWarps];
     const int lane = threadIdx.x & 31, warp = (int)(threadIdx.x >> 5);
     constexpr int groups = kWarps / kSize;
@@ -2032,6 +2061,7 @@ __device__ __forceinline__ void score_queue(const Jobs& jobs, int n, int* next, 
     g.slot = (warp + group * (4 / groups)) % kSize;   // (a group's first slots: each in another quarter of the SM)
     g.barrier = group + 1;
     g.step = step + group * kSize;
+    g.saved = saved + group * kSize;
     g.n_retry = n_retry_of + group;
     g.retry = retry + 2 * group * kSize;
     unsigned char* const mem = smem + sizeof(PoseShared<Compact>) * kSize * group;
