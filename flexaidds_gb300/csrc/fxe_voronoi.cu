@@ -55,11 +55,7 @@ __device__ __forceinline__ void warp_argmin(V& v, int& i) {
     }
 }
 
-__device__ __forceinline__ int warp_sum(int v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-    return v;
-}
+__device__ __forceinline__ int warp_sum(int v) { return __reduce_add_sync(kFull, v); }
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -425,7 +421,7 @@ __device__ __forceinline__ int face_of(const uint16_t* off, int NC, int k) {
 // Whether points vi and vi+1 of a face bound an arc segment: both arc points, of different
 // edges (LIB/Vcontacts.cpp:943-954).
 __device__ __forceinline__ int arc_segment(const VorShared& sh, const uint8_t* pt, int np, int vi) {
-    const uchar4 qa = sh.vp[pt[vi]], qb = sh.vp[pt[(vi + 1) % np]];
+    const uchar4 qa = sh.vp[pt[vi]], qb = sh.vp[pt[vi + 1 < np ? vi + 1 : 0]];
     if (qa.z != kNone || qb.z != kNone) return 0;
     const int sa = (qa.y == kNone ? -1 : qa.y) + qa.x;
     const int sb = (qb.y == kNone ? -1 : qb.y) + qb.x;
@@ -885,7 +881,25 @@ __device__ int voronoi_warp(VorShared& sh, int NC, real rado, int lane, int* no_
     const int NV = nv;
 
     // ---- faces: points per plane in vertex order, plus an antipodal arc point ----
-    // (the edge arrays are dead from here on; their storage holds the face lists)
+    // (the edge arrays are dead from here on; their storage holds the face lists, and first a bit mask
+    // of its vertices per plane, NW words each, which the vertices' lanes set: a face counts and lists
+    // its points without looking at every vertex)
+    static_assert(kMaxCand * ((kMaxVerts + 31) / 32) <= kMaxFacePts, "the masks fit the cosines' storage");
+    uint32_t* vmask = reinterpret_cast<uint32_t*>(sh.u.f.cosv);
+    const int NW = (NV + 31) >> 5;
+    #pragma unroll 1
+    for (int k = lane; k < NC * NW; k += 32) vmask[k] = 0u;
+    __syncwarp();
+    #pragma unroll 1
+    for (int vi = lane; vi < NV; vi += 32) {
+        const uchar4 P = sh.vp[vi];
+        uint32_t* m = vmask + (vi >> 5);
+        const uint32_t b = 1u << (vi & 31);
+        if (P.x < NC) atomicOr(m + P.x * NW, b);
+        if (P.y < NC) atomicOr(m + P.y * NW, b);
+        if (P.z < NC) atomicOr(m + P.z * NW, b);
+    }
+    __syncwarp();
     int tot_pts = 0;
     #pragma unroll 1
     for (int x0 = 0; x0 < NC; x0 += 32) {
@@ -893,10 +907,7 @@ __device__ int voronoi_warp(VorShared& sh, int NC, real rado, int lane, int* no_
         int cnt = 0;
         if (X < NC && sh.flag[X] != 0)
             #pragma unroll 1
-            for (int vi = 0; vi < NV; ++vi) {
-                const uchar4 P = sh.vp[vi];
-                cnt += (P.x == X || P.y == X || P.z == X);
-            }
+            for (int w = 0; w < NW; ++w) cnt += __popc(vmask[X * NW + w]);
         const int need = cnt + (cnt > 2 ? 1 : 0);
         int t;
         const int off = warp_excl_scan(need, lane, &t);
@@ -908,35 +919,37 @@ __device__ int voronoi_warp(VorShared& sh, int NC, real rado, int lane, int* no_
     }
     if (tot_pts > kMaxFacePts) return kAtomCapacity;
     __syncwarp();
-    // the faces' point lists and, for a face of more than two points, the antipode of its first
-    // sphere point, which joins the face when it lies behind every other plane (test_point)
+    #pragma unroll 1
+    for (int X = lane; X < NC; X += 32) {
+        if (sh.flag[X] == 0) continue;
+        uint8_t* pt = &sh.u.f.pt[sh.foff[X]];
+        #pragma unroll 1
+        for (int w = 0; w < NW; ++w)
+            #pragma unroll 1
+            for (uint32_t m = vmask[X * NW + w]; m; m &= m - 1) *pt++ = (uint8_t)(w * 32 + __ffs(m) - 1);
+    }
+    __syncwarp();
+    // for a face of more than two points, the antipode of its first sphere point, which joins the face
+    // when it lies behind every other plane (test_point)
     int nf = 0;
     #pragma unroll 1
     for (int x0 = 0; x0 < NC; x0 += 32) {
         const int X = x0 + lane;
         bool cand = false;
-        if (X < NC && sh.flag[X] != 0) {
-            const int o = sh.foff[X];
-            int k = 0;
+        if (X < NC && sh.flag[X] != 0 && sh.fnp[X] > 2) {
+            const int o = sh.foff[X], k = sh.fnp[X];
+            const real4 cp = centre_of(sh.pl[X]);
             #pragma unroll 1
-            for (int vi = 0; vi < NV; ++vi) {
-                const uchar4 P = sh.vp[vi];
-                if (P.x == X || P.y == X || P.z == X) sh.u.f.pt[o + k++] = (uint8_t)vi;
-            }
-            if (k > 2) {
-                const real4 cp = centre_of(sh.pl[X]);
-                #pragma unroll 1
-                for (int q = 0; q < k; ++q) {
-                    const int vi = sh.u.f.pt[o + q];
-                    if (sh.vp[vi].z == kNone) {
-                        const real4 pv = sh.vx[vi];
-                        real* ex = &sh.u.f.cosv[3 * X];
-                        ex[0] = real(2.0) * cp.x - pv.x;
-                        ex[1] = real(2.0) * cp.y - pv.y;
-                        ex[2] = real(2.0) * cp.z - pv.z;
-                        cand = true;
-                        break;
-                    }
+            for (int q = 0; q < k; ++q) {
+                const int vi = sh.u.f.pt[o + q];
+                if (sh.vp[vi].z == kNone) {
+                    const real4 pv = sh.vx[vi];
+                    real* ex = &sh.u.f.cosv[3 * X];
+                    ex[0] = real(2.0) * cp.x - pv.x;
+                    ex[1] = real(2.0) * cp.y - pv.y;
+                    ex[2] = real(2.0) * cp.z - pv.z;
+                    cand = true;
+                    break;
                 }
             }
         }
@@ -1212,7 +1225,7 @@ __device__ int voronoi_warp(VorShared& sh, int NC, real rado, int lane, int* no_
             for (; vi < np - 1; ++vi)
                 if (arc_segment(sh, pt, np, vi) && j-- == 0) break;
             ia = pt[vi];
-            ib = pt[(vi + 1) % np];
+            ib = pt[vi + 1 < np ? vi + 1 : 0];
         } else if (k < a_run + n_lens) {
             F = sh.llist[k - a_run];
             const uint8_t* pt = &sh.u.f.pt[sh.foff[F]];
@@ -1452,25 +1465,23 @@ __device__ __forceinline__ void score_pose(const DevSystem& S, const DevWork& W,
             for (int o = 16; o > 0; o >>= 1) m |= __shfl_xor_sync(kFull, m, o);
             if (lane == 0) rec[a][w] = m;
         }
-        // save_seeds (LIB/Vcontacts.cpp:601-629): first vertex naming each later atom's plane
-        if (lane == 0) {
-            const int az = slot_of(S, a);
+        // save_seeds (LIB/Vcontacts.cpp:601-629): first vertex naming each later atom's plane, found
+        // by the plane's lane (one lane over all vertices was 1,000 of an atom's 11,600 instructions)
+        #pragma unroll 1
+        for (int k = lane; k < NC; k += 32) {
+            const int m = mobile_of(S, sh.cidx[k]);
+            if (m < 0 || seed[m][0] != -1) continue;
             #pragma unroll 1
             for (int vi = 0; vi < sh.nv; ++vi) {
                 const uchar4 q = sh.vp[vi];
-                if (q.z == kNone || q.x >= NC || q.y >= NC || q.z >= NC) continue;
-                const int j0 = sh.cidx[q.x], j1 = sh.cidx[q.y], j2 = sh.cidx[q.z];
-                const int m0 = mobile_of(S, j0), m1 = mobile_of(S, j1), m2 = mobile_of(S, j2);
-                if (m0 >= 0 && seed[m0][0] == -1) {
-                    seed[m0][0] = az; seed[m0][1] = j1; seed[m0][2] = j2;
-                }
-                if (m1 >= 0 && seed[m1][0] == -1) {
-                    seed[m1][0] = az; seed[m1][1] = j0; seed[m1][2] = j2;
-                }
-                if (m2 >= 0 && seed[m2][0] == -1) {
-                    seed[m2][0] = az; seed[m2][1] = j0; seed[m2][2] = j1;
-                }
+                if ((q.x != k && q.y != k && q.z != k) || q.x >= NC || q.y >= NC || q.z >= NC) continue;
+                seed[m][0] = slot_of(S, a);
+                seed[m][1] = sh.cidx[q.x == k ? q.y : q.x];
+                seed[m][2] = sh.cidx[q.z == k ? q.y : q.z];
+                break;
             }
+        }
+        if (lane == 0) {
             ps.done[a >> 5] |= 1u << (a & 31);
         }
         __syncwarp();
@@ -1538,9 +1549,17 @@ __device__ __forceinline__ void score_pose(const DevSystem& S, const DevWork& W,
                 }
             }
         }
-        c_com = warp_sum(c_com);
-        c_wal = warp_sum(c_wal);
-        c_area = warp_sum(c_area);
+        // both sums in one reduction: after the first exchange the lower half holds c_com's partial
+        // sums, the upper half c_area's (the additions are warp_sum's)
+        {
+            const bool up = lane >= 16;
+            double x = (up ? c_area : c_com) + __shfl_xor_sync(kFull, up ? c_com : c_area, 16);
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(kFull, x, o);
+            c_com = __shfl_sync(kFull, x, 0);
+            c_area = __shfl_sync(kFull, x, 16);
+        }
+        if (__any_sync(kFull, c_wal != 0.0)) c_wal = warp_sum(c_wal);
         double SAS = surfA - c_area;
         if (SAS < 0.0) SAS = 0.0;
         if (!side) totsas += SAS;
