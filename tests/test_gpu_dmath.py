@@ -1,0 +1,91 @@
+"""The short double-precision quotient and root of the polyhedron kernel (fxe_dmath.cuh) against the
+correctly rounded operations, over operands of every kind: bit for bit, with nothing to tolerate."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from flexaidds_gb300 import build
+
+pytestmark = pytest.mark.gpu
+
+SOURCE = r"""
+#include "fxe_dmath.cuh"
+__global__ void short_ops(const double* a, const double* b, double* q, double* s, float* t, double* w, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    bool slow;
+    double v = fxe::div_short(a[i], b[i], &slow);
+    q[i] = slow ? fxe::plain_div(a[i], b[i]) : v;
+    v = fxe::sqrt_short(a[i], &slow);
+    s[i] = slow ? fxe::plain_sqrt(a[i]) : v;
+    t[i] = fxe::d2f_trunc(a[i]);
+    w[i] = fxe::f2d((float)b[i]);
+}
+extern "C" int run(const double* a, const double* b, double* q, double* s, float* t, double* w, int n) {
+    double* d = nullptr;
+    const size_t z = sizeof(double) * n;
+    if (cudaMalloc(&d, 6 * z) != cudaSuccess) return 1;
+    cudaMemcpy(d, a, z, cudaMemcpyHostToDevice);
+    cudaMemcpy(d + n, b, z, cudaMemcpyHostToDevice);
+    short_ops<<<(n + 255) / 256, 256>>>(d, d + n, d + 2 * n, d + 3 * n, (float*)(d + 4 * n), d + 5 * n, n);
+    cudaMemcpy(q, d + 2 * n, z, cudaMemcpyDeviceToHost);
+    cudaMemcpy(s, d + 3 * n, z, cudaMemcpyDeviceToHost);
+    cudaMemcpy(t, d + 4 * n, z / 2, cudaMemcpyDeviceToHost);
+    cudaMemcpy(w, d + 5 * n, z, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return cudaGetLastError() != cudaSuccess;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def ops(tmp_path_factory):
+    d = tmp_path_factory.mktemp("dmath")
+    (d / "ops.cu").write_text(SOURCE)
+    subprocess.run([build.nvcc(), *build.ARCH, "-O3", "-std=c++17", "--fmad=false", "-Xcompiler", "-fPIC", "-shared",
+                    "-cudart", "static", "-I", build.CSRC, "-o", str(d / "ops.so"), str(d / "ops.cu")], check=True)
+    lib = C.CDLL(os.path.join(str(d), "ops.so"))
+
+    def run(a, b):
+        q, s, w, t = (np.empty(len(a)) for _ in range(3)), None, None, np.empty(len(a), np.float32)
+        q, s, w = q
+        p = [x.ctypes.data_as(C.c_void_p) for x in (a, b, q, s, t, w)]
+        assert lib.run(*p, C.c_int(len(a))) == 0
+        return q, s, t, w
+    return run
+
+
+def _operands(kind, n, rng):
+    if kind == "ordinary":
+        return rng.normal(0.0, 10.0, n), rng.normal(0.0, 10.0, n)
+    if kind == "wide":         # the edges of the short forms' exponent range
+        e = rng.integers(-360, 361, (2, n))
+        return tuple(np.ldexp(rng.uniform(1.0, 2.0, n) * rng.choice([-1.0, 1.0], n), k) for k in e)
+    if kind == "bits":         # every exponent, denormals, infinities and NaN among them
+        return tuple(rng.integers(0, 1 << 64, n, dtype=np.uint64).view(np.float64) for _ in range(2))
+    if kind == "midway":       # quotients and roots next to the midpoint of two doubles
+        b = rng.integers(1 << 52, 1 << 53, n).astype(np.float64)
+        q = rng.integers(1 << 52, 1 << 53, n).astype(np.float64)
+        a = q * b
+        return np.nextafter(a, np.where(rng.random(n) < 0.5, 0.0, np.inf)), b
+    special = np.array([0.0, -0.0, 1.0, -1.0, np.inf, -np.inf, np.nan, 5e-324, 2.0 ** -1022, 1.7e308,
+                        np.nextafter(2.0, 1.0), np.nextafter(4.0, 1.0), 2.0 ** 350, 2.0 ** -350, 1.0 + 2.0 ** -52])
+    return tuple(np.ascontiguousarray(x.ravel()) for x in np.meshgrid(special, special))
+
+
+@pytest.mark.parametrize("kind", ["ordinary", "wide", "bits", "midway", "special"])
+def test_short_operations_are_correctly_rounded(ops, kind):
+    a, b = _operands(kind, 1 << 20, np.random.default_rng(17))
+    q, s, t, w = ops(a, b)
+    with np.errstate(all="ignore"):
+        for got, want in ((q, a / b), (s, np.sqrt(a)), (w, b.astype(np.float32).astype(np.float64))):
+            same = (got.view(np.uint64) == want.view(np.uint64)) | (np.isnan(got) & np.isnan(want))
+            assert same.all(), (kind, a[~same][:3], b[~same][:3])
+        # truncated toward zero, below the normal range to zero, past the range to infinity
+        f = np.abs(t.astype(np.float64))
+        normal = (np.abs(a) >= 2.0 ** -126) & (np.abs(a) < 2.0 ** 128)
+        assert np.all(f[normal] <= np.abs(a[normal])) and np.all(np.abs(a[normal]) - f[normal] < np.abs(a[normal]) * 2.0 ** -22)
+        assert np.all(t[np.abs(a) < 2.0 ** -126] == 0.0) and np.all(np.isinf(t[np.abs(a) >= 2.0 ** 128]))
