@@ -61,6 +61,8 @@ constexpr int kWalkBudget = 16;
 // `verts` lie in storage the faces use later), in 14.1 KB per pose, so that sixteen poses fit an SM. A
 // pose one of whose atoms outgrows it is scored again, from its start, in the large shape when its
 // group has no other pose.
+// (With 256 items one pose of the benchmark's in 8,000 was: 3.2 ms more for its launch. With 290 none of
+// 130,000.)
 template <int kV, int kX, int kP, int kI, int kN>
 struct Shape {
     static constexpr int verts = kV;         // of the faces; vertex indices are bytes (255 means "none")
@@ -71,7 +73,7 @@ struct Shape {
     static constexpr int vwords = (kV + 31) / 32;
     static constexpr int over = kV >= kMaxVerts ? kAtomCapacity : kAtomRetry;
 };
-using Compact = Shape<104, kMaxVerts, 352, 256, kWarps>;
+using Compact = Shape<104, kMaxVerts, 352, 290, kWarps>;
 using Large = Shape<kMaxVerts, kMaxVerts, kMaxFacePts, 3 * kMaxFacePts + 8, 5>;
 
 struct __align__(32) real4 {
