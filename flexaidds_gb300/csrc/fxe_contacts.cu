@@ -281,7 +281,7 @@ __device__ __forceinline__ void contacts_atom(const DevSystem& S, const DevWork&
         // The rigid candidates come in order (cells in scan order, Calc order within a cell): a
         // candidate's place is the rigid ones before it (its own place, or by binary search) plus the
         // mobile ones before it (all of them compared: a dozen). A bitonic sort of the list took a
-        // third of the kernel's instructions.
+        // third of the kernel's instructions (a GA generation of 2,000: 455 -> 378 us).
         __syncwarp();
         for (int i = lane; i < nc; i += 32) {
             const int key = cs.key[i];

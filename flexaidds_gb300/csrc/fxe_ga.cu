@@ -306,7 +306,7 @@ __device__ __forceinline__ uint32_t crossed(uint32_t own, uint32_t mate, int np)
 // Pair k of the children of generation g + 1, from the generation's counter-based stream, by one
 // warp: breed_pair_with's draws in its order, the genes spread over the lanes (genes lane and
 // lane + 32; ng <= 64) and a gene's 32 mutation draws one per lane. A thread per pair made 1,216 draws
-// one after another on nine SMs (184 us per generation of 2,000); the warps spread over the device.
+// one after another on nine SMs (184 us per generation of 2,000; 32 by warps, which spread over the device).
 // cand: the pair's two chromosomes; sig: their signatures.
 __device__ void breed_pair_warp(const GaJob& J, int g, int k, int lane, int32_t* cand, uint64_t* sig) {
     const int ng = J.ng;
@@ -400,7 +400,7 @@ constexpr int kGaMaxBatches = 16;   // candidate batches before duplicates are l
 // So the block decides all of a batch's candidates at once: the first occurrences by a hash table of
 // (signature, lowest index) in shared memory, the set by read-only probes, the cut by an ordered
 // scan; then it copies the taken ones into place and inserts their signatures. (A bitonic sort of the
-// signatures in the table's place took most of the kernel's 145 us at 2,000 children.) When a batch runs
+// signatures in the table's place took most of the kernel's 145 us at 2,000 children; 41 us so.) When a batch runs
 // out, the block breeds the next batch of pairs. After kGaMaxBatches batches candidates are taken
 // as they come (counted in gen[2]), where the reference would loop until mutation finds new genes.
 // gen[1] sizes the next generation's first batch from what this one used; gen[3] counts rejected
@@ -551,7 +551,8 @@ __global__ void __launch_bounds__(kAcceptThreads) ga_accept_kernel(const GaJob* 
 // set is ordered by energy (equal energies by place, parents first), the best P kept, saved as the
 // generation's snapshot, and the generation counter advanced. The parents are in order already: the
 // children are sorted, and every entry's place in the merged order is its own place plus the entries
-// of the other list before it, found by binary search.
+// of the other list before it, found by binary search (2,000 and 2,000: 52 us; 82 when all 4,000 were
+// sorted).
 template <bool kInitial>
 __global__ void __launch_bounds__(kGaSortThreads) ga_select_kernel(GaJob* __restrict__ all, const int* __restrict__ run) {
     extern __shared__ __align__(16) unsigned char sel_smem[];
@@ -632,7 +633,8 @@ __global__ void __launch_bounds__(kGaSortThreads) ga_select_kernel(GaJob* __rest
 }
 
 // ICs of the (new) population, clamped into the gene limits as eval_chromosome leaves them in
-// the genes (LIB/gaboom.cpp:1845-1866), for the niche counts.
+// the genes (LIB/gaboom.cpp:1845-1866), for the niche counts. A block per SM: each value is a chain of
+// look-ups (2,000 chromosomes of 19 genes: 69 us on eight blocks, 12 so).
 __global__ void __launch_bounds__(kGaThreads) ga_decode_kernel(const GaJob* __restrict__ all, const int* __restrict__ run) {
     const GaJob& J = all[run[blockIdx.y]];
     if (J.fitness == kFitLinear) return;
@@ -657,7 +659,7 @@ constexpr int kNicheBlocks = (kGaMaxPop + kNicheRows - 1) / kNicheRows;
 // every pair's distance is formed in single precision with a bound on its error, the pairs not
 // surely beyond sig_share are listed and evaluated in double by full warps, and each row's terms
 // are added in j order, the block's eight rows on eight lanes. The FP64 unit (2 lanes per clock and
-// SM) bounded the form that evaluated every pair in double: 0.87 ms per generation at P = 2,000.
+// SM) bounded the form that evaluated every pair in double: 0.87 ms per generation at P = 2,000, 0.11 so.
 //
 // Bound: with coordinates truncated to float (2^-23 of them) the distance's square root moves by at
 // most 2^-23 (|x_i| + |x_j|) and its rounding by 2^-21 of it, so a pair whose float distance is above

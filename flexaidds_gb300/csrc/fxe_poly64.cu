@@ -51,7 +51,7 @@ constexpr int kAtomRetry = 3;    // the atom outgrew this shape's capacities: sc
 // Warps of a block, one block per SM, in groups that step through their poses' atoms together.
 constexpr int kWarps = 16;
 // Batches of edges a hull walk may step before its warp meets its group (it goes on in the group's
-// next step): a walk takes 5.4 on average, forty when it fails. 2,000 poses of the benchmark's system
+// next step): a walk takes 5.4 on average, many more when it fails. 2,000 poses of the benchmark's system
 // take 7.77 ms with 8, 7.59 with 10, 7.40 with 12, 7.37 with 16, 7.36 with 20.
 constexpr int kWalkBudget = 16;
 
