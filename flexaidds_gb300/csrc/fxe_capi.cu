@@ -73,9 +73,6 @@ fxe_status cuda_fail(cudaError_t e, const char* what) {
                 std::string(what) + ": " + cudaGetErrorString(e));
 }
 
-// Entries of a pose order over at most n poses (the poses, then each segment's count of scored ones).
-size_t order_ints(size_t n) { return n + n / fxe::kOrderSeg + 1; }
-
 // Device buffers of one call, freed when the call returns.
 struct CallBuffers {
     std::vector<void*> p;
@@ -682,7 +679,7 @@ fxe_status context_create(const fxe_receptor_desc* rec, const fxe_context* share
         FXE_TRY(ctx->alloc(&W.counters, 8), "workspace");   // [4]: the pose queue of pose_kernel
         FXE_TRY(ctx->alloc(&W.pose_cost, P), "workspace");
         FXE_TRY(ctx->alloc(&W.pose_clash, P), "workspace");
-        FXE_TRY(ctx->alloc(&W.pose_order, order_ints(P)), "workspace");
+        FXE_TRY(ctx->alloc(&W.pose_order, P), "workspace");
         FXE_TRY(ctx->alloc(&ctx->d_genes, P * (ng > 0 ? ng : 1)), "staging");
         FXE_TRY(ctx->alloc(&ctx->d_icin, P * (ng > 0 ? ng : 1)), "staging");
         ctx->hist_bytes = fxe::pose_hist_bytes();
@@ -1304,7 +1301,7 @@ extern "C" fxe_status fxe_batch_create(int32_t max_jobs, int64_t max_poses, int3
         FXE_TRY(cudaEventCreateWithFlags(&b->staged, cudaEventDisableTiming), "cudaEventCreate");
         FXE_TRY(cudaMalloc(&b->d_jobs, sizeof(fxe::Job) * max_jobs), "batch job table");
         FXE_TRY(cudaMalloc(&b->d_next, sizeof(int)), "batch pose queue");
-        FXE_TRY(cudaMalloc(&b->d_order, sizeof(int) * order_ints(max_poses)), "batch pose queue");
+        FXE_TRY(cudaMalloc(&b->d_order, sizeof(int) * max_poses), "batch pose queue");
         FXE_TRY(fxe::f32::configure_voronoi(), "cudaFuncSetAttribute");
         FXE_TRY(fxe::f64::configure_voronoi(), "cudaFuncSetAttribute");
         b->hist_bytes = fxe::pose_hist_bytes();
@@ -1753,7 +1750,7 @@ extern "C" fxe_status fxe_ga_step(fxe_ga* e) {
             if (e->d_order) cudaFree(e->d_order);
             e->d_order = nullptr;
             e->order_cap = 0;
-            FXE_TRY(cudaMalloc(&e->d_order, sizeof(int) * order_ints(total)), "GA pose order");
+            FXE_TRY(cudaMalloc(&e->d_order, sizeof(int) * total), "GA pose order");
             e->order_cap = total;
         }
         FXE_TRY(cudaMemcpyAsync(e->d_run, e->run.data(), sizeof(int) * n, cudaMemcpyHostToDevice, e->stream), "GA table");

@@ -29,7 +29,6 @@ constexpr float kPolyPenalty = 1e6f;     // LIB/flexaid.h:69
 // reported with FXE_POSE_CAPACITY rather than scored.
 constexpr int kMaxCand = 96;    // contact candidates of one atom
 constexpr int kMaxPlanes = kMaxCand + 4;
-constexpr int kOrderSeg = 4096;   // poses an order kernel's block sorts
 constexpr int kMaxEdges = 200;  // the reference aborts the hull walk at 200 edges
 // vertex indices are bytes (255 means "none"); a walk that reaches the reference's 200-edge abort
 // has at most about 135 vertices, a complete one with its arc points about 105

@@ -382,7 +382,8 @@ contacts_kernel_jobs(const Job* __restrict__ jobs, int n_jobs, long long total) 
 // hull walk's plane tests grow with), so that the slowest poses start early and the launch does
 // not end on one of them while the SMs run dry; then the poses that need no polyhedra (the clash
 // pre-filter rejects them, or they left the grid). Sorted in segments of kOrderSeg poses, one block
-// each; each segment's count of scored poses follows the n entries. The order changes no result.
+// each. The order changes no result.
+constexpr int kOrderSeg = 4096;
 
 // The sort key of pose p: the complement of its atoms and cost, the top bit set for a pose the
 // polyhedron launch rejects at once.
@@ -395,16 +396,6 @@ __device__ __forceinline__ uint64_t pose_order_key(const DevWork& W, int nm, int
     return ~kRejected & ~(((uint64_t)nm << 40) | (uint64_t)(unsigned)W.pose_cost[p]);
 }
 
-// The sorted segment's entries, and its scored poses (those before the first rejected one).
-__device__ __forceinline__ void write_order(const uint64_t* key, const int* idx, int base, int m, int n, int* __restrict__ order) {
-    for (int i = threadIdx.x; i < m; i += blockDim.x) {
-        order[base + i] = base + idx[i];
-        const bool scored = key[i] != kRejected;
-        if (scored && (i + 1 == m || key[i + 1] == kRejected)) order[n + blockIdx.x] = i + 1;
-        if (i == 0 && !scored) order[n + blockIdx.x] = 0;
-    }
-}
-
 __global__ void __launch_bounds__(kSortThreads) order_poses_kernel(DevWork W, int nm, int n, int* __restrict__ order) {
     __shared__ uint64_t key[kOrderSeg];
     __shared__ int idx[kOrderSeg];
@@ -415,7 +406,7 @@ __global__ void __launch_bounds__(kSortThreads) order_poses_kernel(DevWork W, in
         idx[i] = i;
     }
     block_sort(key, idx, m);
-    write_order(key, idx, base, m, n, order);
+    for (int i = threadIdx.x; i < m; i += blockDim.x) order[base + i] = base + idx[i];
 }
 
 // The same over the poses of several jobs (global pose index gp of the launch).
@@ -432,7 +423,7 @@ __global__ void __launch_bounds__(kSortThreads) order_poses_jobs_kernel(const Jo
         idx[i] = i;
     }
     block_sort(key, idx, m);
-    write_order(key, idx, base, m, n, order);
+    for (int i = threadIdx.x; i < m; i += blockDim.x) order[base + i] = base + idx[i];
 }
 
 void launch_order_poses_jobs(const Job* jobs, int n_jobs, int total, int* order, cudaStream_t st) {

@@ -2109,34 +2109,17 @@ __device__ __forceinline__ void score_queue(const Jobs& jobs, int n, int* next, 
     }
 }
 
-// Scored poses per block up to which two groups of eight warps share it, so that a pose waits for fewer
-// others; with the block full their code no longer meets in the instruction cache (2,000 poses, 13 per
-// block: 8.7 ms against 7.8; 500, at most four per block: 1,861 us against 1,998; a genetic algorithm's
-// generations of 1,999 of which half are scored, 6 - 7 per block: 51.2 ms against 53.5).
-constexpr int kSplitPoses = 8;
-
-// Whether a launch of both forms is this one's (choose: the scored poses, the first of the order, decide;
-// their counts by segment follow its n entries).
-template <int kSize>
-__device__ __forceinline__ bool chosen(bool choose, int n, const int* __restrict__ order) {
-    if (!choose) return true;
-    long long scored = 0;
-    for (int k = 0; k < (n + kOrderSeg - 1) / kOrderSeg; ++k) scored += order[n + k];
-    return (scored <= (long long)kSplitPoses * gridDim.x) == (kSize < kWarps);
-}
-
 template <int kSize>
 __global__ void __launch_bounds__(kWarps * 32)
-pose_kernel(const __grid_constant__ DevSystem S, const __grid_constant__ DevWork W, int n, int* next, uint8_t* hist_all, int active,
-            bool choose) {
-    if (chosen<kSize>(choose, n, W.pose_order)) score_queue<kSize>(OneJob{S, W}, n, next, W.pose_order, hist_all, active);
+pose_kernel(const __grid_constant__ DevSystem S, const __grid_constant__ DevWork W, int n, int* next, uint8_t* hist_all, int active) {
+    score_queue<kSize>(OneJob{S, W}, n, next, W.pose_order, hist_all, active);
 }
 
 template <int kSize>
 __global__ void __launch_bounds__(kWarps * 32)
 pose_kernel_jobs(const Job* __restrict__ jobs, int n_jobs, int n, int* next, const int* __restrict__ order, uint8_t* hist_all,
-                 int active, bool choose) {
-    if (chosen<kSize>(choose, n, order)) score_queue<kSize>(ManyJobs{jobs, n_jobs}, n, next, order, hist_all, active);
+                 int active) {
+    score_queue<kSize>(ManyJobs{jobs, n_jobs}, n, next, order, hist_all, active);
 }
 
 static int g_sms = 0, g_per_sm = 0;   // SMs, and blocks of pose_kernel one SM holds
@@ -2155,15 +2138,21 @@ static int max_blocks(size_t hist_bytes, int blocks_per_sm) {
     return b > 0 ? b : 1;
 }
 
-// A launch's blocks, and the warps of a block that take poses: all of them, or fewer when the launch's
-// poses would not reach every block the device runs at once, so that they spread over more SMs (a pose's
-// time is its chain of atoms, shorter with fewer warps sharing the SM's double-precision unit). A launch
-// that could fill its blocks past kSplitPoses is queued in both forms, of which one returns at once (13 us;
-// the pair counts as one launch): how many of its poses are scored is known on the device only.
-static void launch_shape(int n, size_t hist_bytes, int blocks_per_sm, int* blocks, int* per_block) {
+// A launch's blocks, its groups' size, and the warps of each group that take poses: all of them, or
+// fewer when the launch's poses would not reach every block the device runs at once, so that they
+// spread over more SMs (a pose's time is its chain of atoms, shorter with fewer warps sharing the
+// SM's double-precision unit). Up to kSplitPoses poses per block two groups of eight warps share it: a
+// pose waits for fewer others (500 poses of 40 atoms: 1,861 us, one group of sixteen 1,998); with the
+// block full their code no longer meets in the instruction cache (2,000 poses: 8.7 ms against 7.8).
+constexpr int kSplitPoses = 4;
+static void launch_shape(int n, size_t hist_bytes, int blocks_per_sm, int* blocks, int* group, int* active) {
     const int r = max_blocks(hist_bytes, blocks_per_sm);
-    *per_block = std::max(1, std::min((n + r - 1) / r, kWarps));
-    *blocks = std::max(1, std::min((n + *per_block - 1) / *per_block, r));
+    const int t = std::max(1, std::min((n + r - 1) / r, kWarps));
+    *group = t <= kSplitPoses ? kWarps / 2 : kWarps;
+    const int groups = kWarps / *group;
+    *active = (t + groups - 1) / groups;
+    const int per = *active * groups;
+    *blocks = std::max(1, std::min((n + per - 1) / per, r));
 }
 
 int pose_max_blocks_per_sm() { return g_per_sm; }
@@ -2173,25 +2162,21 @@ int pose_max_blocks_per_sm() { return g_per_sm; }
 void launch_poses(const DevSystem& S, const DevWork& W, int n, int* next, uint8_t* hist, size_t hist_bytes,
                   int blocks_per_sm, cudaStream_t st) {
     if (hist_bytes < kWarps * kHistStride) hist = nullptr;
-    int blocks, per_block;
-    launch_shape(n, hist ? hist_bytes : 0, blocks_per_sm, &blocks, &per_block);
+    int blocks, group, active;
+    launch_shape(n, hist ? hist_bytes : 0, blocks_per_sm, &blocks, &group, &active);
     cudaMemsetAsync(next, 0, sizeof(int), st);
-    const bool choose = per_block > kSplitPoses;
-    pose_kernel<kWarps / 2><<<blocks, kWarps * 32, kPoseSmem, st>>>(S, W, n, next, hist, (per_block + 1) / 2, choose);
-    if (choose) pose_kernel<kWarps><<<blocks, kWarps * 32, kPoseSmem, st>>>(S, W, n, next, hist, per_block, choose);
+    auto* kernel = group == kWarps ? pose_kernel<kWarps> : pose_kernel<kWarps / 2>;
+    kernel<<<blocks, kWarps * 32, kPoseSmem, st>>>(S, W, n, next, hist, active);
 }
 
 void launch_poses_jobs(const Job* jobs, int n_jobs, int total, int* next, const int* order, uint8_t* hist,
                        size_t hist_bytes, int blocks_per_sm, cudaStream_t st) {
     if (hist_bytes < kWarps * kHistStride) hist = nullptr;
-    int blocks, per_block;
-    launch_shape(total, hist ? hist_bytes : 0, blocks_per_sm, &blocks, &per_block);
+    int blocks, group, active;
+    launch_shape(total, hist ? hist_bytes : 0, blocks_per_sm, &blocks, &group, &active);
     cudaMemsetAsync(next, 0, sizeof(int), st);
-    const bool choose = per_block > kSplitPoses;
-    pose_kernel_jobs<kWarps / 2><<<blocks, kWarps * 32, kPoseSmem, st>>>(jobs, n_jobs, total, next, order, hist,
-                                                                       (per_block + 1) / 2, choose);
-    if (choose)
-        pose_kernel_jobs<kWarps><<<blocks, kWarps * 32, kPoseSmem, st>>>(jobs, n_jobs, total, next, order, hist, per_block, choose);
+    auto* kernel = group == kWarps ? pose_kernel_jobs<kWarps> : pose_kernel_jobs<kWarps / 2>;
+    kernel<<<blocks, kWarps * 32, kPoseSmem, st>>>(jobs, n_jobs, total, next, order, hist, active);
 }
 
 cudaError_t configure_voronoi() {

@@ -8,7 +8,7 @@ from oracle import port
 
 pytestmark = pytest.mark.gpu
 
-SMS, WARPS, SPLIT = 152, 16, 8
+SMS, WARPS, SPLIT = 152, 16, 4
 
 
 @pytest.fixture(scope="module")
