@@ -40,7 +40,6 @@ struct real3 {
     real x, y, z;
 };
 __device__ __forceinline__ real4 make_real4(real x, real y, real z, real w) { return real4{x, y, z, w}; }
-__device__ __forceinline__ real4 to_real4(const float4& v) { return real4{(real)v.x, (real)v.y, (real)v.z, (real)v.w}; }
 
 template <typename V>
 __device__ __forceinline__ void warp_argmin(V& v, int& i) {
@@ -239,9 +238,11 @@ __device__ void faces_inside(VorShared& sh, int NC, int nf, int lane) {
     if (lane < kFaceWords) sh.bad[lane] = 0u;
     __syncwarp();
     const int n = nf * NC;
+    const float per = 1.0f / (float)NC;
     #pragma unroll 1
     for (int k = lane; k < n; k += 32) {
-        const int fi = k / NC, cp = k - fi * NC;
+        // k / NC: (k + 1/2) / NC is at least 1 / (2 NC) > 0.005 from a whole number, its rounding below 2e-5
+        const int fi = (int)(((float)k + 0.5f) * per), cp = k - fi * NC;
         const int X = sh.flist[fi];
         if (cp == X || sh.flag[cp] == 0) continue;
         const real* q = &sh.u.f.cosv[3 * X];
@@ -265,76 +266,17 @@ __device__ void add_edge(VorShared& sh, int en, int p0, int p1, int tp, int sp, 
     sh.u.e.es[en] = make_uchar2((uint8_t)sp, kNone);
 }
 
-struct WalkStep {
-    real x, y, z;
-    int pc;      // closing plane, -1 if none
-};
-
-
-// The vertex that ends edge e (LIB/Vcontacts.cpp:283-330), in full precision: the plane with
-// the smallest positive vt along the edge (planes spread over the lanes) and, when that point
-// lies outside the sphere, the bounding planes too. The result is uniform across the warp.
-__device__ WalkStep walk_step_exact(const VorShared& sh, int NC, int e, real rr, int lane) {
-    const uchar4 ep = sh.u.e.ep[e];
-    const real3 V = sh.u.e.ev[e];
-    const real4 s = sh.vx[sh.u.e.es[e].x];
-    const int pA = ep.x, pB = ep.y, oldC = ep.z;
-    real vtmin = real(9.9e9);
-    int pC = INT_MAX;
-    #pragma unroll 1
-    for (int c = lane; c < NC; c += 32) {
-        if (c == pA || c == pB || c == oldC) continue;
-        const real4 P = sh.pl[c];
-        const real den = P.x * V.x + P.y * V.y + P.z * V.z;
-        if (den != real(0.0)) {
-            const real vt = -(P.x * s.x + P.y * s.y + P.z * s.z + P.w) / den;
-            if (vt < vtmin && vt > real(0.0)) { vtmin = vt; pC = c; }
-        }
-    }
-    warp_argmin(vtmin, pC);
-    real x = s.x + vtmin * V.x, y = s.y + vtmin * V.y, z = s.z + vtmin * V.z;
-    if (x * x + y * y + z * z > rr) {
-        real bvt = vtmin;
-        int bc = pC;
-        if (lane < 4) {
-            const int c = NC + lane;
-            if (c != pA && c != pB && c != oldC) {
-                const real4 P = sh.pl[c];
-                const real den = P.x * V.x + P.y * V.y + P.z * V.z;
-                if (den != real(0.0)) {
-                    const real vt = -(P.x * s.x + P.y * s.y + P.z * s.z + P.w) / den;
-                    if (vt < bvt && vt > real(0.0)) { bvt = vt; bc = c; }
-                }
-            }
-        }
-        warp_argmin(bvt, bc);
-        vtmin = bvt;
-        pC = bc;
-        x = s.x + vtmin * V.x;
-        y = s.y + vtmin * V.y;
-        z = s.z + vtmin * V.z;
-    }
-    WalkStep r;
-    r.x = x;
-    r.y = y;
-    r.z = z;
-    r.pc = pC == INT_MAX ? -1 : pC;
-    return r;
-}
-
 // The hull walk steps several open edges at once: a step's result depends only on its edge (start
 // vertex, direction, planes), all fixed when the edge was made, and the reference takes every edge
 // that is open now, in index order, before any edge the steps append (those get higher indices).
-// So the first kWalkGroups open edges are stepped together, one group of kWalkLanes lanes each (the
-// double-precision arithmetic of the step then serves four edges per warp instruction), and their
-// results are booked one after another in index order, skipping an edge an earlier one closed.
+// So the first kWalkGroups open edges are stepped together, one group of kWalkLanes lanes each (eight
+// groups of four lanes are as fast, 2,000 poses 3.77 against 3.75 ms), and their results are booked one after another in index order, skipping an edge an earlier one closed.
 constexpr int kWalkGroups = 4;
 constexpr int kWalkLanes = 32 / kWalkGroups;
 
 struct GroupStep {
     real x, y, z;
     int pc;        // closing plane, -1 if none
-    bool unsure;   // the single-precision pre-tests did not decide it: redo with walk_step_exact
 };
 
 // Argmin over the lanes of one group (ties to the lower plane index, as the reference's strict
@@ -403,7 +345,6 @@ __device__ GroupStep walk_step_group(const VorShared& sh, int NC, int e, real rr
         r.z = s.z + vtmin * V.z;
     }
     r.pc = pC == INT_MAX ? -1 : pC;
-    r.unsure = false;
     return r;
 }
 
@@ -704,26 +645,14 @@ __device__ int voronoi_warp(VorShared& sh, int NC, real rado, int lane, int* no_
         // book the steps in index order; a new vertex's coordinates are stored by its group's
         // first lane and a new edge's direction is set after the batch (lane j holds the j-th new
         // edge: slot, planes, start vertex)
-        real gx = gs.x, gy = gs.y, gz = gs.z;
         int my_vn = -1;
         int n_pend = 0, pe = 0, p0e = 0, pce = 0, tpe = 0, pve = 0;
         #pragma unroll 1
         for (int g = 0; g < nb; ++g) {
             const int e = (batch >> (8 * g)) & 0xffu;
-            const int pu = __shfl_sync(kFull, (gs.pc << 1) | (int)gs.unsure, g * kWalkLanes);
-            int pC = pu >> 1;   // (an arithmetic shift keeps -1)
-            const bool unsure = (pu & 1) != 0;
+            const int pC = __shfl_sync(kFull, gs.pc, g * kWalkLanes);
             if (sh.u.e.es[e].y != kNone) continue;   // closed by an earlier edge of the batch
             startedge = e;
-            if (unsure) {
-                const WalkStep w = walk_step_exact(sh, NC, e, rr, lane);
-                if (lane == g * kWalkLanes) {
-                    gx = w.x;
-                    gy = w.y;
-                    gz = w.z;
-                }
-                pC = w.pc;
-            }
             if (pC < 0) return kAtomHullFail;
             if (vn >= kMaxVerts - 1) return kAtomCapacity;
             const uchar4 ep = sh.u.e.ep[e];
@@ -782,7 +711,7 @@ __device__ int voronoi_warp(VorShared& sh, int NC, real rado, int lane, int* no_
             ++vn;
             __syncwarp();
         }
-        if (my_vn >= 0) sh.vx[my_vn] = make_real4(gx, gy, gz, real(0.0));
+        if (my_vn >= 0) sh.vx[my_vn] = make_real4(gs.x, gs.y, gs.z, real(0.0));
         __syncwarp();
         // the new edges' directions, oriented away from their third plane (add_vedge)
         if (lane < n_pend) {
