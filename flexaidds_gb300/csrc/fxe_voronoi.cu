@@ -625,8 +625,6 @@ __device__ int voronoi_warp(VorShared& sh, int NC, real rado, int lane, int* no_
     const unsigned gmask = ((1u << kWalkLanes) - 1u) << (lane & ~(kWalkLanes - 1));
     #pragma unroll 1
     for (;;) {
-        while (startedge < edgenum && sh.u.e.es[startedge].y != kNone) ++startedge;
-        if (startedge >= edgenum) break;
         // the first kWalkGroups open edges, in index order (one byte each)
         unsigned batch = 0u;
         int nb = 0;
@@ -640,6 +638,7 @@ __device__ int voronoi_warp(VorShared& sh, int NC, real rado, int lane, int* no_
                 ++nb;
             }
         }
+        if (nb == 0) break;
         const int grp = lane / kWalkLanes;
         const GroupStep gs = walk_step_group(sh, NC, grp < nb ? (int)((batch >> (8 * grp)) & 0xffu) : -1, rr, sub, gmask);
         // book the steps in index order; a new vertex's coordinates are stored by its group's
