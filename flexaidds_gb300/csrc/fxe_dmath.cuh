@@ -1,5 +1,5 @@
-// fxe_dmath.cuh — double-precision quotients and square roots, correctly rounded, with five FP64
-// instructions each, and conversions on the integer units.
+// fxe_dmath.cuh — double-precision quotients and square roots, correctly rounded, with five and four
+// FP64 instructions, and conversions on the integer units.
 //
 // GB300's FP64 unit takes one warp instruction per 64 cycles and SM quarter, whatever its active
 // lanes (measured: 66 cycles per DFMA of one warp, dependent or not; 16.4 per SM with four or more
@@ -13,9 +13,17 @@
 // 2^-84 of 1/b before its rounding, so z0 = a y is within two units in the last place of a / b, and
 // z1 = z0 + (a - b z0) y, whose residual is exact, is correctly rounded (P. W. Markstein,
 // "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34,
-// 1990). Root: two such corrections, z + (x - z z) y / 2: the first leaves z within 2^-80 of the root
-// before its rounding, the second rounds it correctly. Both equal the plain operators bit for bit
-// (checked on 1.6e9 operands of every kind); an exponent out of the range the steps need, and a
+// 1990).
+//
+// Root: g = x (2 h) is within 2^-44 of the root, and g + (x - g g) h within 2^-86 of it before its
+// rounding, so the rounded g is the correctly rounded root unless the root lies within 2^-33 units in
+// the last place of the midpoint of two doubles. A second correction cannot decide those: it is multiplied
+// by the same h, and a root can lie within 2^-54 units of a midpoint. Beside a midpoint the residual
+// x - g g is 2 g times half a unit, so its significand is g's (beside_midpoint, an integer test on 20
+// bits, one operand in 300,000): those fall back to the plain function.
+//
+// Both equal the plain operators bit for bit (tests: operands of every kind, and the operands whose
+// results lie closest to midpoints); an exponent out of the range the steps need, and a
 // divisor whose significand is all ones (the theorem's exception), fall back to them. The plain
 // operators sit in functions of their own that are called: left in line, the compiler evaluates them
 // beside the short form and selects.
@@ -115,13 +123,23 @@ __device__ __forceinline__ double div_short(double a, double b, bool* slow) {
     return q;
 }
 
+// Whether residual r is v times half a unit in the last place of z, both to 20 bits: the half below z (the
+// smaller one when z is a power of two) or the half above. hz: z's high word, its sign bit clear.
+__device__ __forceinline__ bool beside_midpoint(double r, double v, int hz) {
+    const int half = (__double2hiint(v) & 0x7fffffff) + (hz & 0x7ff00000) - (1077 << 20);   // v 2^(e(z) - 54)
+    const unsigned k = (unsigned)((__double2hiint(r) & 0x7fffffff) - half + 1);
+    return (k & ~(1u << 20)) <= 2u;
+}
+
 // sqrt(x); *slow: the plain function is needed.
 __device__ __forceinline__ double sqrt_short(double x, bool* slow) {
     const double h = half_rsqrt45(x);
     double g = __dmul_rn(x, __hiloint2double(__double2hiint(h) + (1 << 20), __double2loint(h)));
     g = __fma_rn(__fma_rn(-g, g, x), h, g);
-    g = __fma_rn(__fma_rn(-g, g, x), h, g);
-    *slow = (unsigned)((__double2hiint(x) >> 20) - (int)kExpLo) >= kExpSpan;
+    const int hg = __double2hiint(g);
+    // (x - g g = (root - g) 2 g: half a unit of g times 2 g)
+    *slow = (unsigned)((__double2hiint(x) >> 20) - (int)kExpLo) >= kExpSpan ||
+            beside_midpoint(__fma_rn(-g, g, x), __hiloint2double(hg + (1 << 20), 0), hg);
     return g;
 }
 

@@ -25,7 +25,7 @@
 //
 // What bounds it: the FP64 unit, which takes one warp instruction per 64 cycles and SM quarter
 // whatever its active lanes. Hence
-//   * quotients and roots in five FP64 instructions (fxe_dmath.cuh);
+//   * quotients in five FP64 instructions and roots in four (fxe_dmath.cuh);
 //   * comparisons on the integer units (the bit patterns of doubles order like the doubles);
 //   * the three coordinates of a vertex or a direction on three lanes, one instruction for all;
 //   * the triangles and arcs of all the group's poses packed into full warps (25 and 7 per atom on

@@ -89,3 +89,35 @@ def test_short_operations_are_correctly_rounded(ops, kind):
         normal = (np.abs(a) >= 2.0 ** -126) & (np.abs(a) < 2.0 ** 128)
         assert np.all(f[normal] <= np.abs(a[normal])) and np.all(np.abs(a[normal]) - f[normal] < np.abs(a[normal]) * 2.0 ** -22)
         assert np.all(t[np.abs(a) < 2.0 ** -126] == 0.0) and np.all(np.isinf(t[np.abs(a) >= 2.0 ** 128]))
+
+
+def _square_root_mod(u, n):
+    """r with r * r = u (mod 2^n), u = 1 (mod 8), a bit at a time."""
+    r = 1
+    for i in range(3, n):
+        if (r * r - u) % (1 << (i + 1)):
+            r += 1 << (i - 1)
+    return r % (1 << n)
+
+
+def _roots_beside_midpoints(n):
+    """x whose root lies as close to the midpoint of two doubles as a root can: k is a midpoint's 54-bit
+    significand, k^2 = u (mod 2^54) with a small u, and x = (k^2 - u) / 2^54 is a significand of 53 bits."""
+    out, m = [], 1 << 54
+    for u in range(1 - 8 * n, 8 * n, 8):
+        r = _square_root_mod(u, 54)
+        for k in {r, -r % m, (r + m // 2) % m, (m // 2 - r) % m}:
+            x = (k * k - u) >> 54
+            if k >= m // 2 and x < m and (x < m // 2 or x % 2 == 0):
+                out.append(x)
+    return np.array(out, np.float64)
+
+
+def test_roots_beside_midpoints(ops):
+    x = _roots_beside_midpoints(6000)
+    assert len(x) > 10000
+    rng = np.random.default_rng(3)
+    x = np.ldexp(x, 2 * rng.integers(-150, 150, len(x)))
+    s = ops(x, np.ones(len(x)))[1]
+    wrong = s != np.sqrt(x)
+    assert not wrong.any(), (int(wrong.sum()), x[wrong][:3])
