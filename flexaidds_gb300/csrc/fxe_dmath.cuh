@@ -9,11 +9,17 @@
 // one Newton-Raphson step on the operand split in two floats, about 45 bits — and is put together as
 // a double with integer arithmetic.
 //
-// Quotient: one more Newton step in double (two fused multiply-adds) leaves the reciprocal y within
-// 2^-84 of 1/b before its rounding, so z0 = a y is within two units in the last place of a / b, and
-// z1 = z0 + (a - b z0) y, whose residual is exact, is correctly rounded (P. W. Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34,
-// 1990).
+// Quotient: one more Newton step in double (two fused multiply-adds) leaves the reciprocal y within half
+// a unit and 2^-84 of 1/b, so z0 = a y is within one and a half units in the last place of a / b, and z1 =
+// z0 + (a - b z0) y, whose residual is exact, is correctly rounded (after P. W. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990, who asks for the
+// correctly rounded reciprocal; y is not that where 1/b itself lies within 2^-84 of a midpoint). For, with
+// b in [1, 2): before its rounding z1 is off by (a/b - z0) (b y - 1), and only a quotient beside the
+// midpoint of two doubles could round wrongly; there |a/b - z0| is half a unit, |b y - 1| at most
+// b (2^-54 + 2^-84), and a/b no nearer to the midpoint than 2^-53 / b units. So b must exceed 2 - 2^-28:
+// a divisor whose significand starts with 29 ones falls back to the plain operator. (Of 159,000
+// quotients beside midpoints, a third of them by divisors 2 - k 2^-52, three were one unit off when only
+// k = 1 fell back.)
 //
 // Root: g = x (2 h) is within 2^-44 of the root, and g + (x - g g) h within 2^-86 of it before its
 // rounding, so the rounded g is the correctly rounded root unless the root lies within 2^-33 units in
@@ -23,10 +29,9 @@
 // bits, one operand in 300,000): those fall back to the plain function.
 //
 // Both equal the plain operators bit for bit (tests: operands of every kind, and the operands whose
-// results lie closest to midpoints); an exponent out of the range the steps need, and a
-// divisor whose significand is all ones (the theorem's exception), fall back to them. The plain
-// operators sit in functions of their own that are called: left in line, the compiler evaluates them
-// beside the short form and selects.
+// results lie closest to midpoints); an exponent out of the range the steps need falls back to them
+// too. The plain operators sit in functions of their own that are called: left in line, the compiler
+// evaluates them beside the short form and selects.
 #pragma once
 
 #include <cstdint>
@@ -118,7 +123,7 @@ __device__ __forceinline__ double div_short(double a, double b, bool* slow) {
     q = __fma_rn(__fma_rn(-ab, q, a), y, q);
     if (__double2hiint(b) < 0) q = -q;
     const bool a_ok = (unsigned)(biased_exp(a) - (int)kExpLo) < kExpSpan || (__double2hiint(a) | __double2loint(a)) == 0;   // (-0: the plain operator)
-    const bool ones = (((unsigned)__double2hiint(b) | 0xfff00000u) & (unsigned)__double2loint(b)) == 0xffffffffu;
+    const bool ones = (((unsigned)__double2hiint(b) | 0xfff00000u) & ((unsigned)__double2loint(b) | 0x00ffffffu)) == 0xffffffffu;
     *slow = !a_ok || (unsigned)(biased_exp(b) - (int)kExpLo) >= kExpSpan || ones;
     return q;
 }

@@ -113,6 +113,19 @@ def _roots_beside_midpoints(n):
     return np.array(out, np.float64)
 
 
+def _quotients_beside_midpoints(divisors):
+    """(a, b) whose quotient lies as close to a midpoint as one can: a 2^54 = c (mod b), c small and odd."""
+    a, b = [], []
+    for B in divisors:
+        inv = pow(2, -54, B)
+        for c in (-7, -5, -3, -1, 1, 3, 5, 7):
+            for A in (c * inv % B, 2 * c * inv % B + B):
+                if 1 << 52 <= A < 1 << 53:
+                    a.append(A)
+                    b.append(B)
+    return np.array(a, np.float64), np.array(b, np.float64)
+
+
 def test_roots_beside_midpoints(ops):
     x = _roots_beside_midpoints(6000)
     assert len(x) > 10000
@@ -121,3 +134,19 @@ def test_roots_beside_midpoints(ops):
     s = ops(x, np.ones(len(x)))[1]
     wrong = s != np.sqrt(x)
     assert not wrong.any(), (int(wrong.sum()), x[wrong][:3])
+
+
+def test_quotients_beside_midpoints(ops):
+    """Divisors of every kind, and those just below a power of two: their reciprocal lies beside a midpoint
+    itself ((2^53 - k) (2^53 + k) = 2^106 - k^2), where its rounding is uncertain."""
+    rng = np.random.default_rng(4)
+    any_b = [int(v) | 1 for v in rng.integers(1 << 52, 1 << 53, 20000)]
+    near = [(1 << 53) - k for k in range(1, 20001, 2)] + [(1 << 52) + k for k in range(1, 2001, 2)]
+    a, b = _quotients_beside_midpoints(any_b + near)
+    assert len(a) > 100000
+    ea, eb = rng.integers(-250, 250, (2, len(a)))
+    a = np.ldexp(a * rng.choice([-1.0, 1.0], len(a)), ea)
+    b = np.ldexp(b * rng.choice([-1.0, 1.0], len(b)), eb)
+    q = ops(a, b)[0]
+    wrong = q != a / b
+    assert not wrong.any(), (int(wrong.sum()), a[wrong][:3], b[wrong][:3])
