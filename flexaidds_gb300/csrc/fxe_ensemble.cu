@@ -15,7 +15,8 @@
 // t (a bounded scan per thread, then one warp per unresolved head scanning 32 at a time); the kept
 // heads are the path 0, next(0), next(next(0)), .... The heads are cut into segments that fit a block's
 // shared memory: one launch finds by pointer jumping where the path leaves the segment from each of its
-// heads, the next follows those exits to its segment and marks the path inside.
+// heads, the next follows those exits to its segment (past 608 segments one thread does it for all, in a
+// launch between) and marks the path inside.
 //
 // What bounds the assembly is its number of dependent launches more than the bytes (12 per chromosome
 // and pass, the genes once): 4-bit digits with a three-launch scan each and log2(n) launches of pointer
@@ -331,12 +332,28 @@ ens_exits_kernel(const int* __restrict__ nxt, const int* __restrict__ Mp, int* _
     }
 }
 
+// Up to this many segments each block of ens_mark_kernel follows the exits to its own segment; beyond,
+// one thread follows them once for all (the walks of S blocks are S^2 / 2 dependent loads, two blocks an
+// SM at a time, so that they cost more than one walk from about 600 segments up). 300,000,000
+// chromosomes, 36,622 segments: 693 ms the call with every block walking, 358 ms so (20,000,000: 21.5 and 20.6; 4,000,000: 4.8 either way).
+constexpr int kOwnWalk = 608;
+
+// entry[s]: the first head on the path from head 0 that lies in segment s or past it.
+__global__ void ens_entries_kernel(const int* __restrict__ exits, const int* __restrict__ Mp, int* __restrict__ entry) {
+    const int M = *Mp;
+    int t = 0;
+    for (long long base = 0; base < M; base += kSegment) {
+        entry[base / kSegment] = t;
+        if (t < base + kSegment) t = exits[t];
+    }
+}
+
 // flag[t] = 1 for the heads on the path from head 0, 0 for the others and for t from M to n: each block
-// follows the exits to its segment, then marks by pointer jumping inside (every marked head marks the
-// head 2^r steps along).
+// takes its segment's entry (entries null: follows the exits to it), then marks by pointer jumping inside
+// (every marked head marks the head 2^r steps along).
 __global__ void __launch_bounds__(kSegThreads)
-ens_mark_kernel(const int* __restrict__ nxt, const int* __restrict__ exits, const int* __restrict__ Mp, long long n,
-                int* __restrict__ flag) {
+ens_mark_kernel(const int* __restrict__ nxt, const int* __restrict__ exits, const int* __restrict__ entries,
+                const int* __restrict__ Mp, long long n, int* __restrict__ flag) {
     extern __shared__ int jump[];
     volatile uint8_t* on = reinterpret_cast<uint8_t*>(jump + kSegment);
     __shared__ int entry;
@@ -345,7 +362,7 @@ ens_mark_kernel(const int* __restrict__ nxt, const int* __restrict__ exits, cons
     const long long end = base + kSegment < M ? base + kSegment : M;
     if (base < M) {
         if (threadIdx.x == 0) {
-            int t = 0;
+            int t = entries ? entries[blockIdx.x] : 0;
             while (t < base) t = exits[t];
             entry = t;
         }
@@ -526,7 +543,12 @@ cudaError_t launch_ensemble(long long n, int ng, const double* e_in, const doubl
     ens_next_far_kernel<<<grid_for(n * 32, kEnsThreads), kEnsThreads, 0, st>>>(ics, ng, H, cnt, nxt, exits, cnt + 1);
     const unsigned segments = (unsigned)((n + kSegment - 1) / kSegment);
     ens_exits_kernel<<<segments, kSegThreads, kSegSmem, st>>>(nxt, cnt, exits);
-    ens_mark_kernel<<<segments, kSegThreads, kSegSmem, st>>>(nxt, exits, cnt, n, kept_flag);
+    int* entries = nullptr;
+    if (segments > kOwnWalk) {
+        entries = stmp;      // (an int per 1,024 chromosomes, free between the scans)
+        ens_entries_kernel<<<1, 1, 0, st>>>(exits, cnt, entries);
+    }
+    ens_mark_kernel<<<segments, kSegThreads, kSegSmem, st>>>(nxt, exits, entries, cnt, n, kept_flag);
     scan_ints(kept_flag, kept_pos, n, stmp, st);
     ens_emit_kernel<<<grid_for(n, kEnsThreads), kEnsThreads, 0, st>>>(H, kept_flag, kept_pos, cnt, v0, e_in, ics, ng, idx_out,
                                                                       e_out, ic_out);

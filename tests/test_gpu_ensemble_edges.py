@@ -7,7 +7,7 @@ from flexaidds_gb300 import evaluator
 
 pytestmark = pytest.mark.gpu
 
-TILE, BLOCKS, SEGMENT = 2048, 4 * 152, 8192
+TILE, BLOCKS, SEGMENT, OWN_WALK = 2048, 4 * 152, 8192, 608
 
 
 def _host(ic, e):
@@ -62,3 +62,25 @@ def test_one_chain_link_spans_segments():
     walk[2 * SEGMENT + 3] = 5.0
     ic[np.argsort(e)] = walk[:, None]
     assert np.array_equal(evaluator.ensemble_dedup(ic, e)["index"], _host(ic, e))
+
+
+@pytest.mark.parametrize("segments", [OWN_WALK - 1, OWN_WALK, OWN_WALK + 1, 2 * OWN_WALK + 1])
+def test_chain_of_many_segments(segments):
+    """Families within the tolerance of their first member, most of a few heads and some longer than a
+    segment, so that the path enters segments at their first head, further in, or not at all."""
+    n = segments * SEGMENT - 5
+    rng = np.random.default_rng(segments)
+    size = rng.integers(1, 40, n // 16)
+    size[rng.integers(0, len(size), 40)] = rng.integers(SEGMENT // 2, 3 * SEGMENT, 40)
+    first = np.concatenate([[0], np.cumsum(size)])
+    first = first[first < n]
+    family = np.zeros(n)
+    family[first] = 1.0
+    # (two values in turn: neighbours differ, so that every chromosome is a head)
+    ic = np.cumsum(family) + 0.05 * (np.arange(n) % 2)
+    order = rng.permutation(n)                                   # input index of each sorted place
+    e, rows = np.empty(n), np.empty((n, 1))
+    e[order] = np.arange(n) * 0.001 - 30.0
+    rows[order, 0] = ic
+    r = evaluator.ensemble_dedup(rows, e)
+    assert np.array_equal(r["index"], order[first])
