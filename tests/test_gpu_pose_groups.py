@@ -65,3 +65,76 @@ def test_polyhedra_past_the_compact_shape(shell, radius, atom):
     assert (want["status"] != 2).sum() >= 50
     err = np.abs(got["evalue"] - want["evalue"]) / np.maximum(1.0, np.abs(want["evalue"]))
     assert err.max() <= 1e-9
+
+
+def _shell_system(shell, radius, seed):
+    """A four-atom ligand inside a shell of receptor atoms all about as far away."""
+    base = system.make_inputs(600, 6.0, 12, 3, seed=5)
+    k = np.arange(shell) + 0.5
+    phi, z = np.pi * (1.0 + 5.0 ** 0.5) * k, 1.0 - 2.0 * k / shell
+    r = np.sqrt(1.0 - z * z)
+    xyz = radius * np.stack([r * np.cos(phi), r * np.sin(phi), z], axis=1)
+    xyz += np.random.default_rng(shell).normal(0.0, 0.05, xyz.shape)
+    far = base.receptor.xyz - base.receptor.cleft_center
+    xyz = np.concatenate([xyz, far[np.linalg.norm(far, axis=1) > 9.5]]).astype(np.float32)
+    n = len(xyz)
+    rec = synth.Receptor(xyz=xyz, type=np.resize(base.receptor.type, n), radius=np.full(n, 2.0, np.float32),
+                         cleft_center=np.zeros(3, np.float32), cleft_radius=2.0, edge=12.0)
+    grid = np.random.default_rng(2).uniform(-0.3, 0.3, (200, 3)).astype(np.float32)
+    return prepare.prepare(system.SystemInputs(receptor=rec, ligand=synth.random_ligand(4, 0, seed=seed), grid_xyz=grid,
+                                               emat=base.emat))
+
+
+FACES_PAST_COMPACT = 56   # a cell of F faces has 2 F - 4 vertices; the compact shape holds 104
+
+
+@pytest.fixture(scope="module", params=[(84, 4.8), (70, 5.2)])
+def oversized(request):
+    """Two systems in one shell (nearly all of the poses outgrow the compact shape, or one in twenty), 8,000
+    and 700 poses, and the oracle's records."""
+    port.set_reference_compat(True)
+    port.set_trig_rounding(False)
+    out = []
+    for seed, n in ((3, 8000), (4, 700)):
+        d = _shell_system(*request.param, seed)
+        genes = synth.random_genes(n, d.n_genes, seed=seed)
+        out.append((d, genes, port.Oracle(d).eval_ic(d.genes_to_ic(genes))["cf"]))
+    d, genes, _ = out[0]
+    c = port.Oracle(d).eval_ic(d.genes_to_ic(genes[:400]), want_contacts=True)["contacts"]
+    faces = np.zeros((400, d.n_lig), int)
+    np.add.at(faces, (c["pose"], c["atom"]), 1)
+    past = (faces.max(axis=1) >= FACES_PAST_COMPACT).mean()
+    assert past > 0.8 if request.param[0] == 84 else 0.02 < past < 0.5
+    return out
+
+
+def _assert_records(got, want):
+    # a hull walk that never closes fails at 200 edges, and one in 10,000 fills the 176 vertices before: the
+    # device reports those poses as over capacity
+    over = got["status"] == 3
+    assert np.all(want["status"][over] == 1) and over.sum() <= 1
+    got, want = got[~over], want[~over]
+    np.testing.assert_array_equal(got["status"], want["status"])
+    err = np.abs(got["evalue"] - want["evalue"]) / np.maximum(1.0, np.abs(want["evalue"]))
+    assert err.max() <= 1e-9
+
+
+@pytest.mark.parametrize("n", [1, 150, 600, SPLIT * SMS + 1, 3100, 8000])
+def test_large_shape_in_every_grouping(oversized, n):
+    """One, some and all warps of the groups of eight; full groups; and so many poses a block that its list of
+    poses to score again fills, its warps stop taking new ones and return to the queue after the large shape."""
+    d, genes, want = oversized[0]
+    ev = evaluator.GPUEvaluator(d, max_poses=8192)
+    _assert_records(ev.eval_genes(np.ascontiguousarray(genes[:n])), want[:n])
+    ev.close()
+
+
+@pytest.mark.parametrize("n", [(60, 30), (400, 200), (5000, 700)])
+def test_large_shape_in_batches(oversized, n):
+    evs = [evaluator.GPUEvaluator(d, max_poses=8192) for d, _, _ in oversized]
+    batch = evaluator.Batch(max_jobs=2, max_poses=8192)
+    got = batch.eval_genes([(ev, np.ascontiguousarray(g[:k])) for ev, (_, g, _), k in zip(evs, oversized, n)])
+    for r, (_, _, want), k in zip(got, oversized, n):
+        _assert_records(r, want[:k])
+    for ev in evs:
+        ev.close()
