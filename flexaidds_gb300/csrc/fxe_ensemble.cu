@@ -335,7 +335,8 @@ ens_exits_kernel(const int* __restrict__ nxt, const int* __restrict__ Mp, int* _
 // Up to this many segments each block of ens_mark_kernel follows the exits to its own segment; beyond,
 // one thread follows them once for all (the walks of S blocks are S^2 / 2 dependent loads, two blocks an
 // SM at a time, so that they cost more than one walk from about 600 segments up). 300,000,000
-// chromosomes, 36,622 segments: 693 ms the call with every block walking, 358 ms so (20,000,000: 21.5 and 20.6; 4,000,000: 4.8 either way).
+// chromosomes, 36,622 segments: 693 ms the call with every block walking, 358 ms so (20,000,000: 21.5
+// and 20.6; 4,000,000: 4.8 either way).
 constexpr int kOwnWalk = 608;
 
 // entry[s]: the first head on the path from head 0 that lies in segment s or past it.
