@@ -1217,9 +1217,7 @@ extern "C" fxe_status fxe_thermo_compute_device_fixed(const double* d_energies, 
         return fail(FXE_ERR_INVALID_ARGS, "invalid arguments (NULL pointer, n <= 0 or T <= 0)");
     if (n > FXE_THERMO_FIXED_MAX_N)
         return fail(FXE_ERR_INVALID_ARGS, "n = " + std::to_string(n) + " exceeds FXE_THERMO_FIXED_MAX_N = " +
-                                              std::to_string((long long)FXE_THERMO_FIXED_MAX_N) +
-                                              " (the fixed scratch holds " +
-                                              std::to_string(FXE_THERMO_FIXED_MAX_BLOCKS) + " block partials)");
+                                              std::to_string((long long)FXE_THERMO_FIXED_MAX_N));
     int dev = 0;
     FXE_TRY(cudaGetDevice(&dev), "cudaGetDevice");
     if (dev < 0 || dev >= kFixedMaxDevices) return fail(FXE_ERR_NO_DEVICE, "device ordinal out of range");

@@ -153,10 +153,12 @@ void thermo_finish(const LsePart* part, int nb, double T, fxe_thermo* out) {
 // ------------------------------------------------------------------------------------------
 namespace fxe {
 
+constexpr int kFixedBlocks = 4 * 152;   // at most
+
 // One partial per block, and after them one slot for the count of finished blocks; every slot a
 // call reads is written (or, the count, cleared) by that call first, so nothing here needs to
 // start at zero.
-static __device__ __align__(256) LsePart g_fixed_part[FXE_THERMO_FIXED_MAX_BLOCKS + 1];
+static __device__ __align__(256) LsePart g_fixed_part[kFixedBlocks + 1];
 
 cudaError_t fixed_scratch_address(LsePart** p) {
     return cudaGetSymbolAddress(reinterpret_cast<void**>(p), g_fixed_part);
@@ -273,7 +275,6 @@ __device__ __forceinline__ LseState block_sums(const LseState& st, double (*ws)[
 // and a running maximum per thread an energy cost 55 of its instructions, 98 us for 1,000,000 energies;
 // 47 us so (14 instructions an energy are 24 us).
 constexpr int kFixedChunk = 8;
-constexpr int kFixedBlocks = 4 * 152;
 
 template <bool kMult>
 __global__ void __launch_bounds__(kThermoThreads, 4)
@@ -380,7 +381,6 @@ thermo_fixed_kernel(const double* __restrict__ e, const int32_t* __restrict__ mu
 
 // Blocks of the fixed-scratch pass: one energy per thread, up to four blocks per SM (the device's
 // full set at 64 registers); past 1,245,184 energies a block takes several chunks.
-static_assert(kFixedBlocks <= FXE_THERMO_FIXED_MAX_BLOCKS, "a partial per block");
 void launch_thermo_fixed(const double* e, const int32_t* mult, long n, double beta, double T,
                          LsePart* scratch, fxe_thermo* d_out, cudaStream_t st) {
     long nb = (n + kThermoThreads - 1) / kThermoThreads;
@@ -389,7 +389,7 @@ void launch_thermo_fixed(const double* e, const int32_t* mult, long n, double be
     // whole warps
     const long per_block = ((n + nb - 1) / nb + 31) & ~31l;
     nb = (n + per_block - 1) / per_block;
-    unsigned* done = reinterpret_cast<unsigned*>(scratch + FXE_THERMO_FIXED_MAX_BLOCKS);
+    unsigned* done = reinterpret_cast<unsigned*>(scratch + kFixedBlocks);
     cudaMemsetAsync(done, 0, sizeof(unsigned), st);
     auto* kernel = mult ? thermo_fixed_kernel<true> : thermo_fixed_kernel<false>;
     kernel<<<(int)nb, kThermoThreads, 0, st>>>(e, mult, n, per_block, beta, T, scratch, done, d_out);
