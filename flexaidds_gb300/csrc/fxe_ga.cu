@@ -51,19 +51,13 @@ __device__ __forceinline__ double uniform(uint64_t seed, uint64_t s, uint64_t k)
     return (double)uniform_bits(seed, s, k) * 0x1.0p-53;
 }
 
-// A probability p with the integer form of the test u < p for draws u = b 2^-53 (b < 2^53 an
-// integer): u < p exactly when b < ceil(p 2^53), the scaling by 2^53 being exact. Tests with it
-// stay on the integer units (a mutation makes 32 such tests per gene).
-struct DrawThreshold {
-    double p;
-    uint64_t bits;
-};
-__device__ __forceinline__ DrawThreshold draw_threshold(double p) {
+// The integer form of the test u < p for draws u = b 2^-53 (b < 2^53 an integer): u < p exactly
+// when b < ceil(p 2^53), the scaling by 2^53 being exact. Tests with it stay on the integer units
+// (a mutation makes 32 such tests per gene).
+__device__ __forceinline__ uint64_t draw_threshold(double p) {
     const double t = p * 0x1.0p53;
-    uint64_t b = 0;                                  // p <= 0 or NaN: no draw is below
-    if (t >= 0x1.0p53) b = 1ull << 53;               // p >= 1: every draw is
-    else if (t > 0.0) b = (uint64_t)ceil(t);
-    return {p, b};
+    if (t >= 0x1.0p53) return 1ull << 53;            // p >= 1: every draw is below
+    return t > 0.0 ? (uint64_t)ceil(t) : 0ull;       // p <= 0 or NaN: no draw is
 }
 
 constexpr int kGaThreads = 256;
@@ -317,7 +311,7 @@ __device__ void breed_pair_warp(const GaJob& J, int g, int k, int lane, int32_t*
     const int a = J.ford[pa], b = J.ford[pb];
     double crossp = J.cross_rate, mutp = J.mut_rate;
     if (J.adaptive) adapt_prob(J, J.fit[pa], J.fit[pb], fit_max, fit_avg, &crossp, &mutp);
-    const DrawThreshold mut = draw_threshold(mutp);
+    const uint64_t mut = draw_threshold(mutp);
     const Crossover x = draw_crossover(J, draw, crossp);
     uint32_t c0[2] = {0u, 0u}, c1[2] = {0u, 0u};
 #pragma unroll
@@ -348,7 +342,7 @@ __device__ void breed_pair_warp(const GaJob& J, int g, int k, int lane, int32_t*
         for (int q = 0; q < ng; ++q) {
             const float pr = J.gene_prob[q];
             if (pr >= 0.0f && !(draw() < (double)pr)) continue;
-            const uint32_t optr = __ballot_sync(0xffffffffu, uniform_bits(draw.seed, draw.st, draw.d + lane) < mut.bits);
+            const uint32_t optr = __ballot_sync(0xffffffffu, uniform_bits(draw.seed, draw.st, draw.d + lane) < mut);
             draw.d += 32;
             if (lane == (q & 31)) {
                 if (q < 32) ch[0] ^= optr;
@@ -407,8 +401,8 @@ constexpr int kGaMaxBatches = 16;   // candidate batches before duplicates are l
 // candidates.
 constexpr int kAcceptThreads = 1024;
 constexpr int kAcceptMax = 2 * (kGaMaxPop + 8);    // candidates of a batch
-constexpr int kAcceptTable = 8192;                 // hash slots: at most half of them taken
-static_assert(kAcceptTable >= kAcceptMax * 3 / 2 && kAcceptTable <= 65536, "");
+constexpr int kAcceptTable = 8192;                 // hash slots: at most two thirds of them taken
+static_assert(2 * kAcceptTable >= 3 * kAcceptMax && kAcceptTable <= 65536, "slots to spare, named by 16 bits");
 constexpr size_t kAcceptSmem = (size_t)kAcceptTable * (sizeof(uint64_t) + sizeof(int)) + (size_t)kAcceptMax * (sizeof(uint16_t) + 1);
 
 template <bool kInitial>

@@ -1059,12 +1059,12 @@ __device__ __forceinline__ int arc_points(Vor<Sh>& sh, double rado, double rr, i
     return nv > Sh::verts - 1 ? Sh::over : kAtomOk;
 }
 
-// The first set bit at or after bit `from` of the vertex mask a & b (b may be null), or -1.
+// The first set bit at or after bit `from` of the vertex mask a & b, or -1.
 template <class Sh>
 __device__ __forceinline__ int first_vertex(const uint32_t* a, const uint32_t* b, int from) {
     #pragma unroll 1
     for (int w = from >> 5; w < Sh::vwords; ++w) {
-        uint32_t m = a[w] & (b ? b[w] : 0xffffffffu);
+        uint32_t m = a[w] & b[w];
         if (w == from >> 5) m &= 0xffffffffu << (from & 31);
         if (m) return 32 * w + __ffs(m) - 1;
     }
