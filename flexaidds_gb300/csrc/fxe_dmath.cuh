@@ -1,5 +1,5 @@
 // fxe_dmath.cuh — double-precision quotients and square roots, correctly rounded, with five and four
-// FP64 instructions, and conversions on the integer units.
+// FP64 instructions, and conversions and comparisons on the integer units.
 //
 // GB300's FP64 unit takes one warp instruction per 64 cycles and SM quarter, whatever its active
 // lanes (measured: 66 cycles per DFMA of one warp, dependent or not; 16.4 per SM with four or more
@@ -47,6 +47,22 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
     float r;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
+}
+
+// --- comparisons on bit patterns (false when a NaN, of either sign, is involved) -----------------
+constexpr long long kInfBits = 0x7ff0000000000000ll;
+__device__ __forceinline__ long long bits(double x) { return __double_as_longlong(x); }
+__device__ __forceinline__ bool gt0(double x) { return bits(x) > 0 && bits(x) <= kInfBits; }   // x > 0
+__device__ __forceinline__ bool lt0(double x) { return gt0(-x); }                               // x < 0
+__device__ __forceinline__ bool is0(double x) { return (bits(x) << 1) == 0; }
+// a < b and a <= b of values whose sign bit is clear (unsigned: a NaN with the bit set lies above them too)
+__device__ __forceinline__ bool lt_nn(double a, double b) {
+    const unsigned long long ua = (unsigned long long)bits(a), ub = (unsigned long long)bits(b);
+    return ua < ub && ub <= (unsigned long long)kInfBits;
+}
+__device__ __forceinline__ bool le_nn(double a, double b) {
+    const unsigned long long ua = (unsigned long long)bits(a), ub = (unsigned long long)bits(b);
+    return ua <= ub && ub <= (unsigned long long)kInfBits;
 }
 
 // Biased exponents of operands the short forms take: 2^-350 .. 2^350.

@@ -82,16 +82,6 @@ struct __align__(32) real4 {
 __device__ __forceinline__ real4 make_real4(double x, double y, double z, double w) { return real4{x, y, z, w}; }
 __device__ __forceinline__ double comp(const real4& v, int c) { return reinterpret_cast<const double*>(&v)[c]; }
 
-// --- comparisons on bit patterns ----------------------------------------------------------------
-constexpr long long kInfBits = 0x7ff0000000000000ll;
-__device__ __forceinline__ long long bits(double x) { return __double_as_longlong(x); }
-__device__ __forceinline__ bool gt0(double x) { return bits(x) > 0 && bits(x) <= kInfBits; }   // x > 0
-__device__ __forceinline__ bool lt0(double x) { return gt0(-x); }                               // x < 0
-__device__ __forceinline__ bool is0(double x) { return (bits(x) << 1) == 0; }
-// a < b and a <= b of values that are not negative (a NaN compares false)
-__device__ __forceinline__ bool lt_nn(double a, double b) { return bits(a) < bits(b) && bits(b) <= kInfBits; }
-__device__ __forceinline__ bool le_nn(double a, double b) { return bits(a) <= bits(b) && bits(b) <= kInfBits; }
-
 // Quotients, roots and arc tangents out of line: an FP64 instruction takes five instruction slots on
 // sm_103a (with those the compiler pads it with), and the kernel is bound by instruction fetch before
 // anything else once its warps are at different points of it.

@@ -24,6 +24,23 @@ __global__ void short_ops(const double* a, const double* b, double* q, double* s
     t[i] = fxe::d2f_trunc(a[i]);
     w[i] = fxe::f2d((float)b[i]);
 }
+__global__ void comparisons(const double* a, const double* b, int* out, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n)
+        out[i] = fxe::gt0(a[i]) | fxe::lt0(a[i]) << 1 | fxe::is0(a[i]) << 2 | fxe::lt_nn(a[i], b[i]) << 3 |
+                 fxe::le_nn(a[i], b[i]) << 4;
+}
+extern "C" int compare(const double* a, const double* b, int* out, int n) {
+    double* d = nullptr;
+    const size_t z = sizeof(double) * n;
+    if (cudaMalloc(&d, 3 * z) != cudaSuccess) return 1;
+    cudaMemcpy(d, a, z, cudaMemcpyHostToDevice);
+    cudaMemcpy(d + n, b, z, cudaMemcpyHostToDevice);
+    comparisons<<<(n + 255) / 256, 256>>>(d, d + n, (int*)(d + 2 * n), n);
+    cudaMemcpy(out, d + 2 * n, sizeof(int) * n, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return cudaGetLastError() != cudaSuccess;
+}
 extern "C" int run(const double* a, const double* b, double* q, double* s, float* t, double* w, int n) {
     double* d = nullptr;
     const size_t z = sizeof(double) * n;
@@ -55,6 +72,7 @@ def ops(tmp_path_factory):
         p = [x.ctypes.data_as(C.c_void_p) for x in (a, b, q, s, t, w)]
         assert lib.run(*p, C.c_int(len(a))) == 0
         return q, s, t, w
+    run.lib = lib
     return run
 
 
@@ -150,3 +168,21 @@ def test_quotients_beside_midpoints(ops):
     q = ops(a, b)[0]
     wrong = q != a / b
     assert not wrong.any(), (int(wrong.sum()), a[wrong][:3], b[wrong][:3])
+
+
+def test_comparisons_on_bit_patterns(ops):
+    """Signs of any value; order of values whose sign bit is clear, with NaN of both signs among them."""
+    rng = np.random.default_rng(6)
+    special = np.array([0.0, 5e-324, 2.0 ** -1022, 1.0, 1.0 + 2.0 ** -52, 1.7e308, np.inf, np.nan, -np.nan])
+    a, b = (np.ascontiguousarray(x.ravel()) for x in np.meshgrid(special, special))
+    x = np.abs(rng.normal(0.0, 1.0, 1000))
+    a, b = np.concatenate([a, x]), np.concatenate([b, np.where(rng.random(1000) < 0.3, x, x[::-1])])
+    out = np.zeros(len(a), np.int32)
+    args = [v.ctypes.data_as(C.c_void_p) for v in (a, b, out)]
+    assert ops.lib.compare(*args, C.c_int(len(a))) == 0
+    np.testing.assert_array_equal(out >> 3, (a < b) | (a <= b).astype(int) << 1)
+    s = np.concatenate([special, -special, rng.normal(0.0, 1.0, 1000)])
+    out = np.zeros(len(s), np.int32)
+    args = [v.ctypes.data_as(C.c_void_p) for v in (s, s, out)]
+    assert ops.lib.compare(*args, C.c_int(len(s))) == 0
+    np.testing.assert_array_equal(out & 7, (s > 0.0) | (s < 0.0).astype(int) << 1 | (s == 0.0).astype(int) << 2)
