@@ -154,7 +154,7 @@ struct DevWork {
     uint32_t* pose_rec;    // [P * kMaxLig * kMaskWords] mobile partners each processed atom kept
     double* atom_terms;    // [P * n_mob * 4] terms of each scored atom (reference precision)
     fxe_cf* out;           // [P]
-    int* counters;         // [4]: unused, hull failures, capacity, no-partner faces
+    int* counters;         // [4]: faces not replayed, hull failures, capacity, no-partner faces
     int* pose_cost;        // [P] sum over the pose's atoms of the squared candidate count (zeroed by the
                            // build, added up by the contact scan; for the pose order only)
     float* pose_clash;     // [P] sum of clash_part, likewise

@@ -3,8 +3,8 @@
 //
 // GB300's FP64 unit takes one warp instruction per 64 cycles and SM quarter, whatever its active
 // lanes (measured: 66 cycles per DFMA of one warp, dependent or not; 16.4 per SM with four or more
-// warps; conversions from and to double and comparisons cost the same), and the compiler's quotient
-// and root are nine such instructions each (146 cycles per SM). Here the reciprocal (or reciprocal
+// warps; conversions from and to double and comparisons cost the same), and a plain quotient or root
+// takes as long as nine of them (146 cycles per SM, measured). Here the reciprocal (or reciprocal
 // root) of the operand's significand comes from the single-precision unit — its approximation, then
 // one Newton-Raphson step on the operand split in two floats, about 45 bits — and is put together as
 // a double with integer arithmetic.

@@ -58,7 +58,7 @@ constexpr int kWalkBudget = 16;
 // Capacities of one polyhedron. The compact shape holds the polyhedra of ordinary poses (on the
 // benchmark's systems at most 44 vertices inside the sphere, 125 face points and 125 area items over
 // 2,300 atoms; means 17, 43 and 33) and any hull walk and its arc points (176 vertices: those past
-// `verts` lie in storage the faces use later), in 14.1 KB per pose, so that sixteen poses fit an SM. A
+// `verts` lie in storage the faces use later), in 14.5 KB per pose, so that sixteen poses fit an SM. A
 // pose one of whose atoms outgrows it is scored again, from its start, in the large shape when its
 // group has no other pose.
 // (With 256 items one pose of the benchmark's in 8,000 was: 3.2 ms more for its launch. With 290 none of
@@ -82,9 +82,8 @@ struct __align__(32) real4 {
 __device__ __forceinline__ real4 make_real4(double x, double y, double z, double w) { return real4{x, y, z, w}; }
 __device__ __forceinline__ double comp(const real4& v, int c) { return reinterpret_cast<const double*>(&v)[c]; }
 
-// Quotients, roots and arc tangents out of line: an FP64 instruction takes five instruction slots on
-// sm_103a (with those the compiler pads it with), and the kernel is bound by instruction fetch before
-// anything else once its warps are at different points of it.
+// Quotients, roots and arc tangents out of line: the kernel's code outgrows the instruction caches (with
+// quotients and roots in line 2,000 poses of the benchmark's system take 8.27 ms instead of 7.49).
 __device__ __noinline__ double ddiv(double a, double b) {
     bool slow;
     double q = div_short(a, b, &slow);
@@ -2132,8 +2131,9 @@ static int max_blocks(size_t hist_bytes, int blocks_per_sm) {
 // fewer when the launch's poses would not reach every block the device runs at once, so that they
 // spread over more SMs (a pose's time is its chain of atoms, shorter with fewer warps sharing the
 // SM's double-precision unit). Up to kSplitPoses poses per block two groups of eight warps share it: a
-// pose waits for fewer others (500 poses of 40 atoms: 1,861 us, one group of sixteen 1,998); with the
-// block full their code no longer meets in the instruction cache (2,000 poses: 8.7 ms against 7.8).
+// pose waits for fewer others (500 poses of 24 atoms: 1,725 us, one group of sixteen 1,924); with the
+// block full their code no longer meets in the instruction cache (2,000 poses of 63 atoms: 8.21 ms, one
+// group 7.43).
 constexpr int kSplitPoses = 4;
 static void launch_shape(int n, size_t hist_bytes, int blocks_per_sm, int* blocks, int* group, int* active) {
     const int r = max_blocks(hist_bytes, blocks_per_sm);
