@@ -30,8 +30,8 @@
 //
 // Both equal the plain operators bit for bit (tests: operands of every kind, and the operands whose
 // results lie closest to midpoints); an exponent out of the range the steps need falls back to them
-// too. The plain operators sit in functions of their own that are called: left in line, the compiler
-// evaluates them beside the short form and selects.
+// too. The plain operators sit in functions of their own that are called, so that the short forms do
+// not carry them.
 #pragma once
 
 #include <cstdint>

@@ -224,8 +224,8 @@ __device__ __forceinline__ double exp_short(double x, const double* tab) {
     return fma(T, c, T);
 }
 
-// The library's exp, for arguments outside exp_short's range (a call, so that it is not evaluated
-// beside it).
+// The library's exp, for arguments outside exp_short's range (called, so that the loop does not carry
+// it).
 __device__ __noinline__ double exp_any(double x) { return exp(x); }
 
 // A double's bits as an integer that orders like it (its own inverse).
